@@ -75,12 +75,16 @@ typedef struct fg_ilu_sweeps {
 	double *o64;                    /* ds: the double-single sweeps' output
 	                                   (natural order), apart from their input */
 	float *bl32, *y32;
-	int *fac_ptr, *fac_prog;   /* precompiled elimination of each row        */
-	/* the same elimination for the cluster kernel: per level-order position
-	 * {rb, offset, length, len | dpos << 8 | ngroups << 16}, and per row
-	 * [nops, operand addresses..., per group (q, cnt, dst...)] */
-	int *fac2_hdr, *fac2;
-	int fac2_ok;
+	/* precompiled elimination of the rows, in slots of fac_lanes (8, 16 or
+	 * 32) lanes ordered by dependency level over all matrix blocks: per slot
+	 * {row start, len | dpos << 8 | groups << 16, row (-1: padding), 0}, per
+	 * slot and group (lower entry) its row and that row's start, per slot,
+	 * lane and group the entry's position in that row (a byte) */
+	int *fac_head, *fac_grp;
+	unsigned char *fac_pos;
+	int fac_lanes, fac_nslot;
+	int fac_wide;              /* slots of the widest level                  */
+	void *fac_ticket;          /* fg_ticket of a launch                      */
 	int nblocks;               /* matrix blocks (1: global ILU(0))           */
 	int *block_first;          /* host [nblocks+1] first row of each block   */
 	/* ILU(p), p > 0: the filled pattern the factor and sweeps use (rows as

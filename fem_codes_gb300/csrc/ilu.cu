@@ -32,10 +32,11 @@
 // each block factorises and sweeps independently: its levels form a
 // contiguous run of the program (levels are numbered block by block) and one
 // thread block per matrix block runs them, P thread blocks at once.  The
-// factorisation runs one thread-block cluster per matrix block.  Every wait is
-// bounded: on timeout the block records FEMGPU_E_TIMEOUT, waits (bounded) for
+// factorisation runs all blocks' rows as one dataflow over the device.  Every
+// wait is bounded: on timeout the block records FEMGPU_E_TIMEOUT, waits (bounded) for
 // the copies it has in flight and returns.
 #include "fg_common.cuh"
+#include "fg_dataflow.cuh"
 #include <string.h>
 #include <vector>
 #include <algorithm>
@@ -46,7 +47,6 @@
 #define SW_SUB (FG_SW2_CW * 32)       // max rows of a sub-block
 #define SW_MAXW 8                     // dependencies per row on the unrolled path
 #define SW_RPT 4                      // rows per consumer thread per pass
-#define FAC_THREADS 1024
 #define SW_RING 4096                  // ring slots (power of two)
 #define SW_NEAR 0x80000000u           // dependency code: ring slot
 #define SW_WAIT_LIMIT (1 << 24)
@@ -866,213 +866,102 @@ __global__ void k_refresh(unsigned char *prog, const long long *val_off, const i
 }
 
 // ---------------------------------------------------------- factor ------
-// IKJ ILU(0) in level order in one block: rows of a level in parallel, one
-// __syncthreads per level; U parts and pivots of earlier levels were written
-// by this block before a barrier, so plain loads see them.  The elimination
-// structure of each row is precompiled (fac_prog): [dpos, ngroups] then per
-// lower entry, in ascending column order, [q, jrow, cnt, (dst, src) x cnt]
-// -- dst the position in row r updated by U(jrow, src) (-1: the pivot) --
-// so a row needs no pattern searches, only independent loads.
-#define FAC_CAP 32
-__global__ void __launch_bounds__(FAC_THREADS, 1)
-k_ilu0_factor_cta(const int *__restrict__ IA, const double *__restrict__ AA,
-                  const int *__restrict__ rows, const int *__restrict__ lev_start, int nlev,
-                  const int *__restrict__ chunk_lev, const int *__restrict__ fac_ptr,
-                  const int *__restrict__ fac_prog, double *LU, double *Dinv, int *err)
+// IKJ ILU(0) as a dataflow of rows (fg_dataflow.cuh): L lanes per row (8, 16
+// or 32, the smallest that holds the longest row), lane q keeping entry q.  A
+// warp takes the next 32 / L rows of one dependency level, and for each lower
+// entry in ascending column order waits for the values of row k it reads --
+// the pivot's inverse in lane "group", U(k, .) in the lanes of the columns both
+// rows have -- and updates its entries, the operations and their order those
+// of ILUp_precond_setup.c:119-139.  What each lane reads is precompiled, so a
+// row needs no pattern searches.
+//
+// What bounds it is the chain of levels: per level one trip of a value
+// through L2 (0.36 us), two dependent rows' groups (three FP64 operations of 31
+// ns each; a warp's FP64 instruction holds this part's FP64 pipe for 64
+// clocks) and the pivot's reciprocal (0.19 us); measured 1.5 us a level.
+// Before it, levels were split over the CTAs of a thread-block cluster with a
+// cluster barrier after each (4.6 us a level), or, for rows of more than 64
+// program words, walked by one CTA (17 us a level).  Measured, before and now:
+// 400x300 transport, one block (1098 levels) 4.80 -> 1.65 ms; 2048x1024 in 32
+// blocks 5.81 -> 2.21 ms; Navier-Stokes 96x96 (27k rows of up to 21 entries)
+// 17.0 -> 1.11 ms.
+#define FAC_CAP 32                    // entries of a row
+#define FAC_TPB 128                   // four warps: one per FP64 pipe
+#define FAC_AHEAD 6                   // levels whose warps are resident (3, 6 and 12 measure within 3 %)
+#define FAC_NONE 0xff                 // position codes: the group leaves the lane's entry alone,
+#define FAC_MULT 0xfe                 // the lane's entry is the group's own (the multiplier)
+
+__global__ void k_ilu0_factor_init(double *LU, long long nnz, double *Dinv, int n, fg_ticket *tk)
 {
-	const int l0 = chunk_lev ? chunk_lev[blockIdx.x] : 0, l1 = chunk_lev ? chunk_lev[blockIdx.x + 1] : nlev;
-	for (int l = l0; l < l1; l++) {
-		int b = lev_start[l], e = lev_start[l + 1];
-		for (int p = b + threadIdx.x; p < e; p += FAC_THREADS) {
-			int r = rows[p];
-			int rb = IA[r], len = IA[r + 1] - rb;
-			double vals[FAC_CAP];
-			for (int q = 0; q < len; q++) vals[q] = AA[rb + q];
-			const int *pr = fac_prog + fac_ptr[p];
-			int dpos = pr[0], ng = pr[1];
-			pr += 2;
-			double d = vals[dpos];
-			for (int g = 0; g < ng; g++) {
-				int q = pr[0], jrow = pr[1], cnt = pr[2];
-				pr += 3;
-				double lq = __dmul_rn(vals[q], Dinv[jrow]);
-				vals[q] = lq;
-				for (int c = 0; c < cnt; c++, pr += 2) {
-					double prod = __dmul_rn(lq, LU[pr[1]]);
-					if (pr[0] < 0) d = __dsub_rn(d, prod);
-					else vals[pr[0]] = __dsub_rn(vals[pr[0]], prod);
+	const long long i0 = blockIdx.x * (long long)blockDim.x + threadIdx.x, st = (long long)gridDim.x * blockDim.x;
+	if (i0 == 0) { tk->next = 0u; tk->abort = 0u; }
+	for (long long i = i0; i < nnz; i += st) LU[i] = __longlong_as_double((long long)FG_UNSET);
+	for (long long i = i0; i < n; i += st) Dinv[i] = __longlong_as_double((long long)FG_UNSET);
+}
+
+__device__ __forceinline__ unsigned fac_code(uint2 c, int k) { return ((k < 4 ? c.x : c.y) >> (8 * (k & 3))) & 255u; }
+
+template <int L>
+__global__ void __launch_bounds__(FAC_TPB)
+k_ilu0_factor_df(const double *__restrict__ AA, const int4 *__restrict__ head, const int2 *__restrict__ grp,
+                 const uint2 *__restrict__ pos, int nslot, double *LU, double *Dinv, fg_ticket *tk, int *err)
+{
+	constexpr int R = 32 / L, NB = L / 8;
+	const int lane = threadIdx.x & 31, q = lane & (L - 1), l0 = lane & ~(L - 1);
+	const unsigned end = (unsigned)(nslot / R);          // slots are padded to whole warps
+	for (;;) {
+		const unsigned t = fg_take(tk, end);
+		if (t >= end) return;
+		const long long sl = (long long)t * R + lane / L;
+		const int4 h = __ldcs(&head[sl]);
+		const int2 g = __ldcs(&grp[sl * L + q]);
+		uint2 code[NB];
+#pragma unroll
+		for (int b = 0; b < NB; b++) code[b] = __ldcs(&pos[(sl * L + q) * NB + b]);
+		const int len = h.y & 255, dpos = (h.y >> 8) & 255, ng = h.y >> 16;
+		const int most = __reduce_max_sync(0xffffffffu, ng);
+		double v = q < len ? __ldcs(&AA[h.x + q]) : 0.0;
+		unsigned long long piv = q < ng ? fg_ld_poll(&Dinv[g.x]) : 0ull;
+#pragma unroll
+		for (int b = 0; b < NB; b++) {
+			unsigned long long u[8];
+#pragma unroll
+			for (int k = 0; k < 8; k++) {
+				const unsigned c = 8 * b < most ? fac_code(code[b], k) : FAC_NONE;
+				const int base = __shfl_sync(0xffffffffu, g.y, l0 + 8 * b + k);
+				u[k] = c < FAC_MULT ? fg_ld_poll(&LU[base + (int)c]) : 0ull;
+			}
+#pragma unroll
+			for (int k = 0; k < 8; k++) {
+				const int gi = 8 * b + k;
+				if (gi < most) {                              // uniform
+					const unsigned c = fac_code(code[b], k);
+					const unsigned own = (__ballot_sync(0xffffffffu, c == FAC_MULT) >> l0) & (0xffffffffu >> (32 - L));
+					const int from = own ? l0 + __ffs(own) - 1 : lane;
+					const int base = __shfl_sync(0xffffffffu, g.y, l0 + gi);
+					unsigned long long uk = u[k];
+					for (int it = 0;; it++) {
+						const bool wu = uk == FG_UNSET, wp = q == gi && piv == FG_UNSET;
+						if (!__any_sync(0xffffffffu, wu || wp)) break;
+						if (!fg_keep_polling(it, tk, err)) return;
+						if (wu) uk = fg_ld_poll(&LU[base + (int)c]);
+						if (wp) piv = fg_ld_poll(&Dinv[g.x]);
+					}
+					const double lq = __dmul_rn(__shfl_sync(0xffffffffu, v, from),
+					                            __shfl_sync(0xffffffffu, __longlong_as_double((long long)piv), l0 + gi));
+					const double w = __dsub_rn(v, __dmul_rn(lq, __longlong_as_double((long long)uk)));
+					v = c == FAC_MULT ? lq : c == FAC_NONE ? v : w;
 				}
 			}
-			for (int q = 0; q < len; q++) LU[rb + q] = (q == dpos) ? d : vals[q];
-			if (d == 0.0) { fg_set_err(err, FEMGPU_E_ZERO_PIVOT); Dinv[r] = 0.0; }
-			else Dinv[r] = 1.0 / d;
 		}
-		__syncthreads();
+		if (q < len) fg_st_value(&LU[h.x + q], v);
+		const double d = __shfl_sync(0xffffffffu, v, l0 + dpos);
+		const double inv = d == 0.0 ? 0.0 : 1.0 / d;
+		if (q == dpos && h.z >= 0) {
+			fg_st_value(&Dinv[h.z], inv);
+			if (d == 0.0) fg_set_err(err, FEMGPU_E_ZERO_PIVOT);
+		}
 	}
-}
-
-// The same factorisation on a thread-block cluster: each level's rows are
-// split over the cluster's CTAs (a single SM's FP64 pipe would otherwise
-// bound it), with one cluster barrier per level.  A row's loads come in three
-// rounds -- its header; its matrix values and elimination program; every
-// operand from earlier levels (pivots and U entries, read from L2: other CTAs
-// wrote them) -- and the first two do not depend on the factorisation, so
-// for each thread's first row of the next level they are issued during the
-// current level (header into registers at its start, values and program by
-// cp.async into the other half of a double buffer before the barrier).  After
-// a barrier only the operand round and the arithmetic remain.  The
-// arithmetic is the reference's, in its order.
-#define FAC2_T 64                     // threads per CTA
-#define FAC2_MAXP 64                  // program ints per row
-#define FAC2_MAXOPS 32                // operands per row
-#define FAC2_BUF (FAC2_T * ((FAC_CAP + 1) * 8 + FAC2_MAXP * 4))
-#define FAC2_SMEM (FAC2_T * FAC2_MAXOPS * 8 + 2 * FAC2_BUF)
-
-__device__ __forceinline__ void cluster_barrier()
-{
-	asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-	asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
-__device__ __forceinline__ unsigned cluster_rank()
-{
-	unsigned r;
-	asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-	return r;
-}
-
-__device__ __forceinline__ unsigned cluster_size()
-{
-	unsigned r;
-	asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
-	return r;
-}
-
-__device__ __forceinline__ void cp_async8(void *dst, const void *src)
-{
-	asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" :: "r"(smem_u32(dst)), "l"(src) : "memory");
-}
-
-__device__ __forceinline__ void cp_async4(void *dst, const void *src)
-{
-	asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" :: "r"(smem_u32(dst)), "l"(src) : "memory");
-}
-
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
-
-__global__ void __launch_bounds__(FAC2_T)
-k_ilu0_factor_cluster(const double *__restrict__ AA, const int *__restrict__ rows,
-                      const int *__restrict__ lev_start, int nlev, const int *__restrict__ chunk_lev,
-                      const int4 *__restrict__ hdr, const int *__restrict__ prog, double *LU, double *Dinv,
-                      int *err)
-{
-	extern __shared__ __align__(16) unsigned char fsm[];
-	// per-thread scratch, element i of thread t at [i * FAC2_T + t] (no bank conflicts)
-	double *so = (double *)fsm + threadIdx.x;
-	unsigned char *bufs = fsm + FAC2_T * FAC2_MAXOPS * 8;
-#define SO(i) so[(i) * FAC2_T]
-#define SV(B, i) ((double *)(bufs + (B) * FAC2_BUF))[(i) * FAC2_T + threadIdx.x]
-#define SP(B, i) ((int *)(bufs + (B) * FAC2_BUF + FAC2_T * (FAC_CAP + 1) * 8))[(i) * FAC2_T + threadIdx.x]
-	const int C = (int)cluster_size(), rank = (int)cluster_rank(), tid = (int)threadIdx.x;
-	// block ILU(0): cluster k factorises matrix block k (its run of levels)
-	const int ck = (int)(blockIdx.x / (unsigned)C);
-	const int L0 = chunk_lev ? chunk_lev[ck] : 0, L1 = chunk_lev ? chunk_lev[ck + 1] : nlev;
-	// level bounds: [b, e) this level, e1 the next level's end, e2 the one after
-	int b = lev_start[L0], e = L1 > L0 ? lev_start[L0 + 1] : b, e1 = L1 > L0 + 1 ? lev_start[L0 + 2] : e;
-	int cur = 0, have = 0;                   // buffer of the prefetched first row; its validity
-	int4 ph = make_int4(0, 0, 0, 0);
-	int pr_ = 0;
-	for (int l = L0; l < L1; l++) {
-		int e2 = (l + 3 <= L1) ? lev_start[l + 3] : e1;
-		int per = (e - b + C - 1) / C, p0 = b + rank * per, p1 = min(e, p0 + per);
-		// round 1 of the next level's first row, into registers
-		int nper = (e1 - e + C - 1) / C, np0 = e + rank * nper, np1 = min(e1, np0 + nper);
-		int np = np0 + tid;
-		bool nhave = (l + 1 < L1) && np < np1;
-		int4 nh = make_int4(0, 0, 0, 0);
-		int nr = 0;
-		if (nhave) { nh = hdr[np]; nr = rows[np]; }
-		for (int p = p0 + tid; p < p1; p += FAC2_T) {
-			int4 h;
-			int r;
-			const int B = cur;
-			if (p == p0 + tid && have) {
-				h = ph; r = pr_;
-				cp_async_wait_all();
-			} else {
-				h = hdr[p]; r = rows[p];
-				const int len0 = h.w & 255;
-				for (int q0 = 0; q0 < len0; q0 += 8) {
-					double t[8];
-#pragma unroll
-					for (int u = 0; u < 8; u++) t[u] = (q0 + u < len0) ? AA[h.x + q0 + u] : 0.0;
-#pragma unroll
-					for (int u = 0; u < 8; u++) if (q0 + u < len0) SV(B, q0 + u) = t[u];
-				}
-				for (int i0 = 0; i0 < h.z; i0 += 8) {
-					int t[8];
-#pragma unroll
-					for (int u = 0; u < 8; u++) t[u] = (i0 + u < h.z) ? prog[h.y + i0 + u] : 0;
-#pragma unroll
-					for (int u = 0; u < 8; u++) if (i0 + u < h.z) SP(B, i0 + u) = t[u];
-				}
-			}
-			const int rb = h.x, len = h.w & 255, dpos = (h.w >> 8) & 255, ng = h.w >> 16;
-			// round 3: pivots (code < 0: -1-row) and U entries of earlier levels
-			const int nops = SP(B, 0);
-			for (int i0 = 0; i0 < nops; i0 += 8) {
-				double t[8];
-#pragma unroll
-				for (int u = 0; u < 8; u++) {
-					int a = (i0 + u < nops) ? SP(B, 1 + i0 + u) : 0;
-					t[u] = (i0 + u < nops) ? __ldcg(a >= 0 ? LU + a : Dinv + (-1 - a)) : 0.0;
-				}
-#pragma unroll
-				for (int u = 0; u < 8; u++) if (i0 + u < nops) SO(i0 + u) = t[u];
-			}
-			// the elimination (ILUp_precond_setup.c:119-139), in the reference's order
-			double d = SV(B, dpos);
-			int gp = 1 + nops, oi = 0;
-			for (int gi = 0; gi < ng; gi++) {
-				int q = SP(B, gp), cnt = SP(B, gp + 1);
-				double lq = __dmul_rn(SV(B, q), SO(oi));
-				oi++;
-				SV(B, q) = lq;
-				for (int c = 0; c < cnt; c++) {
-					double prod = __dmul_rn(lq, SO(oi));
-					oi++;
-					int dst = SP(B, gp + 2 + c);
-					if (dst < 0) d = __dsub_rn(d, prod);
-					else SV(B, dst) = __dsub_rn(SV(B, dst), prod);
-				}
-				gp += 2 + cnt;
-			}
-			for (int q = 0; q < len; q++) LU[rb + q] = (q == dpos) ? d : SV(B, q);
-			if (d == 0.0) { fg_set_err(err, FEMGPU_E_ZERO_PIVOT); Dinv[r] = 0.0; }
-			else Dinv[r] = 1.0 / d;
-		}
-		// round 2 of the next level's first row: cp.async into the other buffer
-		if (nhave) {
-			const int B = cur ^ 1, len = nh.w & 255;
-			for (int q = 0; q < len; q++) cp_async8(&SV(B, q), AA + nh.x + q);
-			for (int i = 0; i < nh.z; i++) cp_async4(&SP(B, i), prog + nh.y + i);
-			cp_async_commit();
-			cur = B;
-		}
-		have = nhave;
-		ph = nh;
-		pr_ = nr;
-		__syncwarp();
-		cluster_barrier();
-		b = e;
-		e = e1;
-		e1 = e2;
-	}
-	cp_async_wait_all();
-#undef SO
-#undef SV
-#undef SP
 }
 
 // ------------------------------------------------------- host: programs
@@ -1768,130 +1657,67 @@ static int build_prog_chain(const int *IA, const int *JA, int n, const ChainLeve
 	return 0;
 }
 
-// Elimination program of every row, in forward level order (the layout
-// k_ilu0_factor_cta reads): the same sequence of updates as
-// ILUp_precond_setup.c:119-139, resolved against the pattern once.
+// Elimination program of every row for k_ilu0_factor_df: the sequence of
+// updates of ILUp_precond_setup.c:119-139, resolved against the pattern once
+// (couplings between matrix blocks dropped).  Slots run over the levels of all
+// matrix blocks side by side (level l of every block, then level l + 1), so the
+// blocks advance together, each level padded to whole warps.
 static int build_factor_prog(const int *IA, const int *JA, int n, const HostLevels &Lo, const Blocks &B,
-                             fg_ilu_sweeps &S)
+                             const std::vector<int> &clev, fg_ilu_sweeps &S)
 {
-	std::vector<int> ptr(n + 1, 0), prog;
-	prog.reserve((size_t)n * 24);
-	for (int p = 0; p < n; p++) {
-		int r = Lo.rows[p], rb = IA[r], len = IA[r + 1] - rb, dpos = -1, ng = 0;
-		if (len > FAC_CAP) return FEMGPU_E_MESH;
-		for (int q = 0; q < len; q++) if (JA[rb + q] == r) dpos = q;
-		if (dpos < 0) return FEMGPU_E_ZERO_PIVOT;           // no diagonal entry
-		ptr[p] = (int)prog.size();
-		size_t hdr = prog.size();
-		prog.push_back(dpos);
-		prog.push_back(0);
-		for (int q = 0; q < len && JA[rb + q] < r; q++) {
-			int jrow = JA[rb + q], cnt = 0;
-			if (!B.same(r, jrow)) continue;              // coupling to another block: dropped
-			size_t g = prog.size();
-			prog.push_back(q);
-			prog.push_back(jrow);
-			prog.push_back(0);
-			for (int k = IA[jrow]; k < IA[jrow + 1]; k++) {
-				int col = JA[k], pos = -1;
-				if (col <= jrow || !B.same(r, col)) continue;
-				for (int m = 0; m < len; m++) if (JA[rb + m] == col) { pos = m; break; }
-				if (pos < 0) continue;
-				prog.push_back(col == r ? -1 : pos);
-				prog.push_back(k);
-				cnt++;
-			}
-			prog[g + 2] = cnt;
-			ng++;
-		}
-		prog[hdr + 1] = ng;
+	int longest = 0, depth = 0;
+	for (int r = 0; r < n; r++) longest = std::max(longest, IA[r + 1] - IA[r]);
+	if (longest > FAC_CAP) return FEMGPU_E_MESH;
+	const int L = longest <= 8 ? 8 : (longest <= 16 ? 16 : 32), R = 32 / L, P = (int)clev.size() - 1;
+	for (int b = 0; b < P; b++) depth = std::max(depth, clev[b + 1] - clev[b]);
+	std::vector<int> slot;                               // row of each slot, -1 padding
+	slot.reserve((size_t)n + (size_t)depth * (R - 1));
+	S.fac_wide = 0;
+	for (int l = 0; l < depth; l++) {
+		const size_t s0 = slot.size();
+		for (int b = 0; b < P; b++)
+			if (clev[b] + l < clev[b + 1])
+				slot.insert(slot.end(), Lo.rows.begin() + Lo.start[clev[b] + l],
+				            Lo.rows.begin() + Lo.start[clev[b] + l + 1]);
+		while (slot.size() % R) slot.push_back(-1);
+		S.fac_wide = std::max(S.fac_wide, (int)(slot.size() - s0));
 	}
-	ptr[n] = (int)prog.size();
-	int rc;
-	if ((rc = up_vec(&S.fac_ptr, ptr))) return rc;
-	return up_vec(&S.fac_prog, prog);
-}
-
-// The elimination program of k_ilu0_factor_cluster: per level-order
-// position a header and a row program whose operand addresses come first
-// (couplings between matrix blocks dropped, as in build_factor_prog).  fac2_ok = 0 when a row exceeds the kernel's per-row capacity.
-static int build_factor_prog2(const int *IA, const int *JA, int n, const HostLevels &Lo, const Blocks &B,
-                              fg_ilu_sweeps &S)
-{
-	std::vector<int> hdr((size_t)n * 4), prog, ops, grp;
-	prog.reserve((size_t)n * 28);
-	S.fac2_ok = 1;
-	for (int p = 0; p < n; p++) {
-		int r = Lo.rows[p], rb = IA[r], len = IA[r + 1] - rb, dpos = -1, ng = 0;
+	const size_t ns = slot.size();
+	std::vector<int> head(4 * ns, 0), grp(2 * ns * L, 0);
+	std::vector<unsigned char> pos(ns * L * L, FAC_NONE);
+	for (size_t s = 0; s < ns; s++) {
+		const int r = slot[s];
+		head[4 * s + 2] = r;
+		if (r < 0) continue;
+		const int rb = IA[r], len = IA[r + 1] - rb;
+		int dpos = -1, ng = 0;
 		for (int q = 0; q < len; q++) if (JA[rb + q] == r) dpos = q;
-		ops.clear();
-		grp.clear();
+		if (dpos < 0) return FEMGPU_E_ZERO_PIVOT;        // no diagonal entry
+		unsigned char *ps = &pos[s * L * L];              // [lane][group]
 		for (int q = 0; q < len && JA[rb + q] < r; q++) {
-			int jrow = JA[rb + q];
-			if (!B.same(r, jrow)) continue;              // coupling to another block: dropped
-			size_t g = grp.size();
-			grp.push_back(q);
-			grp.push_back(0);
-			ops.push_back(-1 - jrow);
+			const int jrow = JA[rb + q];
+			if (!B.same(r, jrow)) continue;
+			grp[2 * (s * L + ng)] = jrow;
+			grp[2 * (s * L + ng) + 1] = IA[jrow];
+			ps[q * L + ng] = FAC_MULT;
 			for (int k = IA[jrow]; k < IA[jrow + 1]; k++) {
-				int col = JA[k], pos = -1;
+				const int col = JA[k];
 				if (col <= jrow || !B.same(r, col)) continue;
-				for (int m = 0; m < len; m++) if (JA[rb + m] == col) { pos = m; break; }
-				if (pos < 0) continue;
-				grp.push_back(col == r ? -1 : pos);
-				ops.push_back(k);
-				grp[g + 1]++;
+				for (int m = 0; m < len; m++)
+					if (JA[rb + m] == col) { ps[m * L + ng] = (unsigned char)(k - IA[jrow]); break; }
 			}
 			ng++;
 		}
-		int plen = 1 + (int)ops.size() + (int)grp.size();
-		if (len > FAC_CAP || dpos < 0 || plen > FAC2_MAXP || (int)ops.size() > FAC2_MAXOPS || ng > 32767) {
-			S.fac2_ok = 0;
-			return 0;
-		}
-		hdr[4 * (size_t)p] = rb;
-		hdr[4 * (size_t)p + 1] = (int)prog.size();
-		hdr[4 * (size_t)p + 2] = plen;
-		hdr[4 * (size_t)p + 3] = len | (dpos << 8) | (ng << 16);
-		prog.push_back((int)ops.size());
-		prog.insert(prog.end(), ops.begin(), ops.end());
-		prog.insert(prog.end(), grp.begin(), grp.end());
+		head[4 * s] = rb;
+		head[4 * s + 1] = len | (dpos << 8) | (ng << 16);
 	}
+	S.fac_lanes = L;
+	S.fac_nslot = (int)ns;
 	int rc;
-	if ((rc = up_vec(&S.fac2_hdr, hdr))) return rc;
-	return up_vec(&S.fac2, prog);
-}
-
-// Cluster size for the factorisation of P matrix blocks (one cluster each):
-// the largest of 16, 8, 4, 2 CTAs with which P clusters fit on the device at
-// once; 0 when none does (the one-block-per-matrix-block kernel runs).
-static int factor_cluster_size(int P)
-{
-	static int init = 0, fits[17];
-	if (!init) {
-		init = 1;
-		if (cudaFuncSetAttribute(k_ilu0_factor_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, FAC2_SMEM) !=
-		    cudaSuccess) { cudaGetLastError(); return 0; }
-		cudaFuncSetAttribute(k_ilu0_factor_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-		cudaGetLastError();
-		for (int c = 16; c >= 1; c /= 2) {
-			cudaLaunchConfig_t cfg = {};
-			cudaLaunchAttribute at[1];
-			at[0].id = cudaLaunchAttributeClusterDimension;
-			at[0].val.clusterDim.x = (unsigned)c; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-			cfg.gridDim = dim3((unsigned)c); cfg.blockDim = dim3(FAC2_T); cfg.dynamicSmemBytes = FAC2_SMEM;
-			cfg.attrs = at; cfg.numAttrs = 1;
-			int ncl = 0;
-			if (cudaOccupancyMaxActiveClusters(&ncl, k_ilu0_factor_cluster, &cfg) == cudaSuccess) fits[c] = ncl;
-			cudaGetLastError();
-		}
-	}
-	// FEMGPU_FACTOR_CLUSTER caps the cluster size (1 allowed: one CTA per
-	// block with the cluster kernel)
-	const char *e = getenv("FEMGPU_FACTOR_CLUSTER");
-	const int cap = e ? atoi(e) : 16;
-	for (int c = 16; c >= (cap == 1 ? 1 : 2); c /= 2)
-		if (c <= cap && fits[c] >= P) return c;
+	if ((rc = up_vec(&S.fac_head, head))) return rc;
+	if ((rc = up_vec(&S.fac_grp, grp))) return rc;
+	if ((rc = up_vec(&S.fac_pos, pos))) return rc;
+	FG_TRY(cudaMalloc(&S.fac_ticket, sizeof(fg_ticket)));
 	return 0;
 }
 
@@ -2126,9 +1952,7 @@ extern "C" int fg_ilu_prepare(femgpu_transport *t, const int *hIA, const int *hJ
 	if ((rc = build_prog<double, false>(hIA, hJA, n, Lo, &Up, B, clo, S.lo64))) return rc;
 	if ((rc = build_prog<float, true>(hIA, hJA, n, Up, nullptr, B, cup, S.up32))) return rc;
 	if ((rc = build_prog<float, false>(hIA, hJA, n, Lo, &Up, B, clo, S.lo32))) return rc;
-	if ((rc = build_factor_prog(hIA, hJA, n, Lo, B, S))) return rc;
-	S.fac2_ok = 0;
-	if ((rc = build_factor_prog2(hIA, hJA, n, Lo, B, S))) return rc;
+	if ((rc = build_factor_prog(hIA, hJA, n, Lo, B, clo, S))) return rc;
 	S.chain = 0;
 	S.ds = 0;
 	size_t nb = (size_t)std::max(Lo.pstart[Lo.nlev], Up.pstart[Up.nlev]) + 64;
@@ -2198,31 +2022,25 @@ extern "C" int fg_ilu0_factor(femgpu_transport *t)
 {
 	cudaStream_t s = t->stream;
 	fg_ilu_sweeps &S = t->sweeps;
-	int P = S.lo64.nchunk, C = S.fac2_ok ? factor_cluster_size(P) : 0;
 	const double *A = t->A;
-	const int *IA = t->IA;
 	if (S.fill) {
 		FG_TRY(cudaMemsetAsync(S.fA, 0, sizeof(double) * ((size_t)S.fnnz + 1), s));
 		k_fill_scatter<<<fg_grid(t->nnz), FG_TPB, 0, s>>>(t->A, S.fmap, t->nnz, S.fA);
 		A = S.fA;
-		IA = S.fIA;
 	}
-	if (C) {
-		cudaLaunchConfig_t cfg = {};
-		cudaLaunchAttribute at[1];
-		at[0].id = cudaLaunchAttributeClusterDimension;
-		at[0].val.clusterDim.x = (unsigned)C; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-		cfg.gridDim = dim3((unsigned)(C * P)); cfg.blockDim = dim3(FAC2_T); cfg.dynamicSmemBytes = FAC2_SMEM;
-		cfg.stream = s; cfg.attrs = at; cfg.numAttrs = 1;
-		FG_TRY(cudaLaunchKernelEx(&cfg, k_ilu0_factor_cluster, A, (const int *)S.lo64.rows,
-		                          (const int *)S.lo64.lev_start, S.lo64.nlev, (const int *)S.lo64.chunk_lev,
-		                          (const int4 *)S.fac2_hdr, (const int *)S.fac2, t->ilu.LU, t->ilu.Dinv,
-		                          &t->st->err));
-	} else {
-		k_ilu0_factor_cta<<<S.lo64.nchunk, FAC_THREADS, 0, s>>>(IA, A, S.lo64.rows, S.lo64.lev_start,
-		                                                       S.lo64.nlev, S.lo64.chunk_lev, S.fac_ptr,
-		                                                       S.fac_prog, t->ilu.LU, t->ilu.Dinv, &t->st->err);
-	}
+	// enough warps for FAC_AHEAD levels: a warp takes its rows, their program
+	// and matrix values while the levels before are computed
+	const int R = 32 / S.fac_lanes, per = FAC_TPB / 32 * R;
+	const long long want = ((long long)FAC_AHEAD * S.fac_wide + per - 1) / per;
+	const int grid = (int)std::min<long long>(std::max<long long>(want, 1), 4 * FG_SMS);
+	fg_ticket *tk = (fg_ticket *)S.fac_ticket;
+	k_ilu0_factor_init<<<fg_grid(t->ilu.nnz), FG_TPB, 0, s>>>(t->ilu.LU, t->ilu.nnz, t->ilu.Dinv, t->neq, tk);
+#define FAC_RUN(L) k_ilu0_factor_df<L><<<grid, FAC_TPB, 0, s>>>(A, (const int4 *)S.fac_head, (const int2 *)S.fac_grp, \
+	(const uint2 *)S.fac_pos, S.fac_nslot, t->ilu.LU, t->ilu.Dinv, tk, &t->st->err)
+	if (S.fac_lanes == 8) FAC_RUN(8);
+	else if (S.fac_lanes == 16) FAC_RUN(16);
+	else FAC_RUN(32);
+#undef FAC_RUN
 	// the double-single chain programs (the FGMRES sweeps) take the new
 	// values now, the others when an application first uses them
 	S.stale = S.chain ? 0xFF : 0x0F;
@@ -2419,8 +2237,8 @@ extern "C" void fg_ilu_free(femgpu_transport *t)
 		memset(all[i], 0, sizeof(fg_sweep));
 	}
 	S.chain = 0;
-	void *v[] = { S.bl64, S.y64, S.o64, S.bl32, S.y32, S.fac_ptr, S.fac_prog, S.fac2_hdr, S.fac2, S.fIA, S.fJA, S.fmap,
-	              S.fA };
+	void *v[] = { S.bl64, S.y64, S.o64, S.bl32, S.y32, S.fac_head, S.fac_grp, S.fac_pos, S.fac_ticket, S.fIA, S.fJA,
+	              S.fmap, S.fA };
 	for (void *q : v) if (q) cudaFree(q);
 	S.bl64 = S.y64 = S.o64 = nullptr;
 	S.bl32 = S.y32 = nullptr;
