@@ -878,13 +878,14 @@ __global__ void k_refresh(unsigned char *prog, const long long *val_off, const i
 // What bounds it is the chain of levels: per level one trip of a value
 // through L2 (0.36 us), two dependent rows' groups (three FP64 operations of 31
 // ns each; a warp's FP64 instruction holds this part's FP64 pipe for 64
-// clocks) and the pivot's reciprocal (0.19 us); measured 1.5 us a level.
+// clocks) and the pivot's reciprocal (0.19 us); measured 1.3 us a level.
 // Before it, levels were split over the CTAs of a thread-block cluster with a
 // cluster barrier after each (4.6 us a level), or, for rows of more than 64
 // program words, walked by one CTA (17 us a level).  Measured, before and now:
-// 400x300 transport, one block (1098 levels) 4.80 -> 1.65 ms; 2048x1024 in 32
-// blocks 5.81 -> 2.21 ms; Navier-Stokes 96x96 (27k rows of up to 21 entries)
-// 17.0 -> 1.11 ms.
+// 400x300 transport, one block (1098 levels) 4.80 -> 1.42 ms; 2048x1024 in 32
+// blocks 5.81 -> 2.2 ms; Navier-Stokes 96x96 (27k rows of up to 21 entries)
+// 17.0 -> 1.00 ms.  (Polling one operand at a time, each missing one costs a
+// trip of its own: 1.65 and 1.11 ms.)
 #define FAC_CAP 32                    // entries of a row
 #define FAC_TPB 128                   // four warps: one per FP64 pipe
 #define FAC_AHEAD 6                   // levels whose warps are resident (3, 6 and 12 measure within 3 %)
@@ -920,16 +921,17 @@ k_ilu0_factor_df(const double *__restrict__ AA, const int4 *__restrict__ head, c
 		for (int b = 0; b < NB; b++) code[b] = __ldcs(&pos[(sl * L + q) * NB + b]);
 		const int len = h.y & 255, dpos = (h.y >> 8) & 255, ng = h.y >> 16;
 		const int most = __reduce_max_sync(0xffffffffu, ng);
-		double v = q < len ? __ldcs(&AA[h.x + q]) : 0.0;
+		double v = q < len ? __ldcs(&AA[h.x + q]) : 1.0;   // (a padding slot's 1/d stays ordinary)
 		unsigned long long piv = q < ng ? fg_ld_poll(&Dinv[g.x]) : 0ull;
 #pragma unroll
 		for (int b = 0; b < NB; b++) {
+			const double *at[8];
 			unsigned long long u[8];
 #pragma unroll
 			for (int k = 0; k < 8; k++) {
 				const unsigned c = 8 * b < most ? fac_code(code[b], k) : FAC_NONE;
-				const int base = __shfl_sync(0xffffffffu, g.y, l0 + 8 * b + k);
-				u[k] = c < FAC_MULT ? fg_ld_poll(&LU[base + (int)c]) : 0ull;
+				at[k] = LU + (__shfl_sync(0xffffffffu, g.y, l0 + 8 * b + k) + (int)c);
+				u[k] = c < FAC_MULT ? fg_ld_poll(at[k]) : 0ull;
 			}
 #pragma unroll
 			for (int k = 0; k < 8; k++) {
@@ -938,28 +940,30 @@ k_ilu0_factor_df(const double *__restrict__ AA, const int4 *__restrict__ head, c
 					const unsigned c = fac_code(code[b], k);
 					const unsigned own = (__ballot_sync(0xffffffffu, c == FAC_MULT) >> l0) & (0xffffffffu >> (32 - L));
 					const int from = own ? l0 + __ffs(own) - 1 : lane;
-					const int base = __shfl_sync(0xffffffffu, g.y, l0 + gi);
-					unsigned long long uk = u[k];
+					// everything still missing is polled again together: operands
+					// that come at the same time cost one trip, not one each
 					for (int it = 0;; it++) {
-						const bool wu = uk == FG_UNSET, wp = q == gi && piv == FG_UNSET;
-						if (!__any_sync(0xffffffffu, wu || wp)) break;
+						if (!__any_sync(0xffffffffu, u[k] == FG_UNSET || (q == gi && piv == FG_UNSET))) break;
 						if (!fg_keep_polling(it, tk, err)) return;
-						if (wu) uk = fg_ld_poll(&LU[base + (int)c]);
-						if (wp) piv = fg_ld_poll(&Dinv[g.x]);
+						if (piv == FG_UNSET) piv = fg_ld_poll(&Dinv[g.x]);
+#pragma unroll
+						for (int m = k; m < 8; m++)
+							if (u[m] == FG_UNSET) u[m] = fg_ld_poll(at[m]);
 					}
 					const double lq = __dmul_rn(__shfl_sync(0xffffffffu, v, from),
 					                            __shfl_sync(0xffffffffu, __longlong_as_double((long long)piv), l0 + gi));
-					const double w = __dsub_rn(v, __dmul_rn(lq, __longlong_as_double((long long)uk)));
+					const double w = __dsub_rn(v, __dmul_rn(lq, __longlong_as_double((long long)u[k])));
 					v = c == FAC_MULT ? lq : c == FAC_NONE ? v : w;
 				}
 			}
 		}
 		if (q < len) fg_st_value(&LU[h.x + q], v);
 		const double d = __shfl_sync(0xffffffffu, v, l0 + dpos);
-		const double inv = d == 0.0 ? 0.0 : 1.0 / d;
+		const bool zero = ((unsigned long long)__double_as_longlong(d) << 1) == 0ull;   // no FP64 compare
+		const double inv = 1.0 / d;
 		if (q == dpos && h.z >= 0) {
-			fg_st_value(&Dinv[h.z], inv);
-			if (d == 0.0) fg_set_err(err, FEMGPU_E_ZERO_PIVOT);
+			fg_st_value(&Dinv[h.z], zero ? 0.0 : inv);
+			if (zero) fg_set_err(err, FEMGPU_E_ZERO_PIVOT);
 		}
 	}
 }
