@@ -11,22 +11,24 @@
 extern "C" {
 #endif
 
-/* A run of consecutive SOR levels: `wide` levels are launched one grid each,
- * a narrow run goes to one thread block that walks its levels in order. */
-typedef struct { int l0, l1, wide; } fg_amg_seg;
+/* The updates of one launch of SOR sweeps in an order in which each comes
+ * after those it reads, levels padded to four: row | second << 30 (second: the update
+ * belongs to the second of two sweeps run together), -1 padding. */
+typedef struct { int *item; int nitem, wide; /* items of the widest level */ } fg_amg_sched;
+
+#define FG_AMG_NW 4
 
 typedef struct fg_amg_level {
-	int n, nnz;
-	/* device: CSR and diagonal (even levels: the ones that are smoothed) */
+	int n, nnz, longest;
+	/* device: CSR, diagonal and its inverse (even levels: the smoothed ones) */
 	int *ptr, *col;
-	double *val, *diag;
-	double *f, *u;
-	/* SOR schedules: rows in processing order, level offsets, segments */
-	int *fw_rows, *fw_lev, *bw_rows, *bw_lev;
-	int fw_nlev, bw_nlev;
-	int *h_fw_lev, *h_bw_lev;
-	fg_amg_seg *fw_seg, *bw_seg;
-	int fw_nseg, bw_nseg;
+	double *val, *diag, *rdiag;
+	double *f;
+	double *w[FG_AMG_NW];        /* iterates of the SOR sweeps (in the arena) */
+	double *u;                   /* the current one                          */
+	/* SOR schedules of the forward and reverse sweeps: [0] one sweep (nr
+	 * odd), [1] two sweeps together (nr >= 2) */
+	fg_amg_sched fw[2], bw[2];
 	/* even l below the coarsest: restriction to level l+2 (4 fine rows per
 	 * level-(l+2) row, -1 where absent) and the composite aggregate map */
 	int4 *quad;
@@ -43,6 +45,11 @@ struct femgpu_amg {
 	int nlevels;                 /* 2*ncl + 1 matrices */
 	fg_amg_level *lv;
 	double *qcopy;               /* [n0]: the input when q and z alias */
+	double *arena;               /* the levels' w vectors */
+	long long narena;
+	void *ticket;                /* [nticket] fg_ticket, one per SOR launch of a cycle */
+	int nticket;
+	int *err;                    /* FEMGPU_E_TIMEOUT after a wait that ran out */
 	cudaStream_t stream, own_stream;
 };
 

@@ -430,57 +430,63 @@ static int galerkin(const hmat *A, const int *rmatch, hmat *C)
 	return 0;
 }
 
-/* ---- level schedules of the SOR sweeps -------------------------------------- */
-/* Rows in the order a level-by-level sweep processes them; lev [nlev+1].  In
- * the forward sweep (SOR_relax) every coupled pair (i, j), i < j, in either
- * row's pattern orders i before j: j reads the new u[i], i the old u[j].  The
- * reverse sweep (SOR_relax_rev) orders j before i. */
-static int sor_levels(const hmat *A, int reverse, int **rows_out, int **lev_out, int *nlev_out)
+/* ---- schedules of the SOR sweeps --------------------------------------------- */
+/* Level of a row's update: one more than the deepest update it reads.  In a
+ * forward sweep (SOR_relax) row i reads this sweep's value of the rows before it
+ * in its pattern, in a reverse one (SOR_relax_rev) of the rows after it; the
+ * other rows' values, and its own, are the previous sweep's (prev: their
+ * levels, or NULL when they are the launch's input). */
+static void sweep_levels(const hmat *A, int reverse, const int *prev, int *lv)
 {
-	int n = A->n, i, nlev = 0;
-	int *lv = calloc((size_t)(n ? n : 1), sizeof(int)), *cnt, *rows, *fill;
-	if (!lv) return FEMGPU_E_NOMEM;
+	int n = A->n;
 	for (int s = 0; s < n; s++) {
-		int r = reverse ? n - 1 - s : s;
-		for (int k = A->ptr[r]; k < A->ptr[r + 1]; k++) {     /* earlier rows of r's own pattern */
+		int r = reverse ? n - 1 - s : s, L = prev ? prev[r] + 1 : 0;
+		for (int k = A->ptr[r]; k < A->ptr[r + 1]; k++) {
 			int c = A->col[k];
-			if ((reverse ? c > r : c < r) && lv[c] + 1 > lv[r]) lv[r] = lv[c] + 1;
+			if (c == r) continue;
+			if (reverse ? c > r : c < r) { if (lv[c] + 1 > L) L = lv[c] + 1; }
+			else if (prev && prev[c] + 1 > L) L = prev[c] + 1;
 		}
-		for (int k = A->ptr[r]; k < A->ptr[r + 1]; k++) {     /* later rows r appears in */
-			int c = A->col[k];
-			if ((reverse ? c < r : c > r) && lv[r] + 1 > lv[c]) lv[c] = lv[r] + 1;
-		}
-		if (lv[r] + 1 > nlev) nlev = lv[r] + 1;
+		lv[r] = L;
 	}
-	cnt = calloc((size_t)nlev + 1, sizeof(int));
-	rows = malloc(sizeof(int) * (size_t)(n ? n : 1));
-	fill = malloc(sizeof(int) * (size_t)nlev + 1);
-	if (!cnt || !rows || !fill) return FEMGPU_E_NOMEM;
-	for (i = 0; i < n; i++) cnt[lv[i] + 1]++;
-	for (i = 0; i < nlev; i++) cnt[i + 1] += cnt[i];
-	memcpy(fill, cnt, sizeof(int) * (size_t)nlev);
-	for (int s = 0; s < n; s++) { int r = reverse ? n - 1 - s : s; rows[fill[lv[r]]++] = r; }
-	free(lv); free(fill);
-	*rows_out = rows; *lev_out = cnt; *nlev_out = nlev;
-	return 0;
 }
 
-/* Runs of levels: a level wider than AMG_WIDE rows is its own grid launch,
- * the levels between wide ones go to one thread block. */
-#define AMG_WIDE 8192
-static int segments(const int *lev, int nlev, fg_amg_seg **out, int *nout)
+/* The updates of `sweeps' (1 or 2) sweeps run together, level by level, each
+ * level padded to the four rows a warp takes at most.  Two sweeps take a few levels more than one:
+ * the second follows the first as soon as the values it reads are there. */
+static int sor_schedule(const hmat *A, int reverse, int sweeps, fg_amg_sched *S)
 {
-	int ns = 0;
-	fg_amg_seg *s = malloc(sizeof(fg_amg_seg) * (size_t)(nlev ? nlev : 1));
-	if (!s) return FEMGPU_E_NOMEM;
-	for (int l = 0; l < nlev;) {
-		if (lev[l + 1] - lev[l] > AMG_WIDE) { s[ns].l0 = l; s[ns].l1 = l + 1; s[ns].wide = 1; ns++; l++; continue; }
-		s[ns].l0 = l;
-		while (l < nlev && lev[l + 1] - lev[l] <= AMG_WIDE) l++;
-		s[ns].l1 = l; s[ns].wide = 0; ns++;
+	int n = A->n, top = 0, rc = FEMGPU_E_NOMEM, *item = NULL, *at = NULL;
+	int *lv = malloc(sizeof(int) * (size_t)sweeps * (size_t)n);
+	if (!lv) return rc;
+	for (int s = 0; s < sweeps; s++) sweep_levels(A, reverse, s ? lv : NULL, lv + (size_t)s * n);
+	for (int i = 0; i < sweeps * n; i++) if (lv[i] + 1 > top) top = lv[i] + 1;
+	at = calloc((size_t)top + 1, sizeof(int));
+	if (at) {
+		long long total = 0;
+		for (int i = 0; i < sweeps * n; i++) at[lv[i]]++;
+		S->wide = 0;
+		for (int l = 0; l < top; l++) {
+			int c = (at[l] + 3) & ~3;
+			if (c > S->wide) S->wide = c;
+			at[l] = (int)total;
+			total += c;
+		}
+		if (total < 0x7fffffff && (item = malloc(sizeof(int) * (size_t)total))) {
+			memset(item, 0xff, sizeof(int) * (size_t)total);
+			for (int s = 0; s < sweeps; s++)
+				for (int q = 0; q < n; q++) {
+					int i = reverse ? n - 1 - q : q;
+					item[at[lv[(size_t)s * n + i]]++] = i | s << 30;
+				}
+			S->nitem = (int)total;
+			rc = fgh_dmalloc((void **)&S->item, sizeof(int) * (size_t)total);
+			if (!rc && cudaMemcpy(S->item, item, sizeof(int) * (size_t)total, cudaMemcpyHostToDevice) != cudaSuccess)
+				rc = FEMGPU_E_CUDA;
+		}
 	}
-	*out = s; *nout = ns;
-	return 0;
+	free(lv); free(at); free(item);
+	return rc;
 }
 
 /* ---- host utilities (no GPU) ---------------------------------------------- */
@@ -540,16 +546,18 @@ static void free_levels(femgpu_amg *g)
 {
 	for (int l = 0; l < g->nlevels; l++) {
 		fg_amg_level *L = &g->lv[l];
-		void *p[] = { L->ptr, L->col, L->val, L->diag, L->fw_rows, L->fw_lev, L->bw_rows, L->bw_lev,
-		              L->quad, L->agg2, l ? L->f : NULL, l ? L->u : NULL };
+		void *p[] = { L->ptr, L->col, L->val, L->diag, L->rdiag, L->fw[0].item, L->fw[1].item, L->bw[0].item,
+		              L->bw[1].item, L->quad, L->agg2, l ? L->f : NULL };
 		for (int i = 0; i < (int)(sizeof p / sizeof p[0]); i++) if (p[i]) cudaFree(p[i]);
 		free(L->h_ptr); free(L->h_col); free(L->h_val); free(L->h_match);
-		free(L->h_fw_lev); free(L->h_bw_lev); free(L->fw_seg); free(L->bw_seg);
 	}
 	free(g->lv);
 	g->lv = NULL;
 	g->nlevels = 0;
 	if (g->qcopy) { cudaFree(g->qcopy); g->qcopy = NULL; }
+	if (g->arena) { cudaFree(g->arena); g->arena = NULL; }
+	if (g->ticket) { cudaFree(g->ticket); g->ticket = NULL; }
+	if (g->err) { cudaFree(g->err); g->err = NULL; }
 }
 
 int femgpu_amg_create(femgpu_amg **out, int ncl, double beta, double omega, int nr)
@@ -585,36 +593,51 @@ int femgpu_amg_set_stream(femgpu_amg *g, void *stream)
 	return 0;
 }
 
-/* Device copy of a smoothed level: CSR, diagonal, SOR schedules; f and u
- * except on level 0 (the caller's vectors). */
+/* Device copy of a smoothed level: CSR, diagonal and its inverse, SOR
+ * schedules; f except on level 0 (the caller's vector). */
 static int upload_level(femgpu_amg *g, int l, fg_amg_level *D, const hmat *A)
 {
-	int *rows, *lev, nlev, rc;
+	int rc = 0;
+	double *rdiag = malloc(sizeof(double) * (size_t)A->n);
+	if (!rdiag) return FEMGPU_E_NOMEM;
+	for (int i = 0; i < A->n; i++) {
+		rdiag[i] = 1.0 / A->diag[i];
+		if (A->ptr[i + 1] - A->ptr[i] > D->longest) D->longest = A->ptr[i + 1] - A->ptr[i];
+	}
+	rc = fgh_dmalloc((void **)&D->rdiag, sizeof(double) * (size_t)A->n);
+	if (!rc && cudaMemcpy(D->rdiag, rdiag, sizeof(double) * (size_t)A->n, cudaMemcpyHostToDevice) != cudaSuccess)
+		rc = FEMGPU_E_CUDA;
+	free(rdiag);
+	if (rc) return rc;
 	UP(D->ptr, A->ptr, sizeof(int) * ((size_t)A->n + 1));
 	UP(D->col, A->col, sizeof(int) * (size_t)(A->nnz ? A->nnz : 1));
 	UP(D->val, A->val, sizeof(double) * (size_t)(A->nnz ? A->nnz : 1));
 	UP(D->diag, A->diag, sizeof(double) * (size_t)A->n);
-	if (l) { DM(D->f, sizeof(double) * (size_t)A->n); DM(D->u, sizeof(double) * (size_t)A->n); }
-	if ((rc = sor_levels(A, 0, &rows, &lev, &nlev))) return rc;
-	D->h_fw_lev = lev; D->fw_nlev = nlev;
-	rc = segments(lev, nlev, &D->fw_seg, &D->fw_nseg);
-	if (!rc) rc = fgh_dmalloc((void **)&D->fw_rows, sizeof(int) * (size_t)A->n);
-	if (!rc) rc = fgh_dmalloc((void **)&D->fw_lev, sizeof(int) * ((size_t)nlev + 1));
-	if (!rc && (cudaMemcpy(D->fw_rows, rows, sizeof(int) * (size_t)A->n, cudaMemcpyHostToDevice) != cudaSuccess ||
-	            cudaMemcpy(D->fw_lev, lev, sizeof(int) * ((size_t)nlev + 1), cudaMemcpyHostToDevice) != cudaSuccess))
-		rc = FEMGPU_E_CUDA;
-	free(rows);
-	if (rc) return rc;
-	if ((rc = sor_levels(A, 1, &rows, &lev, &nlev))) return rc;
-	D->h_bw_lev = lev; D->bw_nlev = nlev;
-	rc = segments(lev, nlev, &D->bw_seg, &D->bw_nseg);
-	if (!rc) rc = fgh_dmalloc((void **)&D->bw_rows, sizeof(int) * (size_t)A->n);
-	if (!rc) rc = fgh_dmalloc((void **)&D->bw_lev, sizeof(int) * ((size_t)nlev + 1));
-	if (!rc && (cudaMemcpy(D->bw_rows, rows, sizeof(int) * (size_t)A->n, cudaMemcpyHostToDevice) != cudaSuccess ||
-	            cudaMemcpy(D->bw_lev, lev, sizeof(int) * ((size_t)nlev + 1), cudaMemcpyHostToDevice) != cudaSuccess))
-		rc = FEMGPU_E_CUDA;
-	free(rows);
-	return rc;
+	if (l) DM(D->f, sizeof(double) * (size_t)A->n);
+	if (g->nr & 1) {
+		if ((rc = sor_schedule(A, 0, 1, &D->fw[0])) || (rc = sor_schedule(A, 1, 1, &D->bw[0]))) return rc;
+	}
+	if (g->nr > 1) {
+		if ((rc = sor_schedule(A, 0, 2, &D->fw[1])) || (rc = sor_schedule(A, 1, 2, &D->bw[1]))) return rc;
+	}
+	return 0;
+}
+
+/* The SOR iterates of every smoothed level, in one allocation (a cycle marks
+ * them unset with one kernel), and the launches' tickets. */
+static int alloc_cycle(femgpu_amg *g)
+{
+	long long n = 0, at = 0;
+	for (int l = 0; l < g->nlevels; l += 2) n += (g->lv[l].n + 1) & ~1;
+	g->narena = FG_AMG_NW * n;
+	DM(g->arena, sizeof(double) * (size_t)g->narena);
+	for (int l = 0; l < g->nlevels; l += 2)
+		for (int k = 0; k < FG_AMG_NW; k++, at += (g->lv[l].n + 1) & ~1) g->lv[l].w[k] = g->arena + at;
+	g->nticket = (g->nlevels + 1) * ((g->nr + 1) / 2);
+	DM(g->ticket, 8 * (size_t)g->nticket);
+	DM(g->err, sizeof(int));
+	CK(cudaMemsetAsync(g->err, 0, sizeof(int), g->stream));
+	return 0;
 }
 
 /* Restriction and prolongation between smoothed levels l and l+2: the <= 4
@@ -698,6 +721,7 @@ int femgpu_amg_setup(femgpu_amg *g, int n, const int *IA, const int *JA, const d
 		H[l].ptr = NULL; H[l].col = NULL; H[l].val = NULL;
 	}
 	if (!rc) rc = fgh_dmalloc((void **)&g->qcopy, sizeof(double) * (size_t)n);
+	if (!rc) rc = alloc_cycle(g);
 	if (!rc && cudaStreamSynchronize(g->stream) != cudaSuccess) rc = FEMGPU_E_CUDA;
 	for (l = 0; l < L; l++) { free(H[l].ptr); free(H[l].col); free(H[l].val); free(H[l].diag); }
 	free(H);
@@ -731,7 +755,7 @@ int femgpu_amg_apply_dev(femgpu_amg *g, const double *q, double *z)
 int femgpu_amg_apply(femgpu_amg *g, const double *q_host, double *z_host)
 {
 	double *q = NULL, *z = NULL;
-	int rc, n;
+	int rc, n, err = 0;
 	if (!g || !q_host || !z_host || !g->nlevels) return FEMGPU_E_ARG;
 	n = g->lv[0].n;
 	if ((rc = fgh_dmalloc((void **)&q, sizeof(double) * (size_t)n)) ||
@@ -740,8 +764,10 @@ int femgpu_amg_apply(femgpu_amg *g, const double *q_host, double *z_host)
 	CK(cudaMemcpyAsync(q, q_host, sizeof(double) * (size_t)n, cudaMemcpyHostToDevice, g->stream));
 	rc = femgpu_amg_apply_dev(g, q, z);
 	if (!rc) CK(cudaMemcpyAsync(z_host, z, sizeof(double) * (size_t)n, cudaMemcpyDeviceToHost, g->stream));
+	if (!rc) CK(cudaMemcpyAsync(&err, g->err, sizeof(int), cudaMemcpyDeviceToHost, g->stream));
 	CK(cudaStreamSynchronize(g->stream));
 	cudaFree(q);
 	cudaFree(z);
+	if (err) { fgh_set_error("device reported error %d", err); return err; }
 	return rc;
 }
