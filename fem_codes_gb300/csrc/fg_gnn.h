@@ -7,7 +7,7 @@
  * off-diagonal CSR graph gptr [n+1], gcol [E], edge weights wA, wT [E] (FP32),
  * diagonal d [n]; activations h [L+1][n][32], m1, m2 [L][n][32] (bf16 or
  * FP32), ReLU masks [L+1][n] (one bit per feature), encoder inputs x [n]
- * (float2); gradients gh [2][n][32], gm1, gm2 [n][32] (FP32). */
+ * (float2); gradients gh [2][n][32] (FP32). */
 #ifndef FG_GNN_H
 #define FG_GNN_H
 #include <cuda_runtime_api.h>
@@ -27,6 +27,9 @@ extern "C" {
 #define GNN_OFF_BD (GNN_OFF_WD + 32)
 #define GNN_NPARAMS (GNN_OFF_BD + 1)
 #define GNN_RED_BLOCKS 304
+#define GNN_BWD_BLOCKS 304      /* most blocks of a backward kernel               */
+#define GNN_PART (GNN_BWD_BLOCKS * (GNN_LAYERS * GNN_LAYER_SIZE + 33 + 96) + 32)   /* partial sums of a
+                                                              backward pass    */
 #define GNN_LOSS_SUPERVISED 0   /* ||z - t||^2 / ||t||^2, t = M^-1 v (ILU target) */
 #define GNN_LOSS_RESIDUAL 1     /* ||A z - v||^2 / ||v||^2                      */
 #define GNN_LOSS_BOTH 2         /* the sum of the two                           */
@@ -44,10 +47,11 @@ struct femgpu_gnn {
 	void *h[GNN_LAYERS + 1], *m1[GNN_LAYERS], *m2[GNN_LAYERS];
 	unsigned *mask[GNN_LAYERS + 1];
 	void *x;                       /* float2 [n]                              */
-	float *gh[2], *gm1, *gm2;
+	float *gh[2];
 	float *part;                   /* weight-gradient partial sums            */
 	double *rpart;                 /* [2*GNN_RED_BLOCKS] reduction partials   */
-	double *sums, *stats;          /* [2] each (device)                       */
+	double *sums, *stats;          /* [2]; rms(r), mean |a_ii|, 1 / rms(r)    */
+	unsigned *ticket;              /* blocks done of a reduction              */
 	double *lsums, *lsums2;        /* [4] loss sums: supervised / residual    */
 	double *gz, *res;              /* [n] dL/dz, A z - v                      */
 	int loss_kind;                 /* GNN_LOSS_*                              */

@@ -24,7 +24,7 @@ static void free_graph(fg_gnn *g)
 	FREE(g->gptr); FREE(g->gcol); FREE(g->wA); FREE(g->wT); FREE(g->d); FREE(g->x);
 	for (l = 0; l <= GNN_LAYERS; l++) { FREE(g->h[l]); FREE(g->mask[l]); }
 	for (l = 0; l < GNN_LAYERS; l++) { FREE(g->m1[l]); FREE(g->m2[l]); }
-	FREE(g->gh[0]); FREE(g->gh[1]); FREE(g->gm1); FREE(g->gm2); FREE(g->gz); FREE(g->res);
+	FREE(g->gh[0]); FREE(g->gh[1]); FREE(g->gz); FREE(g->res);
 	g->cap_n = g->cap_e = 0;
 }
 
@@ -35,12 +35,14 @@ static int create(fg_gnn *g, int bf16_act, const float *theta)
 	CK(cudaStreamCreateWithFlags(&g->own_stream, cudaStreamNonBlocking));
 	g->stream = g->own_stream;
 	DM(g->theta, P); DM(g->grad, P); DM(g->am, P); DM(g->av, P);
-	DM(g->part, sizeof(float) * GNN_RED_BLOCKS * GNN_LAYER_SIZE);
+	DM(g->part, sizeof(float) * GNN_PART);
 	DM(g->rpart, sizeof(double) * 2 * GNN_RED_BLOCKS);
-	DM(g->sums, sizeof(double) * 2); DM(g->stats, sizeof(double) * 2);
+	DM(g->sums, sizeof(double) * 2); DM(g->stats, sizeof(double) * 3);
+	DM(g->ticket, sizeof(unsigned));
 	DM(g->lsums, sizeof(double) * 4); DM(g->lsums2, sizeof(double) * 4);
 	DM(g->err, sizeof(int));
 	CK(cudaMemsetAsync(g->err, 0, sizeof(int), g->stream));
+	CK(cudaMemsetAsync(g->ticket, 0, sizeof(unsigned), g->stream));
 	CK(cudaMemsetAsync(g->grad, 0, P, g->stream));
 	return femgpu_gnn_set_params(g, theta);
 }
@@ -65,7 +67,7 @@ void femgpu_gnn_destroy(femgpu_gnn *g)
 	if (g->stream) cudaStreamSynchronize(g->stream);
 	free_graph(g);
 	FREE(g->theta); FREE(g->grad); FREE(g->am); FREE(g->av); FREE(g->part); FREE(g->rpart);
-	FREE(g->sums); FREE(g->lsums); FREE(g->lsums2); FREE(g->stats); FREE(g->err);
+	FREE(g->sums); FREE(g->lsums); FREE(g->lsums2); FREE(g->stats); FREE(g->ticket); FREE(g->err);
 	if (g->own_stream) cudaStreamDestroy(g->own_stream);
 	free(g);
 }
@@ -128,7 +130,6 @@ static int ensure(fg_gnn *g, int n, int ne)
 		DM(g->m2[l], sa * row * (size_t)n);
 	}
 	DM(g->gh[0], 4 * row * (size_t)n); DM(g->gh[1], 4 * row * (size_t)n);
-	DM(g->gm1, 4 * row * (size_t)n); DM(g->gm2, 4 * row * (size_t)n);
 	DM(g->gz, sizeof(double) * (size_t)n); DM(g->res, sizeof(double) * (size_t)n);
 	g->cap_n = n;
 	g->cap_e = ne;
