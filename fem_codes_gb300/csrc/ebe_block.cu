@@ -30,9 +30,10 @@ __global__ void k_lm_blk(int ndof, int nel, const int *vert, const int *node_id,
 template <int NDOF, bool OFFDIAG>
 __global__ void k_ebemv_blk(int neq, const int *__restrict__ ri_ptr, const int *__restrict__ ri,
                             const int *__restrict__ lm, const double *__restrict__ A,
-                            const double *__restrict__ P, double *__restrict__ Q)
+                            const double *__restrict__ P, double *__restrict__ Q, const int *active)
 {
 	constexpr int M = 3 * NDOF;
+	if (active && !*active) return;
 	for (int I = blockIdx.x * blockDim.x + threadIdx.x; I <= neq; I += gridDim.x * blockDim.x) {
 		double q = 0.0;
 		if (I < neq) {
@@ -64,9 +65,10 @@ __global__ void k_ebemv_blk(int neq, const int *__restrict__ ri_ptr, const int *
 template <int NDOF>
 __global__ void k_ebemv_blk32(int neq, const int *__restrict__ ri_ptr, const int *__restrict__ ri,
                               const int *__restrict__ lm, const float *__restrict__ A,
-                              const float *__restrict__ P, double *__restrict__ Q)
+                              const float *__restrict__ P, double *__restrict__ Q, const int *active)
 {
 	constexpr int M = 3 * NDOF;
+	if (active && !*active) return;
 	for (int I = blockIdx.x * blockDim.x + threadIdx.x; I <= neq; I += gridDim.x * blockDim.x) {
 		double q = 0.0;
 		if (I < neq) {
@@ -187,12 +189,15 @@ __global__ void k_blockdiag_invert(int nnodes, const double *BD, double *invBD)
 
 // MODE 0: z = D^-1 p (BlockDiag_precond), 1: z = p + D^-1 z (BlockDiag2_precond,
 // z holds the off-diagonal product), 2: z += D p (NOBlockDiag2_precond).  Per
-// node; the dump equation neq is never written (zeroed separately).
+// node; the dump equation z[neq] = 0 is written here when p and z are apart
+// (a node's column may read p[neq]), by k_zero_one otherwise.
 template <int NDOF, int MODE>
 __global__ void k_blockdiag_apply(int nnodes, int neq, const int *node_id, const double *B,
-                                  const double *p, double *z)
+                                  const double *p, double *z, const int *active)
 {
 	constexpr int D2 = NDOF * NDOF;
+	if (active && !*active) return;
+	if (p != z && blockIdx.x == 0 && threadIdx.x == 0) z[neq] = 0.0;
 	for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < nnodes; n += gridDim.x * blockDim.x) {
 		int id[NDOF];
 		double v[NDOF];
@@ -223,14 +228,15 @@ __global__ void k_blockdiag_apply(int nnodes, int neq, const int *node_id, const
 }
 
 __global__ void k_zero_one(double *z, int i) { z[i] = 0.0; }
-__global__ void k_zero_one32(float *z, int i) { z[i] = 0.0f; }
 
 // z = D^-1 p per node (BlockDiag_precond's arithmetic), stored in FP32.
 template <int NDOF>
 __global__ void k_blockdiag_apply32(int nnodes, int neq, const int *node_id, const double *B, const double *p,
-                                    float *z)
+                                    float *z, const int *active)
 {
 	constexpr int D2 = NDOF * NDOF;
+	if (active && !*active) return;
+	if (blockIdx.x == 0 && threadIdx.x == 0) z[neq] = 0.0f;
 	for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < nnodes; n += gridDim.x * blockDim.x) {
 		int id[NDOF];
 		double v[NDOF];
@@ -264,14 +270,14 @@ extern "C" int fg_ebe_lm(femgpu_ebe *c)
 	return fg_invert_map(c->vert, 1, 3 * c->nel, c->nnodes, &c->ni_ptr, &c->ni, c->stream);
 }
 
-extern "C" int fg_ebe_matvec(femgpu_ebe *c, const double *P, double *Q, int offdiag)
+extern "C" int fg_ebe_matvec(femgpu_ebe *c, const double *P, double *Q, int offdiag, const int *active)
 {
 	int g = fg_grid(c->neq + 1LL, 128, 32);
 	if (c->ndof == 4) {
-		if (offdiag) k_ebemv_blk<4, true><<<g, 128, 0, c->stream>>>(c->neq, c->ri_ptr, c->ri, c->lm, c->A, P, Q);
-		else k_ebemv_blk<4, false><<<g, 128, 0, c->stream>>>(c->neq, c->ri_ptr, c->ri, c->lm, c->A, P, Q);
+		if (offdiag) k_ebemv_blk<4, true><<<g, 128, 0, c->stream>>>(c->neq, c->ri_ptr, c->ri, c->lm, c->A, P, Q, active);
+		else k_ebemv_blk<4, false><<<g, 128, 0, c->stream>>>(c->neq, c->ri_ptr, c->ri, c->lm, c->A, P, Q, active);
 	} else {
-		k_ebemv_blk<3, false><<<g, 128, 0, c->stream>>>(c->neq, c->ri_ptr, c->ri, c->lm, c->A, P, Q);
+		k_ebemv_blk<3, false><<<g, 128, 0, c->stream>>>(c->neq, c->ri_ptr, c->ri, c->lm, c->A, P, Q, active);
 	}
 	return (int)cudaGetLastError();
 }
@@ -330,18 +336,18 @@ extern "C" int fg_ebe_blockdiag_setup(femgpu_ebe *c)
 	return (int)cudaGetLastError();
 }
 
-extern "C" int fg_ebe_blockdiag_apply(femgpu_ebe *c, const double *p, double *z, int mode)
+extern "C" int fg_ebe_blockdiag_apply(femgpu_ebe *c, const double *p, double *z, int mode, const int *active)
 {
 	int g = fg_grid(c->nnodes);
 	const double *B = (mode == 2) ? c->BD : c->invBD;
 	if (c->ndof == 4) {
-		if (mode == 0) k_blockdiag_apply<4, 0><<<g, FG_TPB, 0, c->stream>>>(c->nnodes, c->neq, c->node_id, B, p, z);
-		else if (mode == 1) k_blockdiag_apply<4, 1><<<g, FG_TPB, 0, c->stream>>>(c->nnodes, c->neq, c->node_id, B, p, z);
-		else k_blockdiag_apply<4, 2><<<g, FG_TPB, 0, c->stream>>>(c->nnodes, c->neq, c->node_id, B, p, z);
+		if (mode == 0) k_blockdiag_apply<4, 0><<<g, FG_TPB, 0, c->stream>>>(c->nnodes, c->neq, c->node_id, B, p, z, active);
+		else if (mode == 1) k_blockdiag_apply<4, 1><<<g, FG_TPB, 0, c->stream>>>(c->nnodes, c->neq, c->node_id, B, p, z, active);
+		else k_blockdiag_apply<4, 2><<<g, FG_TPB, 0, c->stream>>>(c->nnodes, c->neq, c->node_id, B, p, z, active);
 	} else {
-		k_blockdiag_apply<3, 0><<<g, FG_TPB, 0, c->stream>>>(c->nnodes, c->neq, c->node_id, B, p, z);
+		k_blockdiag_apply<3, 0><<<g, FG_TPB, 0, c->stream>>>(c->nnodes, c->neq, c->node_id, B, p, z, active);
 	}
-	k_zero_one<<<1, 1, 0, c->stream>>>(z, c->neq);
+	if (p == z) k_zero_one<<<1, 1, 0, c->stream>>>(z, c->neq);
 	return (int)cudaGetLastError();
 }
 
@@ -353,20 +359,19 @@ extern "C" int fg_ebe_to_f32(femgpu_ebe *c)
 	return (int)cudaGetLastError();
 }
 
-extern "C" int fg_ebe_matvec32(femgpu_ebe *c, const float *P, double *Q)
+extern "C" int fg_ebe_matvec32(femgpu_ebe *c, const float *P, double *Q, const int *active)
 {
 	int g = fg_grid(c->neq + 1LL, 128, 32);
 	if (!c->A32) return FEMGPU_E_NOT_BUILT;
-	if (c->ndof == 4) k_ebemv_blk32<4><<<g, 128, 0, c->stream>>>(c->neq, c->ri_ptr, c->ri, c->lm, c->A32, P, Q);
-	else k_ebemv_blk32<3><<<g, 128, 0, c->stream>>>(c->neq, c->ri_ptr, c->ri, c->lm, c->A32, P, Q);
+	if (c->ndof == 4) k_ebemv_blk32<4><<<g, 128, 0, c->stream>>>(c->neq, c->ri_ptr, c->ri, c->lm, c->A32, P, Q, active);
+	else k_ebemv_blk32<3><<<g, 128, 0, c->stream>>>(c->neq, c->ri_ptr, c->ri, c->lm, c->A32, P, Q, active);
 	return (int)cudaGetLastError();
 }
 
-extern "C" int fg_ebe_blockdiag_apply32(femgpu_ebe *c, const double *p, float *z)
+extern "C" int fg_ebe_blockdiag_apply32(femgpu_ebe *c, const double *p, float *z, const int *active)
 {
 	int g = fg_grid(c->nnodes);
-	if (c->ndof == 4) k_blockdiag_apply32<4><<<g, FG_TPB, 0, c->stream>>>(c->nnodes, c->neq, c->node_id, c->invBD, p, z);
-	else k_blockdiag_apply32<3><<<g, FG_TPB, 0, c->stream>>>(c->nnodes, c->neq, c->node_id, c->invBD, p, z);
-	k_zero_one32<<<1, 1, 0, c->stream>>>(z, c->neq);
+	if (c->ndof == 4) k_blockdiag_apply32<4><<<g, FG_TPB, 0, c->stream>>>(c->nnodes, c->neq, c->node_id, c->invBD, p, z, active);
+	else k_blockdiag_apply32<3><<<g, FG_TPB, 0, c->stream>>>(c->nnodes, c->neq, c->node_id, c->invBD, p, z, active);
 	return (int)cudaGetLastError();
 }

@@ -25,17 +25,18 @@ struct femgpu_ebe {
 };
 
 int fg_ebe_lm(femgpu_ebe *c);
-int fg_ebe_matvec(femgpu_ebe *c, const double *P, double *Q, int offdiag);
+/* active (device flag, may be NULL): the kernels do nothing while it is 0. */
+int fg_ebe_matvec(femgpu_ebe *c, const double *P, double *Q, int offdiag, const int *active);
 int fg_ebe_blockdiag_setup(femgpu_ebe *c);
 /* Block_scaling_EBE's element step (ndof 4): identity rows/columns for the
  * prescribed dofs, each vertex's row block times its invBD. */
 int fg_ebe_block_scale(femgpu_ebe *c);
-int fg_ebe_blockdiag_apply(femgpu_ebe *c, const double *p, double *z, int mode);
+int fg_ebe_blockdiag_apply(femgpu_ebe *c, const double *p, double *z, int mode, const int *active);
 /* Mixed precision: A32 = (float) A; Q = A32 P with FP32 element rows and
  * FP64 row totals; z = D^-1 p in FP64 arithmetic, stored in FP32. */
 int fg_ebe_to_f32(femgpu_ebe *c);
-int fg_ebe_matvec32(femgpu_ebe *c, const float *P, double *Q);
-int fg_ebe_blockdiag_apply32(femgpu_ebe *c, const double *p, float *z);
+int fg_ebe_matvec32(femgpu_ebe *c, const float *P, double *Q, const int *active);
+int fg_ebe_blockdiag_apply32(femgpu_ebe *c, const double *p, float *z, const int *active);
 
 #ifdef __cplusplus
 }

@@ -123,8 +123,10 @@ typedef struct fg_status {
 	double rho, eps;
 	double hdiag;      /* scratch                                            */
 	unsigned ticket;   /* last-block reduction ticket                        */
-	int pad;
+	int step;          /* host mirror only, written by the device: inner     */
+	                   /* iterations done | FG_STEP_DONE once inactive       */
 } fg_status;
+#define FG_STEP_DONE 0x40000000
 
 /* Krylov workspace (device memory unless noted); one per context.  A view
  * of a context's buffers is enough to run the cycles below. */
@@ -140,6 +142,8 @@ typedef struct fg_krylov {
 	fg_status *st;                  /* device status                          */
 	fg_status *st_host;             /* pinned host mirror                     */
 	int dsv;                        /* FGMRES: Arnoldi basis in double-single */
+	double *orth;                   /* device-wide sums of the one-launch steps
+	                                 * and scratch (fg_kry_orth_bytes)        */
 	/* FGMRES look-ahead (la_s != NULL): the preconditioner of the next step
 	 * runs on la_s, on the raw operator output la_w, while the Gram-Schmidt
 	 * of this step runs on stream; la_t [ldv] the combination of the stored
@@ -241,6 +245,7 @@ struct femgpu_transport {
 	float *Z32;                     /* ... (FP32, mixed precision)           */
 	double *xr, *dr;                /* refinement: residual and correction   */
 	double *partials;               /* reduction partials                    */
+	double *orth;                   /* fg_krylov.orth                        */
 	int nblk_red;
 	fg_status *st;                  /* device status                         */
 	fg_status *st_host;             /* pinned mirror                         */
@@ -309,6 +314,14 @@ int fg_build_csr_m(int M, int nel, int neq, const int *ri_ptr, const int *ri, co
                    int *err, int **IA, int **JA, int **sbe, int *nnz);
 int fg_assemble_csr_m(int M, int neq, int nnz, const int *IA, const int *sbe, const int *ri_ptr, const int *ri,
                       const double *Ae, double *AA, cudaStream_t s);
+/* arnoldi.cu: the Givens update of column i, the back substitution, and the
+ * orthogonalisation of step i in one launch (passes 0: MGS, else CGS passes) */
+int fg_kry_givens(const fg_krylov *k, int i);
+int fg_kry_backsolve(const fg_krylov *k);
+size_t fg_kry_orth_bytes(int kmax);
+int fg_kry_orth_fits(const fg_krylov *k);
+int fg_kry_orth_begin(const fg_krylov *k);
+int fg_kry_orth(const fg_krylov *k, int i, int passes);
 /* st->rho = ||B - A X|| (A X is formed in V[kmax]). */
 int fg_kry_true_rho(const fg_krylov *k, const fg_linop *op, const double *B, double *X);
 int fg_kry_dot(const fg_krylov *k, const double *a, const double *b, int n, double *out_dev);

@@ -499,12 +499,22 @@ __global__ void __launch_bounds__(RED_TPB) k_mdot(const double *V, size_t ldv, i
 		for (int q = 0; q < MD_J; q++)
 			if (j0 + q < m) acc[q] += V[(size_t)(j0 + q) * ldv + k] * wk;
 	}
+	// eight sums over the warp with nine additions a lane instead of forty (an
+	// FP64 addition holds the warp's pipe for 64 clocks): each of the first
+	// exchanges halves the sums a lane keeps
 	const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+	static_assert(MD_J == 8, "the exchanges below are for eight sums");
 #pragma unroll
-	for (int q = 0; q < MD_J; q++) {
-		double v = fg_warp_sum(acc[q]);
-		if (lane == 0) sh[q][wid] = v;
-	}
+	for (int o = 4; o > 0; o >>= 1)
+#pragma unroll
+		for (int q = 0; q < o; q++) {
+			const bool hi = lane & (4 * o);
+			const double keep = hi ? acc[q + o] : acc[q], give = hi ? acc[q] : acc[q + o];
+			acc[q] = keep + __shfl_xor_sync(0xffffffffu, give, 4 * o);
+		}
+	acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], 2);
+	acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], 1);
+	if ((lane & 3) == 0) sh[((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1)][wid] = acc[0];
 	__syncthreads();
 	if (threadIdx.x < MD_J && j0 + (int)threadIdx.x < m) {
 		double t = 0.0;
@@ -690,7 +700,7 @@ __global__ void k_scale(double *u, int n, const double *h, fg_status *st)
 // force: run at least one inner iteration (the do-while of pgmres.c:89-163).
 __global__ void __launch_bounds__(RED_TPB) k_residual_start(double *u0, const double *B, int n,
                                                             double *ge, double *partials, fg_status *st,
-                                                            int force)
+                                                            int force, int *step)
 {
 	__shared__ double sh[32];
 	double part = 0.0;
@@ -706,47 +716,7 @@ __global__ void __launch_bounds__(RED_TPB) k_residual_start(double *u0, const do
 		st->rho = ge[0];
 		st->inner = 0;
 		st->active = (force || st->rho > st->eps) ? 1 : 0;
-	}
-}
-
-// Givens QR update of column i (pgmres.c:123-163), single thread.
-__global__ void k_givens(double *H, int ldh, double *cs, double *sn, double *ge, int i, int kmax,
-                         fg_status *st)
-{
-	if (!gmres_live(st)) return;
-	for (int j = 0; j <= i - 1; j++) {
-		double hj = H[j * ldh + i], hj1 = H[(j + 1) * ldh + i];
-		double h1 = __dadd_rn(__dmul_rn(cs[j], hj), __dmul_rn(sn[j], hj1));
-		double h2 = __dadd_rn(__dmul_rn(-sn[j], hj), __dmul_rn(cs[j], hj1));
-		H[j * ldh + i] = h1;
-		H[(j + 1) * ldh + i] = h2;
-	}
-	double hii = H[i * ldh + i], hi1 = H[(i + 1) * ldh + i];
-	double r = sqrt(__dadd_rn(__dmul_rn(hii, hii), __dmul_rn(hi1, hi1)));
-	cs[i] = hii / r;
-	sn[i] = hi1 / r;
-	H[i * ldh + i] = r;
-	H[(i + 1) * ldh + i] = 0.0;
-	ge[i + 1] = __dmul_rn(-sn[i], ge[i]);
-	ge[i] = __dmul_rn(cs[i], ge[i]);
-	double rho = fabs(ge[i + 1]);
-	st->rho = rho;
-	st->inner = i + 1;
-	st->total += 1;
-	if (!(rho > st->eps) || i + 1 >= kmax) st->active = 0;
-	if (!(rho == rho)) { st->active = 0; fg_set_err(&st->err, FEMGPU_E_BREAKDOWN); }
-}
-
-// Back substitution (pgmres.c:165-175), single thread; i = inner - 1.
-__global__ void k_backsolve(const double *H, int ldh, const double *ge, double *gy, fg_status *st)
-{
-	int i = st->inner - 1;
-	if (i < 0) return;
-	gy[i] = ge[i] / H[i * ldh + i];
-	for (int j = i - 1; j >= 0; j--) {
-		double soma = 0.0;
-		for (int k = j + 1; k <= i; k++) soma = __dadd_rn(soma, __dmul_rn(H[j * ldh + k], gy[k]));
-		gy[j] = __dadd_rn(ge[j], -soma) / H[j * ldh + j];
+		if (!st->active) *(volatile int *)step = FG_STEP_DONE;
 	}
 }
 
@@ -764,6 +734,24 @@ __global__ void k_update_x(double *X, const TV *V, size_t ldv, int n, const doub
 
 static int red_grid(femgpu_transport *t) { return t->nblk_red; }
 
+// A cycle's steps are enqueued ahead of the device, STEPS_AHEAD at most: far
+// enough that the device never waits for the host, near enough that a cycle
+// that converges early leaves few launches that find nothing to do (up to ten
+// a step, 1.5 to 2 us each).  True when the device has finished the cycle.
+#define STEPS_AHEAD 6
+static bool cycle_done(const fg_krylov *k, int i)
+{
+	const volatile int *step = &k->st_host->step;
+	for (unsigned spin = 1;; spin++) {
+		const int v = *step;
+		if (v & FG_STEP_DONE) return true;
+		if (v + STEPS_AHEAD > i) return false;
+		// an idle stream that has not got there (an error): the caller's
+		// synchronisation tells
+		if ((spin & 4095u) == 0 && cudaStreamQuery(k->stream) != cudaErrorNotReady) return false;
+	}
+}
+
 // One restart cycle of pgmres.c:58-184, entirely stream-ordered; the status
 // block tells the host afterwards whether to restart.
 extern "C" int fg_kry_pgmres_cycle(const fg_krylov *k, const fg_linop *op, const double *B, double *X)
@@ -773,21 +761,29 @@ extern "C" int fg_kry_pgmres_cycle(const fg_krylov *k, const fg_linop *op, const
 	size_t ldv = k->ldv;
 	double *V = k->V;
 	int *active = &k->st->active;
+	const bool one = fg_kry_orth_fits(k);
+	k->st_host->step = 0;
+	if (one && (rc = fg_kry_orth_begin(k))) return rc;
 	// u0 = M^-1 A X  (precondR is the identity in the drivers using pgmres)
 	if ((rc = op->matvec(op->ctx, X, V, nullptr))) return rc;
 	if (op->precond && (rc = op->precond(op->ctx, V, V, nullptr))) return rc;
-	k_residual_start<<<G, RED_TPB, 0, s>>>(V, B, n, k->ge, k->partials, k->st, 1);
+	k_residual_start<<<G, RED_TPB, 0, s>>>(V, B, n, k->ge, k->partials, k->st, 1, &k->st_host->step);
 	k_scale<<<fg_grid(n), FG_TPB, 0, s>>>(V, n, k->ge, k->st);
 	for (int i = 0; i < kmax; i++) {
 		double *w = V + (size_t)(i + 1) * ldv;
+		if (cycle_done(k, i)) break;
 		if ((rc = op->matvec(op->ctx, V + (size_t)i * ldv, w, active))) return rc;
 		if (op->precond && (rc = op->precond(op->ctx, w, w, active))) return rc;
+		if (one) {
+			if ((rc = fg_kry_orth(k, i, 0))) return rc;
+			continue;
+		}
 		for (int j = 0; j <= i + 1; j++)
 			k_mgs<<<G, RED_TPB, 0, s>>>(V, ldv, n, i, j, k->H, ldh, k->partials, k->st);
 		k_scale<<<fg_grid(n), FG_TPB, 0, s>>>(w, n, k->H + (i + 1) * ldh + i, k->st);
-		k_givens<<<1, 1, 0, s>>>(k->H, ldh, k->cs, k->sn, k->ge, i, kmax, k->st);
+		if ((rc = fg_kry_givens(k, i))) return rc;
 	}
-	k_backsolve<<<1, 1, 0, s>>>(k->H, ldh, k->ge, k->gy, k->st);
+	if ((rc = fg_kry_backsolve(k))) return rc;
 	k_update_x<double><<<fg_grid(n), FG_TPB, 0, s>>>(X, V, ldv, n, k->gy, k->st);
 	return (int)cudaGetLastError();
 }
@@ -874,11 +870,13 @@ static int fgmres_cycle_la(const fg_krylov *k, const fg_linop *op, const double 
 	const int gs = gs_mode(cycle);
 	// the product writes the preconditioner's gathered input itself
 	const bool fused = op->matvec_g && op->precond_g && op->precond_g_out;
+	k->st_host->step = 0;
 	if ((rc = op->matvec(op->ctx, X, V, nullptr))) return rc;
-	k_residual_start<<<G, RED_TPB, 0, s>>>(V, B, n, k->ge, k->partials, k->st, 0);
+	k_residual_start<<<G, RED_TPB, 0, s>>>(V, B, n, k->ge, k->partials, k->st, 0, &k->st_host->step);
 	k_scale<<<fg_grid(n), FG_TPB, 0, s>>>(V, n, k->ge, k->st);
 	if ((rc = op->precond(op->ctx, V, Z, active))) return rc;
 	for (int i = 0; i < kmax; i++) {
+		if (cycle_done(k, i)) break;
 		const int m = i + 1, more = i + 1 < kmax;
 		const size_t hs = sizeof(double) * (size_t)m > LA_SMEM ? sizeof(double) * (size_t)m : LA_SMEM;
 		double *w = V + (size_t)(i + 1) * ldv, *znext = Z + (size_t)(i + 1) * ldv;
@@ -905,7 +903,7 @@ static int fgmres_cycle_la(const fg_krylov *k, const fg_linop *op, const double 
 		}
 		if (more) k_zcombo<<<cgs_grid, RED_TPB, hs, s>>>(Z, ldv, n, m, k->H + i, ldh, k->la_t, k->la_eta, k->st);
 		k_scale<<<fg_grid(n), FG_TPB, 0, s>>>(w, n, k->H + (i + 1) * ldh + i, k->st);
-		k_givens<<<1, 1, 0, s>>>(k->H, ldh, k->cs, k->sn, k->ge, i, kmax, k->st);
+		if ((rc = fg_kry_givens(k, i))) return rc;
 		if (more) {
 			FG_TRY(cudaStreamWaitEvent(s, k->la_ev_y, 0));
 			if (fused)
@@ -914,7 +912,7 @@ static int fgmres_cycle_la(const fg_krylov *k, const fg_linop *op, const double 
 			else k_la_fin<<<fg_grid(n), FG_TPB, 0, s>>>(znext, k->la_t, n, k->la_eta, k->st);
 		}
 	}
-	k_backsolve<<<1, 1, 0, s>>>(k->H, ldh, k->ge, k->gy, k->st);
+	if ((rc = fg_kry_backsolve(k))) return rc;
 	k_update_x<double><<<fg_grid(n), FG_TPB, 0, s>>>(X, Z, ldv, n, k->gy, k->st);
 	return (int)cudaGetLastError();
 }
@@ -941,12 +939,16 @@ extern "C" int fg_kry_fgmres_cycle(const fg_krylov *k, const fg_linop *op, const
 	const int cgs_grid = G * (CGS_GRID < kmax + 1 ? CGS_GRID : kmax + 1);
 	if (mixed && (!op->precond32 || !op->matvec_xf || !k->Z32)) return FEMGPU_E_ARG;
 	if (!mixed && !k->Z) return FEMGPU_E_ARG;
+	const bool one = !dsv && fg_kry_orth_fits(k);
+	k->st_host->step = 0;
+	if (one && (rc = fg_kry_orth_begin(k))) return rc;
 	if ((rc = op->matvec(op->ctx, X, V, nullptr))) return rc;
-	k_residual_start<<<G, RED_TPB, 0, s>>>(V, B, n, k->ge, k->partials, k->st, 0);
+	k_residual_start<<<G, RED_TPB, 0, s>>>(V, B, n, k->ge, k->partials, k->st, 0, &k->st_host->step);
 	if (dsv) k_scale_ds<<<fg_grid(n), FG_TPB, 0, s>>>((dsf *)V, n, k->ge, 1, k->st);
 	else k_scale<<<fg_grid(n), FG_TPB, 0, s>>>(V, n, k->ge, k->st);
 	for (int i = 0; i < kmax; i++) {
 		double *v = V + (size_t)i * ldv, *w = V + (size_t)(i + 1) * ldv;
+		if (cycle_done(k, i)) break;
 		if (mixed) {
 			float *z = k->Z32 + (size_t)i * ldv;
 			if ((rc = op->precond32(op->ctx, v, z, active))) return rc;
@@ -965,6 +967,10 @@ extern "C" int fg_kry_fgmres_cycle(const fg_krylov *k, const fg_linop *op, const
 			if ((rc = op->matvec(op->ctx, z, w, active))) return rc;
 		}
 		int gs = gs_mode(cycle);
+		if (one) {
+			if ((rc = fg_kry_orth(k, i, gs))) return rc;
+			continue;
+		}
 		if (dsv && gs == 0) gs = 1;                        // MGS has no double-single form
 		if (dsv) {
 			const int m = i + 1;
@@ -979,7 +985,7 @@ extern "C" int fg_kry_fgmres_cycle(const fg_krylov *k, const fg_linop *op, const
 				                                                         k->st);
 			}
 			k_scale_ds<<<fg_grid(n), FG_TPB, 0, s>>>((dsf *)w, n, k->H + (i + 1) * ldh + i, 0, k->st);
-			k_givens<<<1, 1, 0, s>>>(k->H, ldh, k->cs, k->sn, k->ge, i, kmax, k->st);
+			if ((rc = fg_kry_givens(k, i))) return rc;
 			continue;
 		}
 		if (gs == 0) {
@@ -998,9 +1004,9 @@ extern "C" int fg_kry_fgmres_cycle(const fg_krylov *k, const fg_linop *op, const
 			}
 		}
 		k_scale<<<fg_grid(n), FG_TPB, 0, s>>>(w, n, k->H + (i + 1) * ldh + i, k->st);
-		k_givens<<<1, 1, 0, s>>>(k->H, ldh, k->cs, k->sn, k->ge, i, kmax, k->st);
+		if ((rc = fg_kry_givens(k, i))) return rc;
 	}
-	k_backsolve<<<1, 1, 0, s>>>(k->H, ldh, k->ge, k->gy, k->st);
+	if ((rc = fg_kry_backsolve(k))) return rc;
 	if (mixed) k_update_x<float><<<fg_grid(n), FG_TPB, 0, s>>>(X, k->Z32, ldv, n, k->gy, k->st);
 	else k_update_x<double><<<fg_grid(n), FG_TPB, 0, s>>>(X, k->Z, ldv, n, k->gy, k->st);
 	return (int)cudaGetLastError();
@@ -1163,7 +1169,7 @@ extern "C" void fg_transport_krylov(femgpu_transport *t, fg_krylov *k, fg_linop 
 {
 	k->n = t->neq; k->kmax = t->kmax; k->nblk = red_grid(t); k->ldv = t->ldv; k->stream = t->stream;
 	k->V = t->V; k->H = t->H; k->cs = t->cs; k->sn = t->sn; k->ge = t->ge; k->gy = t->gy;
-	k->Z = t->Z; k->Z32 = t->Z32; k->partials = t->partials; k->st = t->st; k->st_host = t->st_host;
+	k->Z = t->Z; k->Z32 = t->Z32; k->partials = t->partials; k->orth = t->orth; k->st = t->st; k->st_host = t->st_host;
 	op->ctx = t;
 	op->matvec = tr_matvec;
 	op->precond = tr_precond;

@@ -87,7 +87,7 @@ double *femgpu_ebe_A_dev(femgpu_ebe *c) { return c ? c->A : NULL; }
 int femgpu_ebe_matvec_dev(femgpu_ebe *c, const double *P, double *Q)
 {
 	if (!c || !P || !Q) return FEMGPU_E_ARG;
-	KR(fg_ebe_matvec(c, P, Q, 0));
+	KR(fg_ebe_matvec(c, P, Q, 0, NULL));
 	return 0;
 }
 
@@ -95,7 +95,7 @@ int femgpu_ebe_matvec32_dev(femgpu_ebe *c, const float *P, double *Q)
 {
 	if (!c || !P || !Q) return FEMGPU_E_ARG;
 	if (!c->A32) { fgh_set_error("no FP32 element matrices"); return FEMGPU_E_NOT_BUILT; }
-	KR(fg_ebe_matvec32(c, P, Q));
+	KR(fg_ebe_matvec32(c, P, Q, NULL));
 	return 0;
 }
 
@@ -105,7 +105,7 @@ int femgpu_ebe_matvec(femgpu_ebe *c, const double *P_host, double *Q_host)
 	if (!c || !P_host || !Q_host) return FEMGPU_E_ARG;
 	n1 = (size_t)c->neq + 1;
 	CK(cudaMemcpyAsync(c->P, P_host, sizeof(double) * n1, cudaMemcpyHostToDevice, c->stream));
-	KR(fg_ebe_matvec(c, c->P, c->Q, 0));
+	KR(fg_ebe_matvec(c, c->P, c->Q, 0, NULL));
 	CK(cudaMemcpyAsync(Q_host, c->Q, sizeof(double) * n1, cudaMemcpyDeviceToHost, c->stream));
 	CK(cudaStreamSynchronize(c->stream));
 	return 0;
@@ -115,8 +115,8 @@ int femgpu_ebe_matvec2_dev(femgpu_ebe *c, const double *P, double *Q, int with_i
 {
 	if (!c || !P || !Q || c->ndof != 4) return FEMGPU_E_ARG;
 	if (!c->have_bd) { fgh_set_error("matvec2 before blockdiag_setup"); return FEMGPU_E_NOT_BUILT; }
-	KR(fg_ebe_matvec(c, P, Q, 1));
-	KR(fg_ebe_blockdiag_apply(c, P, Q, with_inverse ? 1 : 2));
+	KR(fg_ebe_matvec(c, P, Q, 1, NULL));
+	KR(fg_ebe_blockdiag_apply(c, P, Q, with_inverse ? 1 : 2, NULL));
 	return 0;
 }
 
@@ -144,7 +144,7 @@ int femgpu_ebe_blockdiag_setup(femgpu_ebe *c, double *F_host, double *BD_host, d
 	c->have_bd = 1;
 	if (F_host) {
 		CK(cudaMemcpyAsync(c->P, F_host, sizeof(double) * n1, cudaMemcpyHostToDevice, c->stream));
-		KR(fg_ebe_blockdiag_apply(c, c->P, c->P, 0));
+		KR(fg_ebe_blockdiag_apply(c, c->P, c->P, 0, NULL));
 		CK(cudaMemcpyAsync(F_host, c->P, sizeof(double) * n1, cudaMemcpyDeviceToHost, c->stream));
 	}
 	if (BD_host) CK(cudaMemcpyAsync(BD_host, c->BD, sizeof(double) * nb, cudaMemcpyDeviceToHost, c->stream));
@@ -157,7 +157,7 @@ int femgpu_ebe_blockdiag_apply_dev(femgpu_ebe *c, const double *p, double *z)
 {
 	if (!c || !p || !z) return FEMGPU_E_ARG;
 	if (!c->have_bd) { fgh_set_error("blockdiag apply before setup"); return FEMGPU_E_NOT_BUILT; }
-	KR(fg_ebe_blockdiag_apply(c, p, z, 0));
+	KR(fg_ebe_blockdiag_apply(c, p, z, 0, NULL));
 	return 0;
 }
 

@@ -42,30 +42,26 @@ void femgpu_euler_default_opts(femgpu_euler_opts *o)
 /* ---- operator callbacks of the Krylov solver ---------------------------- */
 static int op_matvec(void *ctx, const double *p, double *q, const int *active)
 {
-	(void)active;
-	return fg_ebe_matvec(((femgpu_euler *)ctx)->ebe, p, q, 0);
+	return fg_ebe_matvec(((femgpu_euler *)ctx)->ebe, p, q, 0, active);
 }
 
 static int op_precond(void *ctx, const double *p, double *z, const int *active)
 {
-	(void)active;
-	return fg_ebe_blockdiag_apply(((femgpu_euler *)ctx)->ebe, p, z, 0);
+	return fg_ebe_blockdiag_apply(((femgpu_euler *)ctx)->ebe, p, z, 0, active);
 }
 
 /* mixed precision: z = D^-1 p in FP32, q = A32 z */
 static int op_precond32(void *ctx, const double *p, float *z, const int *active)
 {
 	femgpu_euler *c = (femgpu_euler *)ctx;
-	(void)active;
-	if (c->o.precond == FEMGPU_PREC_BLOCKDIAG) return fg_ebe_blockdiag_apply32(c->ebe, p, z);
+	if (c->o.precond == FEMGPU_PREC_BLOCKDIAG) return fg_ebe_blockdiag_apply32(c->ebe, p, z, active);
 	return fg_to_f32(p, z, (long long)c->neq + 1, c->stream);
 }
 
 static int op_matvec_xf(void *ctx, const float *p, double *q, const int *active, int op32)
 {
-	(void)active;
 	if (!op32) return FEMGPU_E_ARG;                   /* only the FP32 operator is provided */
-	return fg_ebe_matvec32(((femgpu_euler *)ctx)->ebe, p, q);
+	return fg_ebe_matvec32(((femgpu_euler *)ctx)->ebe, p, q, active);
 }
 
 /* CSR storage: csrmv and ILUp_precond */
@@ -325,7 +321,7 @@ int femgpu_euler_scale_dev(femgpu_euler *c)
 	if (!c->built) { fgh_set_error("scaling before build"); return FEMGPU_E_NOT_BUILT; }
 	if (c->o.scheme != FEMGPU_EBE) { fgh_set_error("BlockScaling needs EBE storage (setScaling.c)"); return FEMGPU_E_ARG; }
 	KR(fg_ebe_blockdiag_setup(c->ebe));
-	KR(fg_ebe_blockdiag_apply(c->ebe, c->R, c->R, 0));
+	KR(fg_ebe_blockdiag_apply(c->ebe, c->R, c->R, 0, NULL));
 	KR(fg_ebe_block_scale(c->ebe));
 	c->ebe->have_bd = 0;
 	c->have_bd = 0;
@@ -368,7 +364,7 @@ int femgpu_euler_precond_setup_dev(femgpu_euler *c)
 	KR(fg_ebe_blockdiag_setup(c->ebe));
 	c->ebe->have_bd = 1;
 	c->have_bd = 1;
-	if (c->o.solver == FEMGPU_PGMRES) KR(fg_ebe_blockdiag_apply(c->ebe, c->R, c->R, 0));
+	if (c->o.solver == FEMGPU_PGMRES) KR(fg_ebe_blockdiag_apply(c->ebe, c->R, c->R, 0, NULL));
 	return 0;
 }
 

@@ -35,6 +35,7 @@ int fgh_kry_alloc(fg_krylov *k, int n, int kmax, int zmode, void *stream)
 	if (zmode == 1) DM(k->Z, sizeof(double) * k->ldv * (size_t)kmax);
 	if (zmode == 2) DM(k->Z32, sizeof(float) * k->ldv * (size_t)kmax);
 	DM(k->partials, sizeof(double) * ((size_t)k->nblk * (m1 + 1) + m1 + 1));
+	DM(k->orth, fg_kry_orth_bytes(kmax));
 	DM(k->st, sizeof(fg_status));
 	CK(cudaMemsetAsync(k->V, 0, sizeof(double) * k->ldv * m1, k->stream));
 	CK(cudaMemsetAsync(k->st, 0, sizeof(fg_status), k->stream));
@@ -45,7 +46,7 @@ int fgh_kry_alloc(fg_krylov *k, int n, int kmax, int zmode, void *stream)
 
 void fgh_kry_free(fg_krylov *k)
 {
-	void *p[] = { k->V, k->H, k->cs, k->sn, k->ge, k->gy, k->Z, k->Z32, k->partials, k->st };
+	void *p[] = { k->V, k->H, k->cs, k->sn, k->ge, k->gy, k->Z, k->Z32, k->partials, k->orth, k->st };
 	int i;
 	for (i = 0; i < (int)(sizeof p / sizeof p[0]); i++) if (p[i]) cudaFree(p[i]);
 	if (k->st_host) cudaFreeHost(k->st_host);

@@ -36,14 +36,12 @@ void femgpu_ns_default_opts(femgpu_ns_opts *o)
 
 static int op_matvec(void *ctx, const double *p, double *q, const int *active)
 {
-	(void)active;
-	return fg_ebe_matvec(((femgpu_ns *)ctx)->ebe, p, q, 0);
+	return fg_ebe_matvec(((femgpu_ns *)ctx)->ebe, p, q, 0, active);
 }
 
 static int op_precond(void *ctx, const double *p, double *z, const int *active)
 {
-	(void)active;
-	return fg_ebe_blockdiag_apply(((femgpu_ns *)ctx)->ebe, p, z, 0);
+	return fg_ebe_blockdiag_apply(((femgpu_ns *)ctx)->ebe, p, z, 0, active);
 }
 
 /* CSR storage: csrmv and ILUp_precond */
@@ -234,7 +232,7 @@ static int setup_dev(femgpu_ns *c)
 	KR(fg_ebe_blockdiag_setup(c->ebe));
 	c->ebe->have_bd = 1;
 	c->have_bd = 1;
-	if (c->o.solver == FEMGPU_PGMRES) KR(fg_ebe_blockdiag_apply(c->ebe, c->F, c->F, 0));
+	if (c->o.solver == FEMGPU_PGMRES) KR(fg_ebe_blockdiag_apply(c->ebe, c->F, c->F, 0, NULL));
 	return 0;
 }
 

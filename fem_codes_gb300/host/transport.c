@@ -330,6 +330,7 @@ int femgpu_transport_create(femgpu_transport **out, const femgpu_transport_opts 
 	/* reduction partials: one row per basis vector for the CGS multi-dot,
 	 * then the projection coefficients */
 	DM(t->partials, sizeof(double) * ((size_t)t->nblk_red * ((size_t)t->kmax + 2) + (size_t)t->kmax + 2));
+	DM(t->orth, fg_kry_orth_bytes(t->kmax));
 	for (i = 0; i < 4; i++) CK(cudaEventCreate(&t->ev[i]));
 	CK(cudaDeviceSynchronize());
 	rc = sync_err(t);
@@ -350,7 +351,7 @@ void femgpu_transport_destroy(femgpu_transport *t)
 		t->lm, t->ri_ptr, t->ri, t->IA, t->JA, t->sbe, t->diag, t->lm2, t->order, t->ec_ptr,
 		t->ec, t->e2_ptr, t->e2, t->A, t->ke, t->fe, t->A32, t->u, t->F, t->F0, t->invDiag,
 		t->invDiag32, t->ilu.LU, t->ilu.Dinv, t->V, t->H, t->cs, t->sn, t->ge, t->gy, t->w2,
-		t->Z, t->Z32, t->xr, t->dr, t->partials, t->st, t->du, t->uold, t->Da, t->re, t->dold,
+		t->Z, t->Z32, t->xr, t->dr, t->partials, t->orth, t->st, t->du, t->uold, t->Da, t->re, t->dold,
 		t->u1, t->u2, t->uB, t->aB, t->bub, t->uB1, t->uB2, t->la_buf, t->la_flag, t->sell_base, t->sell_w, t->sell_src, t->sell_JA, t->sell_A };
 	for (i = 0; i < (int)(sizeof ptrs / sizeof ptrs[0]); i++) if (ptrs[i]) cudaFree(ptrs[i]);
 	if (t->la_s) {
