@@ -13,13 +13,15 @@
 // This translation unit is compiled with --fmad=false: every product and sum
 // is rounded separately, as in the reference compiled without contraction.
 #include "fg_common.cuh"
+#include "fg_div.cuh"
 
 struct BuildArgs {
 	const double *x, *y, *u, *upresc, *beta, *fsrc;
 	const int *vert, *node_id;
 	double k, gamma, cbx, cby;
 	int nel, shock, hshock, beta_const, fsrc_zero;
-	double *ke, *fe;
+	double bnorm, rbnorm;         // constant velocity: its norm and the inverse
+	double *ke, *fe;              // fe: NULL without a source (steady build)
 	// transient builds only
 	const double *du;             // the time derivative a (neq+1)
 	double adt;                   // Alpha * DeltaT
@@ -56,6 +58,7 @@ __device__ __forceinline__ double h_shock(int opt, double bx, double by, double 
 // CAU_ShockCapture.c:3-30 (the division by |grad u|^2 is only evaluated when
 // |grad u| > 0; the reference computes it first and discards a NaN) and
 // YZBeta_ShockCapture.c:3-27.
+template <bool SRC, bool REACT>
 __device__ __forceinline__ double shock_capture(int kind, double kx, double ky, double bx, double by,
                                                 double g, double ue1, double ue2, double ue3,
                                                 double ueb, double feb, double y23, double y31,
@@ -63,7 +66,9 @@ __device__ __forceinline__ double shock_capture(int kind, double kx, double ky, 
                                                 double invArea, double h)
 {
 	double BetaGradu = 0.5*invArea*(ue1*(bx*y23 + by*x32) + ue2*(bx*y31 + by*x13) + ue3*(bx*y12 + by*x21));
-	double Ru = BetaGradu + g*ueb - feb;
+	double Ru = BetaGradu;
+	if (REACT) Ru = Ru + g*ueb;
+	if (SRC) Ru = Ru - feb;
 	double G0 = 0.5*invArea*(y23*ue1 + y31*ue2 + y12*ue3);
 	double G1 = 0.5*invArea*(x32*ue1 + x13*ue2 + x21*ue3);
 	double nG = sqrt(G0*G0 + G1*G1);
@@ -77,15 +82,29 @@ __device__ __forceinline__ double shock_capture(int kind, double kx, double ky, 
 	double kp = bxp*bxp*kx + byp*byp*ky;
 	double nbp = sqrt(bxp*bxp + byp*byp);
 	double Pee = 0.5*h*nbp*nbp*nbp/kp;
-	if (third*Pee < 0.7) return 0.5*h*third*Pee*fabs(Ru)/nG;
-	return 0.5*h*0.7*fabs(Ru)/nG;
+	// one quotient for both branches: a warp that takes both pays for one
+	double num = third*Pee < 0.7 ? 0.5*h*third*Pee*fabs(Ru) : 0.5*h*0.7*fabs(Ru);
+	return num/nG;
 }
 
+// SRC: a source term; REACT: gamma != 0 (their terms are exact zeros otherwise
+// and are left out, as is Fe without a source).
+//
+// Bound by the FP64 pipes: 64 clocks a warp's instruction on this part, about
+// 360 instructions an element with the terms that vanish, 270 without them, the
+// constant velocity's norm formed once, h_shock = h for 2sqrtArea (2 Area is
+// TwoA exactly) and one quotient where shock_capture had one a branch.  The
+// element matrices leave through shared memory in whole lines (nine 8-byte
+// stores 72 bytes apart touch every sector four times).  At 2.16M elements, constant velocity, no
+// source or reaction: 1270 us before, 919 with both.
+template <bool SRC, bool REACT>
 __global__ void __launch_bounds__(128) k_build_supg(BuildArgs a)
 {
+	__shared__ __align__(16) double ske[128 * 9];
 	const double third = 1.0/3.0, sixth = 1.0/6.0, twelfth = 1.0/12.0;
 	const double kx = a.k, ky = a.k, gamma = a.gamma;
-	for (int E = blockIdx.x * blockDim.x + threadIdx.x; E < a.nel; E += gridDim.x * blockDim.x) {
+	for (int E0 = blockIdx.x * blockDim.x; E0 < a.nel; E0 += gridDim.x * blockDim.x) {
+		const int E = E0 + threadIdx.x < a.nel ? E0 + threadIdx.x : a.nel - 1;   // past the end: the last one again
 		int J1 = __ldg(&a.vert[3*E]), J2 = __ldg(&a.vert[3*E+1]), J3 = __ldg(&a.vert[3*E+2]);
 		double X0 = __ldg(&a.x[J1]), X1 = __ldg(&a.x[J2]), X2 = __ldg(&a.x[J3]);
 		double Y0 = __ldg(&a.y[J1]), Y1 = __ldg(&a.y[J2]), Y2 = __ldg(&a.y[J3]);
@@ -93,13 +112,18 @@ __global__ void __launch_bounds__(128) k_build_supg(BuildArgs a)
 		double x32 = X2 - X1, x13 = X0 - X2, x21 = X1 - X0;
 		double TwoA = x21*y31 - x13*y12, Area = 0.5*TwoA, invArea = 1.0/Area;
 		double h = sqrt(fabs(TwoA));
-		double bx, by;
-		if (a.beta_const) { bx = a.cbx; by = a.cby; }
-		else { bx = __ldg(&a.beta[2*E]); by = __ldg(&a.beta[2*E+1]); }
-		double norm = sqrt(bx*bx + by*by), tau = (norm > 0) ? 0.5*h/norm : 0.0;
+		double bx, by, tau = 0.0;
+		if (a.beta_const) {
+			bx = a.cbx; by = a.cby;
+			if (a.bnorm > 0) tau = fg_div(0.5*h, a.bnorm, a.rbnorm);
+		} else {
+			bx = __ldg(&a.beta[2*E]); by = __ldg(&a.beta[2*E+1]);
+			double norm = sqrt(bx*bx + by*by);
+			if (norm > 0) tau = 0.5*h/norm;
+		}
 		double fe1 = 0.0, fe2 = 0.0, fe3 = 0.0;
-		if (!a.fsrc_zero) { fe1 = __ldg(&a.fsrc[3*E]); fe2 = __ldg(&a.fsrc[3*E+1]); fe3 = __ldg(&a.fsrc[3*E+2]); }
-		double feb = third*(fe1+fe2+fe3);
+		if (SRC) { fe1 = __ldg(&a.fsrc[3*E]); fe2 = __ldg(&a.fsrc[3*E+1]); fe3 = __ldg(&a.fsrc[3*E+2]); }
+		double feb = SRC ? third*(fe1+fe2+fe3) : 0.0;
 		// eval_U.c:12-22
 		int i1 = __ldg(&a.node_id[J1]), i2 = __ldg(&a.node_id[J2]), i3 = __ldg(&a.node_id[J3]);
 		double ue1 = (i1 >= 0) ? a.u[i1] : __ldg(&a.upresc[J1]);
@@ -113,37 +137,57 @@ __global__ void __launch_bounds__(128) k_build_supg(BuildArgs a)
 		double C11 = sixth*(bx*y23 + by*x32);
 		double C12 = sixth*(bx*y31 + by*x13);
 		double C13 = sixth*(bx*y12 + by*x21);
-		double R11 = sixth*(gamma*Area);
-		double R12 = twelfth*(gamma * Area);
+		double R11 = REACT ? sixth*(gamma*Area) : 0.0;
+		double R12 = REACT ? twelfth*(gamma * Area) : 0.0;
 		double Cpg12 = 0.25*invArea*tau * (y23*(bx*bx*y31 + bx*by*x13) + x32*(bx*by*y31 + by*by*x13));
 		double Cpg13 = 0.25*invArea*tau * (y23*(bx*bx*y12 + bx*by*x21) + x32*(bx*by*y12 + by*by*x21));
 		double Cpg23 = 0.25*invArea*tau * (y31*(bx*bx*y12 + bx*by*x21) + x13*(bx*by*y12 + by*by*x21));
-		double Rpg11 = sixth*tau*gamma * (bx*y23 + by*x32);
-		double Rpg21 = sixth*tau*gamma * (bx*y31 + by*x13);
-		double Rpg31 = sixth*tau*gamma * (bx*y12 + by*x21);
+		double Rpg11 = REACT ? sixth*tau*gamma * (bx*y23 + by*x32) : 0.0;
+		double Rpg21 = REACT ? sixth*tau*gamma * (bx*y31 + by*x13) : 0.0;
+		double Rpg31 = REACT ? sixth*tau*gamma * (bx*y12 + by*x21) : 0.0;
 
-		double hs = h_shock(a.hshock, bx, by, ue1, ue2, ue3, y23, y31, y12, x32, x13, x21, Area);
-		double Eu = shock_capture(a.shock, kx, ky, bx, by, gamma, ue1, ue2, ue3, ueb, feb,
+		double hs = a.hshock == FEMGPU_H_2SQRTAREA ? h : h_shock(a.hshock, bx, by, ue1, ue2, ue3, y23, y31, y12, x32, x13, x21, Area);
+		double Eu = shock_capture<SRC, REACT>(a.shock, kx, ky, bx, by, gamma, ue1, ue2, ue3, ueb, feb,
 		                          y23, y31, y12, x32, x13, x21, invArea, hs);
 		double Csc12 = Eu*0.25*invArea*(y23*y31 + x32*x13);
 		double Csc13 = Eu*0.25*invArea*(y23*y12 + x32*x21);
 		double Csc23 = Eu*0.25*invArea*(y31*y12 + x13*x21);
 
-		double *ke = a.ke + 9LL*E;
-		ke[0] = -(D12 + D13) + C11 - (Cpg12 + Cpg13) + R11 + Rpg11 - (Csc12 + Csc13);
-		ke[1] = D12 + C12 + Cpg12 + R12 + Rpg11 + Csc12;
-		ke[2] = D13 + C13 + Cpg13 + R12 + Rpg11 + Csc13;
-		ke[3] = D12 + C11 + Cpg12 + R12 + Rpg21 + Csc12;
-		ke[4] = -(D12 + D23) + C12 - (Cpg12 + Cpg23) + R11 + Rpg21 - (Csc12 + Csc23);
-		ke[5] = D23 + C13 + Cpg23 + R12 + Rpg21 + Csc23;
-		ke[6] = D13 + C11 + Cpg13 + R12 + Rpg31 + Csc13;
-		ke[7] = D23 + C12 + Cpg23 + R12 + Rpg31 + Csc23;
-		ke[8] = -(D13 + D23) + C13 - (Cpg13 + Cpg23) + R11 + Rpg31 - (Csc13 + Csc23);
-
-		double *fe = a.fe + 3LL*E;
-		fe[0] = Area*twelfth*(2*fe1 +  fe2  +  fe3 ) + sixth*tau*(fe1+fe2+fe3)*(bx*y23 + by*x32);
-		fe[1] = Area*twelfth*(  fe1 + 2*fe2 +  fe3 ) + sixth*tau*(fe1+fe2+fe3)*(bx*y31 + by*x13);
-		fe[2] = Area*twelfth*(  fe1 +  fe2  + 2*fe3) + sixth*tau*(fe1+fe2+fe3)*(bx*y12 + by*x21);
+		double *ke = ske + 9*threadIdx.x;
+		if (REACT) {
+			ke[0] = -(D12 + D13) + C11 - (Cpg12 + Cpg13) + R11 + Rpg11 - (Csc12 + Csc13);
+			ke[1] = D12 + C12 + Cpg12 + R12 + Rpg11 + Csc12;
+			ke[2] = D13 + C13 + Cpg13 + R12 + Rpg11 + Csc13;
+			ke[3] = D12 + C11 + Cpg12 + R12 + Rpg21 + Csc12;
+			ke[4] = -(D12 + D23) + C12 - (Cpg12 + Cpg23) + R11 + Rpg21 - (Csc12 + Csc23);
+			ke[5] = D23 + C13 + Cpg23 + R12 + Rpg21 + Csc23;
+			ke[6] = D13 + C11 + Cpg13 + R12 + Rpg31 + Csc13;
+			ke[7] = D23 + C12 + Cpg23 + R12 + Rpg31 + Csc23;
+			ke[8] = -(D13 + D23) + C13 - (Cpg13 + Cpg23) + R11 + Rpg31 - (Csc13 + Csc23);
+		} else {
+			ke[0] = -(D12 + D13) + C11 - (Cpg12 + Cpg13) - (Csc12 + Csc13);
+			ke[1] = D12 + C12 + Cpg12 + Csc12;
+			ke[2] = D13 + C13 + Cpg13 + Csc13;
+			ke[3] = D12 + C11 + Cpg12 + Csc12;
+			ke[4] = -(D12 + D23) + C12 - (Cpg12 + Cpg23) - (Csc12 + Csc23);
+			ke[5] = D23 + C13 + Cpg23 + Csc23;
+			ke[6] = D13 + C11 + Cpg13 + Csc13;
+			ke[7] = D23 + C12 + Cpg23 + Csc23;
+			ke[8] = -(D13 + D23) + C13 - (Cpg13 + Cpg23) - (Csc13 + Csc23);
+		}
+		if (SRC) {
+			double *fe = a.fe + 3LL*E;
+			fe[0] = Area*twelfth*(2*fe1 +  fe2  +  fe3 ) + sixth*tau*(fe1+fe2+fe3)*(bx*y23 + by*x32);
+			fe[1] = Area*twelfth*(  fe1 + 2*fe2 +  fe3 ) + sixth*tau*(fe1+fe2+fe3)*(bx*y31 + by*x13);
+			fe[2] = Area*twelfth*(  fe1 +  fe2  + 2*fe3) + sixth*tau*(fe1+fe2+fe3)*(bx*y12 + by*x21);
+		}
+		__syncthreads();
+		const int cnt = 9*min((int)blockDim.x, a.nel - E0);
+		double *out = a.ke + 9LL*E0;                          // E0 even: 16-byte aligned
+		for (int q = 2*threadIdx.x; q + 1 < cnt; q += 2*blockDim.x)
+			*reinterpret_cast<double2 *>(&out[q]) = *reinterpret_cast<const double2 *>(&ske[q]);
+		if ((cnt & 1) && threadIdx.x == 0) out[cnt - 1] = ske[cnt - 1];
+		__syncthreads();
 	}
 }
 
@@ -155,9 +199,16 @@ extern "C" int fg_build_elements(femgpu_transport *t)
 	a.k = t->k; a.gamma = t->gamma; a.cbx = t->cbx; a.cby = t->cby;
 	a.nel = t->nel; a.shock = t->o.shock; a.hshock = t->o.hshock;
 	a.beta_const = t->beta_const; a.fsrc_zero = t->fsrc_zero;
+	a.bnorm = sqrt(a.cbx*a.cbx + a.cby*a.cby);
+	a.rbnorm = 1.0/a.bnorm;
 	a.ke = (t->o.scheme == FEMGPU_EBE) ? t->A : t->ke;
 	a.fe = t->fe;
-	k_build_supg<<<fg_grid(t->nel, 128, 32), 128, 0, t->stream>>>(a);
+	const int g = fg_grid(t->nel, 128, 32);
+	const bool src = !t->fsrc_zero, react = t->gamma != 0.0;
+	if (src && react) k_build_supg<true, true><<<g, 128, 0, t->stream>>>(a);
+	else if (src) k_build_supg<true, false><<<g, 128, 0, t->stream>>>(a);
+	else if (react) k_build_supg<false, true><<<g, 128, 0, t->stream>>>(a);
+	else k_build_supg<false, false><<<g, 128, 0, t->stream>>>(a);
 	return (int)cudaGetLastError();
 }
 
@@ -633,45 +684,79 @@ extern "C" int fg_tr_correct(femgpu_transport *t, double c)
 #define FG_ROWCAP 32
 
 // F_assembly.c:5-27 for row I: for each incident element (ascending), add Fe
-// then subtract the Dirichlet lift of every other vertex with Type == 0.
-__device__ __forceinline__ double gather_F(int I, const int *ri_ptr, const int *ri, const double *ke,
-                                           const double *fe, const int *vert, const int *node_type,
+// (fe NULL: no source) then subtract the Dirichlet lift of every other vertex
+// with Type == 0; those are among the vertices without an equation (lm == neq).
+__device__ __forceinline__ double lift(double F, int e, int aa, int b, const double *ke, const int *vert,
+                                       const int *node_type, const double *upresc)
+{
+	int v = __ldg(&vert[3 * e + b]);
+	if (__ldg(&node_type[v]) == 0) F -= __ldg(&ke[9LL * e + 3 * aa + b]) * __ldg(&upresc[v]);
+	return F;
+}
+
+__device__ __forceinline__ double gather_F(int I, int neq, const int *ri_ptr, const int *ri, const int *lm,
+                                           const double *ke, const double *fe, const int *vert, const int *node_type,
                                            const double *upresc)
 {
 	double F = 0.0;
 	for (int q = ri_ptr[I]; q < ri_ptr[I + 1]; q++) {
 		int code = __ldg(&ri[q]), e = code / 3, aa = code - 3 * e;
-		F += __ldg(&fe[3LL * e + aa]);
-		for (int b = 0; b < 3; b++) {
-			if (b == aa) continue;
-			int v = __ldg(&vert[3 * e + b]);
-			if (__ldg(&node_type[v]) == 0) F -= __ldg(&ke[9LL * e + 3 * aa + b]) * __ldg(&upresc[v]);
-		}
+		if (fe) F += __ldg(&fe[3LL * e + aa]);
+		for (int b = 0; b < 3; b++)
+			if (b != aa && __ldg(&lm[3 * e + b]) == neq) F = lift(F, e, aa, b, ke, vert, node_type, upresc);
 	}
 	return F;
 }
 
-// CSR rows: csr_assembly.c:9-22 gathered per row, plus F.
-__global__ void k_assemble_csr(int neq, int nnz, const int *IA, const int *sbe, const int *ri_ptr,
-                               const int *ri, const double *ke, const double *fe, const int *vert,
-                               const int *node_type, const double *upresc, double *AA, double *F,
-                               int *err)
+// CSR rows: csr_assembly.c:9-22 gathered per row, plus F (when given) and the
+// SELL-32 copy of the values (when given: row I's entry j at base[I / 32] + 32 j
+// + I % 32, padded with zeros to the slice's width), which a warp stores in whole
+// lines.  A row's sums are kept in shared memory, a column of 128 threads per
+// entry; a vertex without an equation is known from its slot (the dump).
+// Bound by the element matrices' gather.  At 1.08M rows:
+// 163 us and 21 for a kernel of its own that copied the values into the slices,
+// 137 now; with room for 32 entries a row whatever the rows' length 177
+// (seven blocks to an SM).
+__global__ void __launch_bounds__(128)
+k_assemble_csr(int neq, int nnz, const int *__restrict__ IA, const int *__restrict__ sbe, const int *__restrict__ ri_ptr,
+               const int *__restrict__ ri, const double *__restrict__ ke, const double *__restrict__ fe,
+               const int *__restrict__ vert, const int *__restrict__ node_type, const double *__restrict__ upresc,
+               double *AA, double *F, const long long *__restrict__ sbase, const int *__restrict__ swidth, double *AS,
+               int cap, int *err)
 {
-	double acc[FG_ROWCAP];
+	extern __shared__ double sacc[];                      // [cap][128]
+	double *acc = sacc + threadIdx.x;
+#define ACC(q) acc[(q) * 128]
 	for (int I = blockIdx.x * blockDim.x + threadIdx.x; I < neq; I += gridDim.x * blockDim.x) {
 		int base = IA[I], len = IA[I + 1] - base;
-		if (len > FG_ROWCAP) { fg_set_err(err, FEMGPU_E_MESH); continue; }
-		for (int q = 0; q < len; q++) acc[q] = 0.0;
+		if (len > cap) { fg_set_err(err, FEMGPU_E_MESH); continue; }
+		for (int q = 0; q < len; q++) ACC(q) = 0.0;
+		double f = 0.0;
 		for (int q = ri_ptr[I]; q < ri_ptr[I + 1]; q++) {
 			int code = __ldg(&ri[q]), e = code / 3, aa = code - 3 * e;
+			int pos[3];
+			double v[3];
+#pragma unroll
 			for (int b = 0; b < 3; b++) {
-				int pos = __ldg(&sbe[9 * e + 3 * aa + b]);
-				if (pos < nnz) acc[pos - base] += __ldg(&ke[9LL * e + 3 * aa + b]);
+				pos[b] = __ldg(&sbe[9 * e + 3 * aa + b]);
+				v[b] = __ldg(&ke[9LL * e + 3 * aa + b]);
+			}
+			if (F && fe) f += __ldg(&fe[3LL * e + aa]);
+#pragma unroll
+			for (int b = 0; b < 3; b++) {
+				if (pos[b] < nnz) ACC(pos[b] - base) += v[b];
+				else if (F && b != aa) f = lift(f, e, aa, b, ke, vert, node_type, upresc);
 			}
 		}
-		for (int q = 0; q < len; q++) AA[base + q] = acc[q];
-		if (F) F[I] = gather_F(I, ri_ptr, ri, ke, fe, vert, node_type, upresc);
+		for (int q = 0; q < len; q++) AA[base + q] = ACC(q);
+		if (AS) {
+			const int sl = I >> 5, w = __ldg(&swidth[sl]);
+			const long long at = __ldg(&sbase[sl]) + (I & 31);
+			for (int q = 0; q < w; q++) AS[at + 32LL * q] = q < len ? ACC(q) : 0.0;
+		}
+		if (F) F[I] = f;
 	}
+#undef ACC
 	if (blockIdx.x == 0 && threadIdx.x == 0) AA[nnz] = 0.0;
 }
 
@@ -697,13 +782,18 @@ __global__ void k_assemble_ede(int nedge, const int *ec_ptr, const int *ec, cons
 	}
 }
 
-__global__ void k_assemble_F(int neq, const int *ri_ptr, const int *ri, const double *ke,
+__global__ void k_assemble_F(int neq, const int *ri_ptr, const int *ri, const int *lm, const double *ke,
                              const double *fe, const int *vert, const int *node_type,
                              const double *upresc, double *F)
 {
 	for (int I = blockIdx.x * blockDim.x + threadIdx.x; I < neq; I += gridDim.x * blockDim.x)
-		F[I] = gather_F(I, ri_ptr, ri, ke, fe, vert, node_type, upresc);
+		F[I] = gather_F(I, neq, ri_ptr, ri, lm, ke, fe, vert, node_type, upresc);
 }
+
+// Entries of a row the assembly has room for (the longest row's), and its
+// shared memory.
+static int row_cap(const femgpu_transport *t) { return t->longest < FG_ROWCAP ? t->longest : FG_ROWCAP; }
+static size_t row_smem(const femgpu_transport *t) { return sizeof(double) * 128 * (size_t)row_cap(t); }
 
 // Storage assembly of the transient element matrices (the same gathers as
 // the steady build) and the residual gather into F.
@@ -712,33 +802,31 @@ extern "C" int fg_assemble_transient(femgpu_transport *t)
 	cudaStream_t s = t->stream;
 	int neq = t->neq;
 	if (t->o.scheme == FEMGPU_CSR)
-		k_assemble_csr<<<fg_grid(neq, 128, 32), 128, 0, s>>>(neq, t->nnz, t->IA, t->sbe, t->ri_ptr,
-			t->ri, t->ke, NULL, t->vert, t->node_type, t->upresc, t->A, NULL, &t->st->err);
+		k_assemble_csr<<<fg_grid(neq, 128, 32), 128, row_smem(t), s>>>(neq, t->nnz, t->IA, t->sbe, t->ri_ptr,
+			t->ri, t->ke, NULL, t->vert, t->node_type, t->upresc, t->A, NULL, t->sell_base, t->sell_w, t->sell_A,
+			row_cap(t), &t->st->err);
 	else if (t->o.scheme == FEMGPU_EDE)
 		k_assemble_ede<<<fg_grid(t->nedge + 1LL), FG_TPB, 0, s>>>(t->nedge, t->ec_ptr, t->ec, t->order,
 			t->ke, t->A);
 	k_gather_R<<<fg_grid(neq + 1LL), FG_TPB, 0, s>>>(neq, t->ri_ptr, t->ri, t->re, t->F);
-	FG_TRY(cudaGetLastError());
-	return t->o.scheme == FEMGPU_CSR ? fg_sell_refresh(t) : 0;
+	return (int)cudaGetLastError();
 }
 
 extern "C" int fg_assemble(femgpu_transport *t)
 {
 	cudaStream_t s = t->stream;
 	int neq = t->neq;
+	const double *ke = t->o.scheme == FEMGPU_EBE ? t->A : t->ke, *fe = t->fsrc_zero ? NULL : t->fe;
 	if (t->o.scheme == FEMGPU_CSR) {
-		k_assemble_csr<<<fg_grid(neq, 128, 32), 128, 0, s>>>(neq, t->nnz, t->IA, t->sbe, t->ri_ptr,
-			t->ri, t->ke, t->fe, t->vert, t->node_type, t->upresc, t->A, t->F, &t->st->err);
-		FG_TRY(cudaGetLastError());
-		return fg_sell_refresh(t);
-	} else if (t->o.scheme == FEMGPU_EDE) {
+		k_assemble_csr<<<fg_grid(neq, 128, 32), 128, row_smem(t), s>>>(neq, t->nnz, t->IA, t->sbe, t->ri_ptr,
+			t->ri, ke, fe, t->vert, t->node_type, t->upresc, t->A, t->F, t->sell_base, t->sell_w, t->sell_A,
+			row_cap(t), &t->st->err);
+		return (int)cudaGetLastError();
+	}
+	if (t->o.scheme == FEMGPU_EDE)
 		k_assemble_ede<<<fg_grid(t->nedge + 1LL), FG_TPB, 0, s>>>(t->nedge, t->ec_ptr, t->ec, t->order,
 			t->ke, t->A);
-		k_assemble_F<<<fg_grid(neq), FG_TPB, 0, s>>>(neq, t->ri_ptr, t->ri, t->ke, t->fe, t->vert,
-			t->node_type, t->upresc, t->F);
-	} else {
-		k_assemble_F<<<fg_grid(neq), FG_TPB, 0, s>>>(neq, t->ri_ptr, t->ri, t->A, t->fe, t->vert,
-			t->node_type, t->upresc, t->F);
-	}
+	k_assemble_F<<<fg_grid(neq), FG_TPB, 0, s>>>(neq, t->ri_ptr, t->ri, t->lm, ke, fe, t->vert,
+		t->node_type, t->upresc, t->F);
 	return (int)cudaGetLastError();
 }

@@ -200,23 +200,6 @@ __global__ void __launch_bounds__(256) k_sellmv(int n, const long long *__restri
 	if (GATHER) G[__ldg(&dpos[i])] = ds_from(q);
 }
 
-__global__ void k_sell_refresh(long long nslot, const int *__restrict__ src, const double *__restrict__ AA,
-                               double *__restrict__ AS)
-{
-	for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < nslot;
-	     k += (long long)gridDim.x * blockDim.x) {
-		const int q = src[k];
-		AS[k] = q >= 0 ? AA[q] : 0.0;
-	}
-}
-
-extern "C" int fg_sell_refresh(femgpu_transport *t)
-{
-	if (!t->sell_A) return 0;
-	k_sell_refresh<<<fg_grid(t->nslot), FG_TPB, 0, t->stream>>>(t->nslot, t->sell_src, t->A, t->sell_A);
-	return (int)cudaGetLastError();
-}
-
 // The FGMRES operator (fused form) that also writes the ILU sweeps' gathered
 // double-single input.
 static int sellmv_gather(femgpu_transport *t, const double *P, double *Q, const int *active)

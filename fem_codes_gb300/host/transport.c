@@ -83,43 +83,36 @@ static int sync_err(femgpu_transport *t)
 
 /* The SELL-32 layout of the CSR pattern (rows in slices of 32, each slice
  * padded to its longest row and stored entry index by entry index): the
- * slots' columns, their CSR positions and the slice offsets. */
+ * slots' columns and the slice offsets; the assembly writes the values. */
 static int build_sell(femgpu_transport *t, const int *IA, const int *JA)
 {
 	const int n = t->neq, ns = (n + 31) / 32;
 	long long *base = malloc(sizeof(long long) * ((size_t)ns + 1)), nslot = 0;
-	int *w = malloc(sizeof(int) * (size_t)ns), *src = NULL, *col = NULL, s, r, j, rc = 0;
+	int *w = malloc(sizeof(int) * (size_t)ns), *col = NULL, s, r, j, rc = 0;
 	if (!base || !w) { free(base); free(w); return FEMGPU_E_NOMEM; }
 	for (s = 0; s < ns; s++) {
 		int wm = 0;
 		for (r = 32 * s; r < n && r < 32 * s + 32; r++) if (IA[r + 1] - IA[r] > wm) wm = IA[r + 1] - IA[r];
 		base[s] = nslot;
 		w[s] = wm;
+		if (wm > t->longest) t->longest = wm;
 		nslot += 32LL * wm;
 	}
 	base[ns] = nslot;
-	src = malloc(sizeof(int) * ((size_t)nslot + 1));
-	col = malloc(sizeof(int) * ((size_t)nslot + 1));
-	if (!src || !col) rc = FEMGPU_E_NOMEM;
+	col = calloc((size_t)nslot + 1, sizeof(int));
+	if (!col) rc = FEMGPU_E_NOMEM;
 	if (!rc) {
-		long long k;
-		for (k = 0; k < nslot; k++) { src[k] = -1; col[k] = 0; }
 		for (r = 0; r < n; r++)
-			for (j = 0; j < IA[r + 1] - IA[r]; j++) {
-				long long at = base[r / 32] + 32LL * j + (r & 31);
-				src[at] = IA[r] + j;
-				col[at] = JA[IA[r] + j];
-			}
+			for (j = 0; j < IA[r + 1] - IA[r]; j++) col[base[r / 32] + 32LL * j + (r & 31)] = JA[IA[r] + j];
 		t->nslice = ns;
 		t->nslot = nslot;
 		if (upload((void **)&t->sell_base, base, sizeof(long long) * ((size_t)ns + 1)) ||
 		    upload((void **)&t->sell_w, w, sizeof(int) * (size_t)ns) ||
-		    upload((void **)&t->sell_src, src, sizeof(int) * ((size_t)nslot + 1)) ||
 		    upload((void **)&t->sell_JA, col, sizeof(int) * ((size_t)nslot + 1)) ||
 		    fgh_dmalloc((void **)&t->sell_A, sizeof(double) * ((size_t)nslot + 1)))
 			rc = FEMGPU_E_NOMEM;
 	}
-	free(base); free(w); free(src); free(col);
+	free(base); free(w); free(col);
 	return rc;
 }
 
@@ -352,7 +345,7 @@ void femgpu_transport_destroy(femgpu_transport *t)
 		t->ec, t->e2_ptr, t->e2, t->A, t->ke, t->fe, t->A32, t->u, t->F, t->F0, t->invDiag,
 		t->invDiag32, t->ilu.LU, t->ilu.Dinv, t->V, t->H, t->cs, t->sn, t->ge, t->gy, t->w2,
 		t->Z, t->Z32, t->xr, t->dr, t->partials, t->orth, t->st, t->du, t->uold, t->Da, t->re, t->dold,
-		t->u1, t->u2, t->uB, t->aB, t->bub, t->uB1, t->uB2, t->la_buf, t->la_flag, t->sell_base, t->sell_w, t->sell_src, t->sell_JA, t->sell_A };
+		t->u1, t->u2, t->uB, t->aB, t->bub, t->uB1, t->uB2, t->la_buf, t->la_flag, t->sell_base, t->sell_w, t->sell_JA, t->sell_A };
 	for (i = 0; i < (int)(sizeof ptrs / sizeof ptrs[0]); i++) if (ptrs[i]) cudaFree(ptrs[i]);
 	if (t->la_s) {
 		cudaStreamSynchronize(t->la_s);
