@@ -27,7 +27,8 @@ extern "C" {
 
 /* One triangular sweep compiled into level blocks (see ilu.cu). */
 typedef struct fg_sweep {
-	int nlev, nsb;             /* levels, sub-blocks (<= 512 rows each)      */
+	int nlev, nsb;             /* levels, sub-blocks (<= 512 rows each; 32
+	                            * when swept without level barriers)         */
 	long long bytes, maxblk, nval;
 	int npad;                  /* padded length of the level-ordered vector  */
 	unsigned char *prog;       /* sub-blocks                                 */
@@ -42,10 +43,11 @@ typedef struct fg_sweep {
 	int *chunk_sb, *chunk_lev; /* [nchunk+1] first sub-block / level of each */
 	int rw;                    /* record layout width (0: ELL sub-blocks)    */
 	int df;                    /* record layout swept without level barriers */
-	int skew;                  /* ... levels a warp may run ahead            */
+	int ring, look, warps;     /* ... ring slots, chunks a warp may run
+	                            * ahead, warps of a block                    */
 	int bvo, cmax;             /* record layout: input slice offset in a
 	                            * stage, most rows of a sub-block            */
-	/* chain-scan programs (k_sweep_cs): levels of warp segments, 32 slots a
+	/* chain-scan programs: levels of warp segments, 32 slots a
 	 * segment chunk; per slot the byte offset of its five scan multipliers
 	 * (-1: padding), the CSR position of its chain coefficient (-1: none)
 	 * and its row */

@@ -8,19 +8,20 @@
 //   * at set-up, each sweep is compiled into a "program": every level is cut
 //     into sub-blocks of at most SW_SUB rows, 16-byte aligned -- one record
 //     per row (dependency codes, output slot, factor values, the inverted
-//     pivot backward; k_sweep_rec / k_sweep_df) when no row has more than 16
+//     pivot backward; k_sweep_df / k_sweep_rec) when no row has more than 16
 //     dependencies, else ELL arrays (k_sweep); factor values are refreshed
 //     after every factorisation;
-//   * one producer warp streams sub-blocks (and their slice of the input
-//     vector) into a ring of shared-memory stages with TMA bulk copies
-//     (cp.async.bulk, completion on a "full" mbarrier; stage reuse gated by an
-//     "empty" mbarrier the consumer warps arrive on);
-//   * consumer warps compute a level, publish its values in a shared-memory
-//     ring indexed by level-order position (older dependencies are re-read
-//     from global memory) and synchronise either with one named barrier per
-//     level (k_sweep, k_sweep_rec) or through per-warp progress flags that a
-//     warp waits on only for the warps it reads from (k_sweep_df, the
-//     default for records).
+//   * records: chunks of up to 32 rows are dealt to the warps in turn; each
+//     warp streams its chunks (and their slice of the input vector) into
+//     shared-memory stages of its own with TMA bulk copies and polls the values
+//     its rows read in a shared-memory ring (k_sweep_df, k_sweep_fb);
+//   * ELL arrays and FEMGPU_SWEEP_SYNC=barrier: one producer warp streams the
+//     sub-blocks into a ring of stages (cp.async.bulk, completion on a "full"
+//     mbarrier; stage reuse gated by an "empty" mbarrier), consumer warps
+//     compute a level, publish its values in a shared-memory ring indexed by
+//     level-order position and meet at one named barrier per level (k_sweep,
+//     k_sweep_rec);
+//   * dependencies older than the ring are re-read from global memory.
 // Rows are computed in the reference's order (ascending columns) and the
 // FP64 variant rounds each operation separately, so its results are
 // bit-identical to the reference's sweeps; FGMRES uses the fused
@@ -48,11 +49,12 @@
 #define SW_MAXW 8                     // dependencies per row on the unrolled path
 #define SW_RPT 4                      // rows per consumer thread per pass
 #define SW_RING 4096                  // ring slots (power of two)
-#define SW_NEAR 0x80000000u           // dependency code: ring slot
+#define SW_RING_WIDE 8192             // ... of dataflow programs with wide levels
+#define SW_NEAR 0x80000000u           // dependency code: ring slot (dataflow programs: global position)
 #define SW_WAIT_LIMIT (1 << 24)
 #define SW_MAXD 12                    // max stages
 #define SW_BAR_BYTES (2 * SW_MAXD * 8)
-#define SW_SMEM_CAP (220 * 1024)
+#define SW_SMEM_CAP (226 * 1024)
 #define SW_HDR 32
 
 // ------------------------------------------------------------ PTX helpers
@@ -211,7 +213,7 @@ struct SweepArgs {
 	const int *chunk_sb;          // [P+1] first sub-block of each matrix block (NULL: one block)
 	const int *chunk_lev;         // [P+1] first level of each matrix block
 	int bvo, cmax;                // record layout: input slice offset, most rows of a sub-block
-	int skew;                     // dataflow: levels a warp may run ahead of the slowest one
+	int ring, look;               // dataflow: ring slots (power of two), chunks a warp may run ahead
 	int wait;                     // spins of a warp waiting for the rows it depends on
 };
 
@@ -384,7 +386,6 @@ __host__ __device__ constexpr int rec_bytes(int w, bool upper, int ts)
 	                                                        : rec_ib(w) + rec_vb(w, upper, ts) + 16;
 }
 #define SW2_CW FG_SW2_CW              // consumer warps of the record-layout sweep (SW_SUB rows)
-#define NEED_STRIDE (((SW2_CW) + 15) / 16 * 16)   // bytes of a warp's need table
 
 template <typename T, bool UPPER, bool FMA, int W>
 __global__ void __launch_bounds__((SW2_CW + 1) * 32, 1)
@@ -474,133 +475,105 @@ k_sweep_rec(SweepArgs a, const T *__restrict__ in, T *out)
 }
 
 // ------------------------------------------- dataflow sweep (record layout)
-// The same records, without a barrier per level: every consumer warp
-// publishes the last level it has finished (prog[warp], shared memory) and,
-// before computing a sub-block, waits only for the warps whose rows its own
-// rows read (a table of 16 bytes per warp in the sub-block header: for each
-// producer warp the smallest level distance of a dependency it supplies, 255
-// when it supplies none within S + 1 levels) and for every warp to have
-// finished level l - S - 1 (S = the program's skew).  The second wait bounds
-// how far warps drift apart, so a ring slot is rewritten only after every
-// reader of its old value is done: the program reads from the ring only
-// dependencies within SW_RING - S * (widest level) positions of their level's
-// end.  A warp publishes a level with a release store right after its ring
-// writes and only then stores the level's outputs to global memory, so no
-// level waits for its own global stores; a dependency read back from global
-// memory therefore waits for its producer's next level (whose release covers
-// those stores), and the program keeps such dependencies at least two levels
-// back.  A warp releases a stage (mbarrier of CW arrivals) as soon as its
-// rows are in registers.  Header: {rows, sub-blocks of the level, first
-// position, far flag}, then CW need tables of 16 bytes, then the records.
-#define DF_HDR (16 + SW2_CW * NEED_STRIDE)
+// The same records without barriers or a producer warp.  A level is cut into
+// chunks of up to 32 rows and the chunks of a matrix block are dealt to the
+// block's warps in turn, so consecutive levels go to different warps: a warp
+// stages its own chunks (bulk copies into D stages of its own, one mbarrier
+// each), takes its next record and its rows' older dependencies while other
+// warps compute the levels before, and only the newest value's arrival and the
+// operations on it stand between two levels.  (With level l's rows always on
+// warps 0, 1, ... a level took one warp's whole turn, about 980 clocks, the
+// values it waited for being there long before it looked.)
+//
+// Ring slots hold the mark "not yet written" (all ones: a NaN no arithmetic
+// produces; a value with these bits is stored as the ordinary NaN) until their
+// value is there, and a row polls the values it reads: one trip through shared
+// memory from a producer to its readers.  A row's terms are taken in order,
+// each as soon as its value is there.
+//
+// Ring slot of lane t of chunk c: 32 c + t modulo the ring (R chunks).  Slots
+// are marked again by the writers: chunk c marks chunk c - (R - X - 1).  Warps
+// publish their progress (prog[warp]: all its chunks below are done; release)
+// and chunk c starts only when all chunks below c - X are done.  A chunk reads
+// from the ring at most R - 2 X - 2 chunks back, so nobody still reads what is
+// marked, and the chunk that takes the slot next (X + 1 past c) starts only
+// when c is done and its marks are known.  Older dependencies come from global
+// memory: a warp stores a chunk's outputs after publishing it, so they are
+// there once the warp has published its next one; the chunk's header holds
+// what it has to wait for (1 + its last chunk with such a dependency, 0: none;
+// the program keeps them more than one turn of all warps back).
+// Header: {rows, 0, 0, far}, then the records.
+//
+// Both sweeps of an application, before (per-warp progress flags, rows of a
+// level always on the first warps) and now: 64x64 cells, 2 x 127 levels, FP64:
+// 117 us, 67; 400x300 cells, 2 x 1098 levels, FP64: 1.50 ms, 0.80; 2048x1024
+// cells in 32 blocks, double-single chains, the largest block 9106 chunks:
+// 0.70 ms, 0.46.  FP64: a level is a poll (about 100 clocks) and the newest
+// values' multiplications and subtractions, 64 clocks each on a warp; four
+// chunks a level and more keep the four FP64 pipes (6 or 7 such operations a
+// chunk) half busy.  Double-single: issue slots, about 130 FP32 operations a
+// chunk of some 380 slots.
+#define DF_HDR 16
+#define DF_WARPS 24                   // most warps of a block
+#define DF_MAXD 8                     // ... stages of a warp
+#define DF_BARS 128                   // most stages of a block
+#define DF_DONE 0x7fffffff
+// Warps: rows in FP64 wait for their level (20 or 24 warps gain nothing over
+// 16); a chain chunk is a long run of dependent FP32 operations, so the narrow
+// ones, whose registers allow it, take 24 (2048x1024, 32 blocks: 667 us an
+// application with 16, 586 with 20, 554 with 24).
+__host__ __device__ constexpr int df_warps(bool cs, int w) { return cs && w <= 4 ? 24 : 16; }
 
-template <typename T, bool UPPER, bool FMA, int W>
-__global__ void __launch_bounds__((SW2_CW + 1) * 32, 1)
-k_sweep_df(SweepArgs a, const T *__restrict__ in, T *out)
+// Ring values: polled loads, stores, the mark.
+template <typename T> __device__ __forceinline__ bool ring_unset(T v)
 {
-	constexpr int CW = SW2_CW;
-	constexpr int IB = rec_ib(W), VB = rec_vb(W, UPPER, (int)sizeof(T)), RB = rec_bytes(W, UPPER, (int)sizeof(T));
-	static_assert(SW_SUB == CW * 32, "one row per consumer thread and sub-block");
-	static_assert(CW <= NEED_STRIDE && CW <= 32, "one need byte per consumer warp in a warp's table");
-	if (a.active && !*a.active) return;
-	extern __shared__ __align__(128) unsigned char sm[];
-	const unsigned ring_b = (unsigned)al16((SW_RING + 1) * sizeof(T));
-	T *ring = (T *)sm;
-	unsigned long long *full = (unsigned long long *)(sm + ring_b);
-	unsigned long long *empty = full + SW_MAXD;
-	unsigned char *stages = sm + ((ring_b + SW_BAR_BYTES + 127) & ~127u);
-	__shared__ int failed, issued, pdone;
-	__shared__ int prog[CW];
-	volatile int *vfailed = &failed;
-	const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, D = a.D;
-	const unsigned sbytes = (unsigned)a.stage_bytes;
-	const int sb0 = a.chunk_sb ? a.chunk_sb[blockIdx.x] : 0, sb1 = a.chunk_sb ? a.chunk_sb[blockIdx.x + 1] : a.nsb;
-	const int l0 = a.chunk_lev ? a.chunk_lev[blockIdx.x] : 0, l1 = a.chunk_lev ? a.chunk_lev[blockIdx.x + 1] : a.nlev;
-
-	if (tid == 0) {
-		failed = 0; issued = 0; pdone = 0;
-		ring[SW_RING] = T(0);
-		for (int s = 0; s < D; s++) { mbar_init(&full[s], 1); mbar_init(&empty[s], CW); }
-		fence_mbar_init();
+	if (sizeof(T) == 8) {
+		const uint2 u = *(const uint2 *)&v;
+		return (u.x & u.y) == ~0u;
 	}
-	if (tid < CW) prog[tid] = -1;
-	__syncthreads();
-
-	if (warp == CW) {                                     // ---- producer warp
-		sweep_producer(a, in, stages, sbytes, full, empty, D, sb0, sb1, lane, vfailed, &issued, &pdone, true);
-		return;
-	}
-
-	const int ctid = tid;                                 // ---- consumer warps
-	const unsigned roff = (unsigned)DF_HDR + (unsigned)(ctid < a.cmax ? ctid : a.cmax - 1) * RB;
-	const unsigned boff = (unsigned)a.bvo + (unsigned)(ctid < a.cmax ? ctid : a.cmax - 1) * sizeof(T);
-	int s = 0, waited = 0;
-	unsigned ph = 0;
-	bool fail = false;
-	T ydef = T(0);                                        // an output not yet stored to global memory
-	int odef = -1;
-	for (int l = l0; l < l1 && !fail; l++) {
-		const int ll = l - l0;
-		int nsub = 1;
-		for (int j = 0; j < nsub; j++) {
-			if (!mbar_wait_or_fail(&full[s], ph, vfailed)) { *vfailed = 1; fail = true; break; }
-			waited++;
-			const unsigned char *st = stages + (unsigned)s * sbytes;
-			union { int4 q[IB / 16]; int i[IB / 4]; } ci;
-			union { int4 q[VB / 16]; T v[VB / sizeof(T)]; } cv;
-#pragma unroll
-			for (int k = 0; k < IB / 16; k++) ci.q[k] = ((const int4 *)(st + roff))[k];
-#pragma unroll
-			for (int k = 0; k < VB / 16; k++) cv.q[k] = ((const int4 *)(st + roff + IB))[k];
-			const T x0 = *(const T *)(st + boff);
-			const int4 h = *(const int4 *)st;
-			const int need = lane < CW ? (int)st[16 + warp * NEED_STRIDE + lane] : 255;
-			if (j == 0) nsub = h.y;
-			__syncwarp();
-			if (lane == 0) mbar_arrive(&empty[s]);        // this warp's rows are in registers
-			if (++s == D) { s = 0; ph ^= 1u; }
-			if (32 * warp >= h.x) continue;               // no rows of this warp here
-			// producers of this warp's dependencies, and every warp within the skew
-			const int want = ll - (need == 255 ? a.skew + 1 : need);
-			bool ready = false;
-			for (int it = 0; it < a.wait; it++) {
-				const bool mine = lane >= CW || lane == warp || ld_acquire_cta(&prog[lane]) >= want;
-				if (__all_sync(0xffffffffu, mine)) { ready = true; break; }
-				if (__any_sync(0xffffffffu, *vfailed != 0)) break;
-			}
-			if (!ready) { *vfailed = 1; fail = true; break; }
-			__syncwarp();                                 // the lanes' acquires order every lane's reads
-			T d[W];
-#pragma unroll
-			for (int k = 0; k < W; k++) {
-				unsigned c = (unsigned)ci.i[k] & ~SW_NEAR;
-				d[k] = ring[c < SW_RING ? c : SW_RING];
-			}
-			if (ctid < h.x) {
-				if (h.w) {
-#pragma unroll
-					for (int k = 0; k < W; k++)
-						if (!((unsigned)ci.i[k] & SW_NEAR)) d[k] = __ldcg(&out[ci.i[k]]);
-				}
-				T y = x0;
-#pragma unroll
-				for (int k = 0; k < W; k++) y = fmsub<T, FMA>(y, d[k], cv.v[k]);
-				if (UPPER) y = mul(y, cv.v[W]);
-				ring[(h.z + ctid) & (SW_RING - 1)] = y;
-				if (odef >= 0) out[odef] = ydef;          // an earlier sub-block of this level
-				ydef = y;
-				odef = ci.i[W];
-			}
-		}
-		if (fail) break;
-		__syncwarp();
-		if (lane == 0) st_release_cta(&prog[warp], ll);
-		if (odef >= 0) { out[odef] = ydef; odef = -1; }
-	}
-	consumer_sync<CW>();
-	if (*vfailed && ctid == 0) sweep_drain(a, full, D, waited, &issued, &pdone);
+	return *(const unsigned *)&v == ~0u;
 }
-
+template <typename T> __device__ __forceinline__ T ring_ld(unsigned p)      // p: a shared-memory address
+{
+	T v;
+	if (sizeof(T) == 8) {
+		unsigned long long u;
+		asm volatile("ld.relaxed.cta.shared.u64 %0, [%1];" : "=l"(u) : "r"(p) : "memory");
+		*(unsigned long long *)&v = u;
+	} else {
+		unsigned u;
+		asm volatile("ld.relaxed.cta.shared.u32 %0, [%1];" : "=r"(u) : "r"(p) : "memory");
+		*(unsigned *)&v = u;
+	}
+	return v;
+}
+template <typename T> __device__ __forceinline__ void ring_st(unsigned p, T v)
+{
+	if (sizeof(T) == 8)
+		asm volatile("st.relaxed.cta.shared.u64 [%0], %1;" :: "r"(p), "l"(*(const unsigned long long *)&v) : "memory");
+	else
+		asm volatile("st.relaxed.cta.shared.u32 [%0], %1;" :: "r"(p), "r"(*(const unsigned *)&v) : "memory");
+}
+template <typename T> __device__ __forceinline__ T ring_mark()
+{
+	T v;
+	if (sizeof(T) == 8) *(unsigned long long *)&v = ~0ull;
+	else *(unsigned *)&v = ~0u;
+	return v;
+}
+template <typename T> __device__ __forceinline__ T ring_value(T v)       // never the mark
+{
+	if (ring_unset(v)) {
+		if (sizeof(T) == 8) *(unsigned long long *)&v = 0x7ff8000000000000ull;
+		else *(unsigned *)&v = 0x7fc00000u;
+	}
+	return v;
+}
+template <> __device__ __forceinline__ dsf ring_value(dsf v)
+{
+	if (ring_unset(v)) v.hi = __uint_as_float(0x7fc00000u);
+	return v;
+}
 // ------------------------------------------------ chain-scan sweep (records)
 // After SYMRCM the rows of a matrix block form fronts, and along a front every
 // row depends on its predecessor in the sweep order: y_i = a_i + b_i y_pred,
@@ -619,163 +592,236 @@ k_sweep_df(SweepArgs a, const T *__restrict__ in, T *out)
 // for bit: it serves the fused-arithmetic (FGMRES) and FP32 sweeps only.
 // Records: W dependency codes (the predecessor excluded) and the output slot
 // (-1: padding), then W values, the inverted pivot (backward) and M_0..M_4.
-// Staging, progress flags, need tables and bounded waits are k_sweep_df's.
+// Staging, ring and bounded waits are the dataflow sweep's.
 __host__ __device__ constexpr int rec_vb_cs(int w, bool upper, int ts) { return ((w + (upper ? 1 : 0) + 5) * ts + 15) & ~15; }
-__host__ __device__ constexpr int rec_bytes_cs(int w, bool upper, int ts)
-{
-	return (((rec_ib(w) + rec_vb_cs(w, upper, ts)) / 16) & 1) ? rec_ib(w) + rec_vb_cs(w, upper, ts)
-	                                                           : rec_ib(w) + rec_vb_cs(w, upper, ts) + 16;
-}
 
 template <typename T> __device__ __forceinline__ T fma_t(T a, T b, T c);
 template <> __device__ __forceinline__ double fma_t(double a, double b, double c) { return fma(a, b, c); }
 template <> __device__ __forceinline__ float fma_t(float a, float b, float c) { return fmaf(a, b, c); }
 template <> __device__ __forceinline__ dsf fma_t(dsf a, dsf b, dsf c) { return ds_fma(a, b, c); }
 
-// One chain-scan sweep of this thread block's matrix block: the staging,
-// dataflow and scan of k_sweep_cs, on the barriers full/empty (D of them);
-// every thread returns after a block barrier, true when a wait gave up.
-template <typename T, bool UPPER, int W>
-__device__ __forceinline__ bool cs_sweep(const SweepArgs &a, const T *__restrict__ in, T *out, unsigned char *sm,
-                                         unsigned long long *full, unsigned long long *empty, int *failed,
-                                         int *issued, int *pdone, int *prog)
-{
-	constexpr int CW = SW2_CW;
-	constexpr int IB = rec_ib(W), VB = rec_vb_cs(W, UPPER, (int)sizeof(T)), RB = rec_bytes_cs(W, UPPER, (int)sizeof(T));
-	constexpr int MO = W + (UPPER ? 1 : 0);              // first scan multiplier
-	static_assert(SW_SUB == CW * 32, "one slot per consumer thread and sub-block");
-	const unsigned ring_b = (unsigned)al16((SW_RING + 1) * sizeof(T));
-	T *ring = (T *)sm;
-	unsigned char *stages = sm + ((ring_b + SW_BAR_BYTES + 127) & ~127u);
-	volatile int *vfailed = failed;
-	const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, D = a.D;
-	const unsigned sbytes = (unsigned)a.stage_bytes;
-	const int sb0 = a.chunk_sb ? a.chunk_sb[blockIdx.x] : 0, sb1 = a.chunk_sb ? a.chunk_sb[blockIdx.x + 1] : a.nsb;
-	const int l0 = a.chunk_lev ? a.chunk_lev[blockIdx.x] : 0, l1 = a.chunk_lev ? a.chunk_lev[blockIdx.x + 1] : a.nlev;
-
-	if (tid == 0) {
-		*failed = 0; *issued = 0; *pdone = 0;
-		ring[SW_RING] = zero_t<T>();
-		for (int s = 0; s < D; s++) { mbar_init(&full[s], 1); mbar_init(&empty[s], CW); }
-		fence_mbar_init();
+// A row's record in registers.  Row programs: the rows' records one after the
+// other; chain programs (32 rows to a chunk always): the lanes' 16-byte words
+// side by side, without the padding that keeps whole records off each other's
+// banks.
+template <typename T, bool UPPER, bool CS, int W> struct SweepRec {
+	static constexpr int IB = rec_ib(W), VB = CS ? rec_vb_cs(W, UPPER, (int)sizeof(T)) : rec_vb(W, UPPER, (int)sizeof(T));
+	static constexpr int FIRST = CS ? 16 : rec_bytes(W, UPPER, (int)sizeof(T)), STEP = CS ? 512 : 16;
+	int i[IB / 4];
+	T v[VB / sizeof(T)];
+	T x0;
+	int rows, far;
+	__device__ __forceinline__ void load(const unsigned char *st, unsigned roff, unsigned boff)
+	{
+#pragma unroll
+		for (int k = 0; k < IB / 16; k++) {
+			const int4 q = *(const int4 *)(st + roff + k * STEP);
+			i[4 * k] = q.x; i[4 * k + 1] = q.y; i[4 * k + 2] = q.z; i[4 * k + 3] = q.w;
+		}
+#pragma unroll
+		for (int k = 0; k < VB / 16; k++) {
+			union { int4 q; T t[16 / sizeof(T)]; } u;
+			u.q = *(const int4 *)(st + roff + (IB / 16 + k) * STEP);
+#pragma unroll
+			for (int j = 0; j < (int)(16 / sizeof(T)); j++) v[k * (16 / sizeof(T)) + j] = u.t[j];
+		}
+		x0 = *(const T *)(st + boff);
+		rows = CS ? 32 : *(const int *)st;
+		far = *(const int *)(st + 12);
 	}
-	if (tid < CW) prog[tid] = -1;
+};
+
+// One sweep of this thread block's matrix block with the barriers `full' (D a
+// warp); every thread returns after a block barrier, true when a wait gave up.
+// CS: a chain-scan program.
+template <typename T, bool UPPER, bool FMA, bool CS, int W>
+__device__ __forceinline__ bool sweep_run(const SweepArgs &a, const T *__restrict__ in, T *out, unsigned char *sm,
+                                          unsigned long long *full, int *failed, int *prog)
+{
+	typedef SweepRec<T, UPPER, CS, W> Rec;
+	const unsigned mask = (unsigned)a.ring - 1, rb = smem_u32(sm), zero = rb + (unsigned)a.ring * (unsigned)sizeof(T);
+	const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, D = a.D, nw = blockDim.x >> 5;
+	const int sb0 = a.chunk_sb[blockIdx.x], cnt = a.chunk_sb[blockIdx.x + 1] - sb0;
+	unsigned char *stages = sm + (((unsigned)al16((a.ring + 1) * sizeof(T)) + 2 * DF_BARS * 8 + 127) & ~127u) +
+	                        (unsigned)(warp * D) * (unsigned)a.stage_bytes;
+	volatile int *vfailed = failed;
+	full += warp * D;
+
+	if (tid == 0) *failed = 0;
+	if (lane == 0) {
+		for (int s = 0; s < D; s++) mbar_init(&full[s], 1);
+		fence_mbar_init();
+		prog[warp] = warp < cnt ? warp : DF_DONE;
+	}
+	for (int q = tid; q <= a.ring; q += blockDim.x) ((T *)sm)[q] = q < a.ring ? ring_mark<T>() : zero_t<T>();
 	__syncthreads();
 
-	if (warp == CW) {                                     // ---- producer warp
-		sweep_producer(a, in, stages, sbytes, full, empty, D, sb0, sb1, lane, vfailed, issued, pdone, true);
-	} else {                                              // ---- consumer warps
-		const int ctid = tid;
-		const unsigned roff = (unsigned)DF_HDR + (unsigned)(ctid < a.cmax ? ctid : a.cmax - 1) * RB;
-		const unsigned boff = (unsigned)a.bvo + (unsigned)(ctid < a.cmax ? ctid : a.cmax - 1) * sizeof(T);
-		int s = 0, waited = 0;
-		unsigned ph = 0;
-		bool fail = false;
-		T ydef = zero_t<T>();                             // an output not yet stored to global memory
-		int odef = -1;
-		for (int l = l0; l < l1 && !fail; l++) {
-			const int ll = l - l0;
-			int nsub = 1;
-			for (int j = 0; j < nsub; j++) {
-				if (!mbar_wait_or_fail(&full[s], ph, vfailed)) { *vfailed = 1; fail = true; break; }
-				waited++;
-				const unsigned char *st = stages + (unsigned)s * sbytes;
-				union { int4 q[IB / 16]; int i[IB / 4]; } ci;
-				union { int4 q[VB / 16]; T v[VB / sizeof(T)]; } cv;
+	// row programs: lane k: where turn tb + k's chunk and its input slice lie (and, mn, turn tb + 32 + k's)
+	struct Meta { long long off; int len, p0, vb; } m, mn;
+	auto meta = [&](int turn) {
+		Meta r = { 0, 0, 0, 0 };
+		const long long c = warp + (long long)turn * nw;
+		if (c < cnt) {
+			const int i = sb0 + (int)c;
+			r.off = __ldg(&a.blk_off[i]);
+			r.len = (int)(__ldg(&a.blk_off[i + 1]) - r.off);
+			r.p0 = __ldg(&a.sb_in[i]);
+			r.vb = __ldg(&a.sb_inb[i]);
+		}
+		return r;
+	};
+	int tb = 0;
+	if (!CS) { m = meta(lane); mn = meta(32 + lane); }
+	auto issue = [&](int turn, int s) {                   // turn's chunk into stage s (turns in order)
+		long long off;
+		int len, p0, vb;
+		if (CS) {                                         // whole chunks, one after the other
+			const int i = sb0 + warp + turn * nw;
+			len = a.bvo; off = (long long)i * len; p0 = 32 * i; vb = 32 * (int)sizeof(T);
+		} else {
+			if (turn == tb + 32) { tb += 32; m = mn; mn = meta(tb + 32 + lane); }
+			const int k = turn - tb;
+			off = __shfl_sync(0xffffffffu, m.off, k);
+			len = __shfl_sync(0xffffffffu, m.len, k);
+			p0 = __shfl_sync(0xffffffffu, m.p0, k);
+			vb = __shfl_sync(0xffffffffu, m.vb, k);
+		}
+		if (lane == 0) {
+			unsigned char *dst = stages + (unsigned)s * (unsigned)a.stage_bytes;
+			fence_proxy_async();
+			mbar_expect_tx(&full[s], (unsigned)(len + vb));
+			bulk_g2s(dst, a.prog + off, (unsigned)len, &full[s]);
+			bulk_g2s(dst + (unsigned)a.bvo, in + p0, (unsigned)vb, &full[s]);
+		}
+	};
+	const int turns = warp < cnt ? (cnt - warp + nw - 1) / nw : 0;
+	int issued = 0, waited = 0;
+	for (; issued < D && issued < turns; issued++) issue(issued, issued);
+
+	const int rl = lane < a.cmax ? lane : a.cmax - 1;     // rows past a chunk's count are read but not used
+	const unsigned roff = (unsigned)DF_HDR + (unsigned)rl * Rec::FIRST, boff = (unsigned)a.bvo + (unsigned)rl * sizeof(T);
+	int s = 0, known = -DF_DONE;
+	unsigned ph = 0;
+	bool fail = false;
+	for (int t = 0; t < turns && !fail; t++) {
+		const int c = warp + t * nw;
+		if (!mbar_wait_or_fail(&full[s], ph, vfailed)) { fail = true; break; }
+		waited++;
+		Rec cur;
+		cur.load(stages + (unsigned)s * (unsigned)a.stage_bytes, roff, boff);
+		__syncwarp();                                     // the chunk is in registers: its stage takes the next
+		if (issued < turns) { issue(issued, s); issued++; }
+		if (++s == D) { s = 0; ph ^= 1u; }
+		// every chunk below c - X, and a far dependency's warp past its next chunk
+		const int far = cur.far, want = max(c - a.look, far ? far + nw : 0);
+		for (int it = 0; known < want && it < a.wait; it++) {
+			known = __reduce_min_sync(0xffffffffu, lane < nw && lane != warp ? ld_acquire_cta(&prog[lane]) : DF_DONE);
+			if (known < want && (it & 63) == 63 && __any_sync(0xffffffffu, *vfailed != 0)) break;
+		}
+		if (known < want) { fail = true; break; }
+		__syncwarp();                                     // the lanes' acquires order every lane's reads
+		const bool on = CS || lane < cur.rows;
+		unsigned src[W];
+		T d[W], y = cur.x0;
 #pragma unroll
-				for (int k = 0; k < IB / 16; k++) ci.q[k] = ((const int4 *)(st + roff))[k];
+		for (int k = 0; k < W; k++) src[k] = on ? rb + (unsigned)cur.i[k] : zero;
+		if (far) {
 #pragma unroll
-				for (int k = 0; k < VB / 16; k++) cv.q[k] = ((const int4 *)(st + roff + IB))[k];
-				const T x0 = *(const T *)(st + boff);
-				const int4 h = *(const int4 *)st;
-				const int need = lane < CW ? (int)st[16 + warp * NEED_STRIDE + lane] : 255;
-				if (j == 0) nsub = h.y;
-				__syncwarp();
-				if (lane == 0) mbar_arrive(&empty[s]);    // this warp's slots are in registers
-				if (++s == D) { s = 0; ph ^= 1u; }
-				if (32 * warp >= h.x) continue;           // no chunk of this warp here (uniform)
-				const int want = ll - (need == 255 ? a.skew + 1 : need);
-				bool ready = false;
-				for (int it = 0; it < a.wait; it++) {
-					const bool mine = lane >= CW || lane == warp || ld_acquire_cta(&prog[lane]) >= want;
-					if (__all_sync(0xffffffffu, mine)) { ready = true; break; }
-					if (__any_sync(0xffffffffu, *vfailed != 0)) break;
+			for (int k = 0; k < W; k++)                   // read back from global memory (below), zero meanwhile
+				if (on && ((unsigned)cur.i[k] & SW_NEAR)) src[k] = zero;
+		}
+		bool miss = false;
+#pragma unroll
+		for (int k = 0; k < W; k++) d[k] = ring_ld<T>(src[k]);
+		if (far) {
+#pragma unroll
+			for (int k = 0; k < W; k++)
+				if (on && ((unsigned)cur.i[k] & SW_NEAR)) d[k] = ld_cg(&out[(unsigned)cur.i[k] & ~SW_NEAR]);
+		}
+#pragma unroll
+		for (int k = 0; k < W; k++) miss = miss || ring_unset(d[k]);
+		if (!__any_sync(0xffffffffu, miss)) {
+#pragma unroll
+			for (int k = 0; k < W; k++) y = fmsub<T, FMA>(y, d[k], cur.v[k]);
+		} else {
+#pragma unroll
+			for (int k = 0; k < W; k++) {
+				if (__any_sync(0xffffffffu, ring_unset(d[k]))) {
+					int it = 0;
+					do {
+						if (it >= a.wait || ((it & 63) == 63 && __any_sync(0xffffffffu, *vfailed != 0))) { fail = true; break; }
+						it++;
+						if (ring_unset(d[k])) d[k] = ring_ld<T>(src[k]);
+					} while (__any_sync(0xffffffffu, ring_unset(d[k])));
+					if (fail) break;
+#pragma unroll
+					for (int q = k + 1; q < W; q++)       // the others may have come meanwhile
+						if (ring_unset(d[q])) d[q] = ring_ld<T>(src[q]);
 				}
-				if (!ready) { *vfailed = 1; fail = true; break; }
-				__syncwarp();
-				T d[W];
-#pragma unroll
-				for (int k = 0; k < W; k++) {
-					unsigned c = (unsigned)ci.i[k] & ~SW_NEAR;
-					d[k] = ring[c < SW_RING ? c : SW_RING];
-				}
-				if (h.w) {
-#pragma unroll
-					for (int k = 0; k < W; k++)
-						if (!((unsigned)ci.i[k] & SW_NEAR)) d[k] = ld_cg(&out[ci.i[k]]);
-				}
-				T y = x0;
-#pragma unroll
-				for (int k = 0; k < W; k++) y = fmsub<T, true>(y, d[k], cv.v[k]);
-				if (UPPER) y = mul(y, cv.v[W]);
-				// the segments' recurrences across the warp's lanes
-#pragma unroll
-				for (int k = 0; k < 5; k++) {
-					const T up = shfl_up_t(y, 1 << k);
-					if (lane >= (1 << k)) y = fma_t(cv.v[MO + k], up, y);
-				}
-				ring[(h.z + ctid) & (SW_RING - 1)] = y;
-				if (odef >= 0) out[odef] = ydef;          // an earlier sub-block of this level
-				ydef = y;
-				odef = ci.i[W];
+				y = fmsub<T, FMA>(y, d[k], cur.v[k]);
 			}
 			if (fail) break;
-			__syncwarp();
-			if (lane == 0) st_release_cta(&prog[warp], ll);
-			if (odef >= 0) { out[odef] = ydef; odef = -1; }
 		}
-		consumer_sync<CW>();
-		if (*vfailed && ctid == 0) sweep_drain(a, full, D, waited, issued, pdone);
+		if (UPPER) y = mul(y, cur.v[W]);
+		if (CS) {
+			// the segments' recurrences across the warp's lanes
+#pragma unroll
+			for (int k = 0; k < 5; k++) {
+				const T up = shfl_up_t(y, 1 << k);
+				if (lane >= (1 << k)) y = fma_t(cur.v[W + (UPPER ? 1 : 0) + k], up, y);
+			}
+		}
+		if (on) y = ring_value(y);
+		const unsigned pos = (unsigned)(32 * c + lane), next = pos + 32u * (unsigned)(a.look + 1);
+		if (on) ring_st(rb + (pos & mask) * (unsigned)sizeof(T), y);
+		ring_st(rb + (next & mask) * (unsigned)sizeof(T), ring_mark<T>());
+		__syncwarp();
+		if (lane == 0) st_release_cta(&prog[warp], c + nw);
+		if (on && cur.i[W] >= 0) out[cur.i[W]] = y;
 	}
+	if (fail) {
+		// record the timeout, wait (bounded) for this warp's copies in flight
+		*vfailed = 1;
+		if (lane == 0) {
+			fg_set_err(a.err, FEMGPU_E_TIMEOUT);
+			for (int q = waited; q < issued; q++) (void)mbar_wait(&full[q % D], (unsigned)((q / D) & 1));
+		}
+	}
+	__syncwarp();
+	if (lane == 0) st_release_cta(&prog[warp], DF_DONE);  // its last outputs are stored
 	__syncthreads();
 	return *vfailed != 0;
 }
 
-template <typename T, bool UPPER, int W>
-__global__ void __launch_bounds__((SW2_CW + 1) * 32, 1)
-k_sweep_cs(SweepArgs a, const T *__restrict__ in, T *out)
+#define DF_SMEM(ring) (sm + (unsigned)al16(((ring) + 1) * sizeof(T)))
+template <typename T, bool UPPER, bool FMA, bool CS, int W>
+__global__ void __launch_bounds__(df_warps(CS, W) * 32, 1)
+k_sweep_df(SweepArgs a, const T *__restrict__ in, T *out)
 {
 	if (a.active && !*a.active) return;
 	extern __shared__ __align__(128) unsigned char sm[];
-	const unsigned ring_b = (unsigned)al16((SW_RING + 1) * sizeof(T));
-	unsigned long long *full = (unsigned long long *)(sm + ring_b);
-	__shared__ int failed, issued, pdone;
-	__shared__ int prog[SW2_CW];
-	(void)cs_sweep<T, UPPER, W>(a, in, out, sm, full, full + SW_MAXD, &failed, &issued, &pdone, prog);
+	__shared__ int failed, prog[DF_WARPS];
+	(void)sweep_run<T, UPPER, FMA, CS, W>(a, in, out, sm, (unsigned long long *)DF_SMEM(a.ring), &failed, prog);
 }
 
 // Both sweeps of one preconditioner application in one launch: each thread
 // block sweeps its matrix block forward (in -> y) and then backward (y ->
-// out), keeping its SM between the two (block ILU(0): a block's backward
-// sweep reads only its own forward results).  The consumers' global stores
-// of y are ordered before the producer's bulk copies of y by an async-proxy
-// fence and the block barrier; the backward sweep runs on barriers of its
-// own.  Dynamic shared memory: the larger of the two sweeps' layouts.
-template <typename T, int WL, int WU>
-__global__ void __launch_bounds__((SW2_CW + 1) * 32, 1)
-k_sweep_cs_fb(SweepArgs al, SweepArgs au, const T *__restrict__ in, T *y, T *out)
+// out), keeping its SM between the two (a block's backward sweep reads only
+// its own forward results).  The forward sweep's global stores of y are
+// ordered before the bulk copies of y by an async-proxy fence and the block
+// barrier; the backward sweep runs on barriers of its own.  Dynamic shared
+// memory: the larger of the two sweeps' layouts.
+template <typename T, bool FMA, bool CS, int W>
+__global__ void __launch_bounds__(df_warps(CS, W) * 32, 1)
+k_sweep_fb(SweepArgs al, SweepArgs au, const T *__restrict__ in, T *y, T *out)
 {
 	if (al.active && !*al.active) return;
 	extern __shared__ __align__(128) unsigned char sm[];
-	const unsigned ring_b = (unsigned)al16((SW_RING + 1) * sizeof(T));
-	unsigned long long *full = (unsigned long long *)(sm + ring_b);
-	__shared__ unsigned long long bar2[2 * SW_MAXD];
-	__shared__ int failed, issued, pdone;
-	__shared__ int prog[SW2_CW];
-	if (cs_sweep<T, false, WL>(al, in, y, sm, full, full + SW_MAXD, &failed, &issued, &pdone, prog)) return;
+	__shared__ int failed, prog[DF_WARPS];
+	if (sweep_run<T, false, FMA, CS, W>(al, in, y, sm, (unsigned long long *)DF_SMEM(al.ring), &failed, prog)) return;
 	asm volatile("fence.proxy.async.global;" ::: "memory");
 	__syncthreads();
-	(void)cs_sweep<T, true, WU>(au, y, out, sm, bar2, bar2 + SW_MAXD, &failed, &issued, &pdone, prog);
+	(void)sweep_run<T, true, FMA, CS, W>(au, y, out, sm, (unsigned long long *)DF_SMEM(au.ring) + DF_BARS, &failed, prog);
 }
 
 // Scan multipliers of a chain-scan program from the factor, one warp per
@@ -783,7 +829,7 @@ k_sweep_cs_fb(SweepArgs al, SweepArgs au, const T *__restrict__ in, T *y, T *out
 // (0 at a segment start and in padding); M_0 = b and, as the scan composes
 // the recurrences, M_{k+1,t} = M_k,t M_k,t-2^k for t >= 2^k (else M_k,t).
 template <typename T, bool UPPER>
-__global__ void k_chain_mult(unsigned char *prog, const long long *voff, const int *src, const int *row, int nslot,
+__global__ void k_chain_mult(unsigned char *prog, const long long *voff, const int *src, const int *row, int nslot, int mo,
                              const double *LU, const double *Dinv)
 {
 	const int lane = threadIdx.x & 31;
@@ -803,9 +849,10 @@ __global__ void k_chain_mult(unsigned char *prog, const long long *voff, const i
 		}
 		const long long o = i < nslot ? voff[i] : -1;
 		if (o >= 0) {
-			T *dst = (T *)(prog + o);
+			constexpr int PER = 16 / (int)sizeof(T);     // value v of a slot: word v / PER of its lane
 #pragma unroll
-			for (int k = 0; k < 5; k++) dst[k] = from_d<T>(M[k]);
+			for (int k = 0; k < 5; k++)
+				((T *)(prog + o + (mo + k) / PER * 512))[(mo + k) % PER] = from_d<T>(M[k]);
 		}
 	}
 }
@@ -1152,8 +1199,7 @@ static int sweep_near_limit(void)
 }
 
 // Record-layout sweeps run as dataflow (k_sweep_df) unless
-// FEMGPU_SWEEP_SYNC=barrier asks for one barrier per level (k_sweep_rec).  At
-// 2048x1024 with 16 blocks: 1.36 ms per FP64 application against 1.47.
+// FEMGPU_SWEEP_SYNC=barrier asks for one barrier per level (k_sweep_rec).
 static bool sweep_dataflow(void)
 {
 	const char *e = getenv("FEMGPU_SWEEP_SYNC");
@@ -1176,13 +1222,41 @@ static bool sweep_ds(void)
 	return !(e && !strcmp(e, "0"));
 }
 
-// Levels a dataflow warp may run ahead of the slowest one (FEMGPU_SWEEP_SKEW,
-// 1..64; default 4).
-static int sweep_skew(void)
+// Chunks a dataflow warp may run ahead of the slowest one: 8 times
+// FEMGPU_SWEEP_SKEW (1..64; default 4, two turns of 16 warps).
+static int sweep_look(void)
 {
 	const char *e = getenv("FEMGPU_SWEEP_SKEW");
 	int v = e ? atoi(e) : 4;
-	return (v >= 1 && v <= 64) ? v : 4;
+	return 8 * ((v >= 1 && v <= 64) ? v : 4);
+}
+
+// Layout of a dataflow program whose chunks take `stage' bytes: warps (at most
+// `most', fewer until two stages of each fit), stages a warp, ring (the wide one
+// if it fits with all of `most'), lookahead X and the ring's reach in chunks.
+// False when nothing fits.
+struct DfFit { int ring, look, reach, warps, D; };
+static bool df_stages(int ring, long long stage, long long tsize, int warps, int *D)
+{
+	const long long fixed = (al16(((long long)ring + 1) * tsize) + 2 * DF_BARS * 8 + 127) & ~127LL;
+	*D = (int)std::min<long long>((SW_SMEM_CAP - fixed) / (warps * al16(stage)), std::min(DF_MAXD, DF_BARS / warps));
+	return *D >= 2;
+}
+static bool df_fit(int most, long long stage, long long tsize, DfFit &f)
+{
+	f.ring = SW_RING_WIDE;
+	f.warps = most;
+	if (!df_stages(f.ring, stage, tsize, f.warps, &f.D)) {
+		f.ring = SW_RING;
+		while (f.warps >= 4 && !df_stages(f.ring, stage, tsize, f.warps, &f.D)) f.warps -= 4;
+		if (f.warps < 4) return false;
+	}
+	const int R = f.ring / 32;
+	f.look = std::min(sweep_look() * (f.ring / SW_RING), (R - 2 - f.warps) / 3);
+	// a lowered reach (FEMGPU_SWEEP_NEAR): a dependency read back from global
+	// memory must be more than a turn of all warps back
+	f.reach = std::min(R - 2 * f.look - 2, std::max((sweep_near_limit() + 31) / 32, f.warps + 1));
+	return true;
 }
 
 // One sweep program.  Forward (lower): L part, outputs to the backward
@@ -1200,10 +1274,25 @@ static int build_prog(const int *IA, const int *JA, int n, const HostLevels &H, 
 	struct Sub { int l, j0, c, w; };
 	std::vector<Sub> subs;
 	subs.reserve(nlev + 16);
+	int wmax = 0, lmax = 1;
+	for (int r = 0; r < n; r++) {
+		int cnt = 0;
+		for (int k = IA[r]; k < IA[r + 1]; k++)
+			if ((lower ? JA[k] < r : JA[k] > r) && B.same(r, JA[k])) cnt++;
+		wmax = std::max(wmax, cnt);
+	}
+	for (int l = 0; l < nlev; l++) lmax = std::max(lmax, H.start[l + 1] - H.start[l]);
+	int rw = rec_width(wmax);                                         // 0: ELL sub-blocks
+	const long long RB0 = rw ? rec_bytes(rw, UPPER, (int)tsize) : 0;
+	DfFit fit = { SW_RING, 0, 0, 0, 0 };
+	const int widest = std::min(lmax, 32);
+	const bool df = rw && sweep_dataflow() && 
+	                df_fit(df_warps(false, rw), DF_HDR + widest * RB0 + al16((long long)((widest + 3) & ~3) * tsize), tsize, fit);
+	const int sub = df ? 32 : SW_SUB;
 	for (int l = 0; l < nlev; l++) {
 		int c = H.start[l + 1] - H.start[l];
-		for (int j0 = 0; j0 < c; j0 += SW_SUB) {
-			int cc = std::min(SW_SUB, c - j0), w = 0;
+		for (int j0 = 0; j0 < c; j0 += sub) {
+			int cc = std::min(sub, c - j0), w = 0;
 			for (int p = H.start[l] + j0; p < H.start[l] + j0 + cc; p++) {
 				int r = H.rows[p], cnt = 0;
 				for (int k = IA[r]; k < IA[r + 1]; k++)
@@ -1214,28 +1303,30 @@ static int build_prog(const int *IA, const int *JA, int n, const HostLevels &H, 
 		}
 	}
 	int nsb = (int)subs.size();
-	int wmax = 0, cmax = 1, lmax = 1;
-	for (const Sub &S : subs) { wmax = std::max(wmax, S.w); cmax = std::max(cmax, S.c); }
-	for (int l = 0; l < nlev; l++) lmax = std::max(lmax, H.start[l + 1] - H.start[l]);
-	int rw = rec_width(wmax);                                         // 0: ELL sub-blocks
-	if (rw) {
+	int cmax = 1;
+	for (const Sub &S : subs) cmax = std::max(cmax, S.c);
+	if (rw && !df) {
 		// wide records must still leave room for two stages of the widest sub-block
 		const long long fixed = (al16((SW_RING + 1) * tsize) + SW_BAR_BYTES + 127) & ~127LL;
-		const long long stage = DF_HDR + (long long)cmax * rec_bytes(rw, UPPER, (int)tsize) +
-		                        al16((long long)((cmax + 3) & ~3) * tsize);
+		const long long stage = 16 + (long long)cmax * RB0 + al16((long long)((cmax + 3) & ~3) * tsize);
 		if (fixed + 2 * ((stage + 127) & ~127LL) > SW_SMEM_CAP) rw = 0;
 	}
-	const long long RB = rw ? rec_bytes(rw, UPPER, (int)tsize) : 0;
-	// dataflow: the ring holds only what no warp up to the skew behind can still overwrite
-	const int skew = sweep_skew();
-	bool df = rw && sweep_dataflow() && SW_RING - skew * lmax >= 2 * lmax;
-	if (df) near_lim = std::min(near_lim, SW_RING - skew * lmax);
-	if (df && near_lim < 2 * lmax) df = false;      // a far dependency must be two levels back
-	const long long hdrb = df ? DF_HDR : 16;
-	std::vector<int> lev_of(df ? n : 0);
-	if (df)
-		for (int l = 0; l < nlev; l++)
-			for (int q = H.start[l]; q < H.start[l + 1]; q++) lev_of[q] = l;
+	const long long RB = rw ? RB0 : 0;
+	const long long hdrb = 16;
+	// dataflow: chunk of each level-order position, counted from its matrix block's first
+	std::vector<int> chunk(df ? n : 0), lane(df ? n : 0), cfirst(df ? nsb : 0);
+	if (df) {
+		size_t b = 0;
+		int first = 0;
+		for (int i = 0; i < nsb; i++) {
+			while (b + 1 < clev.size() && subs[i].l >= clev[b + 1]) { b++; first = i; }
+			cfirst[i] = i - first;
+			for (int j = 0; j < subs[i].c; j++) {
+				chunk[H.start[subs[i].l] + subs[i].j0 + j] = i - first;
+				lane[H.start[subs[i].l] + subs[i].j0 + j] = j;
+			}
+		}
+	}
 	std::vector<long long> off(nsb + 1, 0);
 	std::vector<int> sb_in(nsb), sb_inb(nsb);
 	long long maxblk = 0, bvo = 0, maxin = 0;
@@ -1259,49 +1350,38 @@ static int build_prog(const int *IA, const int *JA, int n, const HostLevels &H, 
 		const Sub &S = subs[i];
 		int l = S.l, c = S.c, w = S.w, cp = (c + 3) & ~3, start = H.start[l] + S.j0;
 		int end = H.start[l + 1];
-		int nsub = (H.start[l + 1] - H.start[l] + SW_SUB - 1) / SW_SUB;
+		int nsub = (H.start[l + 1] - H.start[l] + sub - 1) / sub;
 		unsigned char *b = prog.data() + off[i];
 		int hasfar = 0;
+		auto near = [&](int p) { return df ? cfirst[i] - chunk[p] <= fit.reach : end - p <= near_lim; };
+		auto ring_slot = [&](int p) {
+			return (unsigned)(df ? (32 * chunk[p] + lane[p]) & (fit.ring - 1) : p & (SW_RING - 1));
+		};
+		// dataflow: the ring slot's byte offset, or the global position and the top bit
+		auto code = [&](bool ring, unsigned at) {
+			return (int)(df ? (ring ? at * (unsigned)tsize : SW_NEAR | at) : (ring ? SW_NEAR | at : at));
+		};
 		for (int j = 0; j < c; j++) {
 			int r = H.rows[start + j];
 			for (int q = IA[r]; q < IA[r + 1]; q++) {
 				int col = JA[q];
-				if ((lower ? col < r : col > r) && B.same(r, col) && end - H.pos[col] > near_lim) hasfar = 1;
+				if ((lower ? col < r : col > r) && B.same(r, col) && !near(H.pos[col]))
+					hasfar = df ? std::max(hasfar, chunk[H.pos[col]] + 1) : 1;
 			}
 		}
 		if (rw) {
-			const int hh[4] = { c, nsub, start, hasfar };
+			const int hh[4] = { c, df ? 0 : nsub, df ? 0 : start, hasfar };
 			memcpy(b, hh, sizeof hh);
-			if (df) {
-				// need[w][pw]: smallest level distance of a dependency of warp w's rows
-				// produced by warp pw (255: none within skew + 1 levels)
-				unsigned char *need = b + 16;
-				memset(need, 255, (size_t)SW2_CW * NEED_STRIDE);
-				for (int j = 0; j < c; j++) {
-					int r = H.rows[start + j];
-					for (int q = IA[r]; q < IA[r + 1]; q++) {
-						int col = JA[q];
-						if ((lower ? !(col < r) : !(col > r)) || !B.same(r, col)) continue;
-						int p = H.pos[col], lp = lev_of[p], dl = l - lp;
-						if (end - p > near_lim) dl--;      // read back from global memory: the next level's release
-						if (dl > skew + 1) continue;
-						int pw = ((p - H.start[lp]) % SW_SUB) / 32;
-						unsigned char &e = need[(j / 32) * NEED_STRIDE + pw];
-						if (dl < (int)e) e = (unsigned char)dl;
-					}
-				}
-			}
 			for (int j = 0; j < c; j++) {
 				int *ri = (int *)(b + hdrb + (size_t)j * RB), r = H.rows[start + j], k = 0;
 				long long vo = off[i] + hdrb + (long long)j * RB + rec_ib(rw);
-				for (int q = 0; q < rw; q++) ri[q] = (int)(SW_NEAR | SW_RING);   // the zero slot
+				for (int q = 0; q < rw; q++) ri[q] = code(true, (unsigned)fit.ring);   // the zero slot
 				ri[rw] = lower ? target->ppos[r] : r;
 				for (int q = IA[r]; q < IA[r + 1]; q++) {
 					int col = JA[q];
 					if ((lower ? !(col < r) : !(col > r)) || !B.same(r, col)) continue;
 					int p = H.pos[col];
-					ri[k] = (int)((end - p <= near_lim) ? (SW_NEAR | (unsigned)(p & (SW_RING - 1)))
-					                                   : (unsigned)(lower ? target->ppos[col] : col));
+					ri[k] = near(p) ? code(true, ring_slot(p)) : code(false, (unsigned)(lower ? target->ppos[col] : col));
 					val_off.push_back(vo + k * tsize);
 					val_src.push_back(q);
 					k++;
@@ -1350,7 +1430,9 @@ static int build_prog(const int *IA, const int *JA, int n, const HostLevels &H, 
 	sw.nchunk = (int)clev.size() - 1;
 	sw.rw = rw;
 	sw.df = df;
-	sw.skew = skew;
+	sw.ring = fit.ring;
+	sw.look = fit.look;
+	sw.warps = fit.warps;
 	sw.bvo = (int)bvo;
 	sw.cmax = cmax;
 	sw.nlev = nlev;
@@ -1378,7 +1460,7 @@ static int build_prog(const int *IA, const int *JA, int n, const HostLevels &H, 
 }
 
 // ------------------------------------------- host: chain-scan programs
-// Segments of one sweep (the order of k_sweep_cs): rows in sweep order
+// Segments of one chain-scan sweep: rows in sweep order
 // (forward ascending, backward descending) within their matrix block; a row
 // joins the current segment when it depends on its sweep predecessor, the
 // segment has fewer than 32 rows and the row's other dependencies are all on
@@ -1480,12 +1562,12 @@ static ChainLevels host_chain_levels(const int *IA, const int *JA, int n, bool l
 	return H;
 }
 
-// The chain-scan program of one sweep (k_sweep_cs): sub-blocks of up to
-// SW_SUB slots of one level, the k_sweep_df header and need tables, one record
-// per slot, the input slice at a fixed stage offset.  Forward: L part, outputs
-// to the backward program's slots; backward: U part and pivots, outputs in
-// natural order.  Returns FEMGPU_E_MESH when the ring cannot hold the widest
-// level (the caller keeps the row-by-row programs then).
+// The chain-scan program of one sweep: chunks of 32 slots of one level, the
+// dataflow header, one record per slot (the lanes' 16-byte words side by side),
+// the input slice at a fixed stage offset.  Forward: L part, outputs to the
+// backward program's slots; backward: U part and pivots, outputs in natural
+// order.  Returns FEMGPU_E_MESH when its stages do not fit (the caller keeps
+// the row-by-row programs then).
 template <typename T, bool UPPER>
 static int build_prog_chain(const int *IA, const int *JA, int n, const ChainLevels &H, const ChainLevels *target,
                             const Blocks &B, fg_sweep &sw)
@@ -1495,30 +1577,28 @@ static int build_prog_chain(const int *IA, const int *JA, int n, const ChainLeve
 	const int nlev = H.nlev;
 	int rw = rec_width(std::max(H.maxw, 1));
 	if (!rw) return FEMGPU_E_MESH;
-	const long long RB = rec_bytes_cs(rw, UPPER, (int)tsize), IBy = rec_ib(rw);
-	int lmax = 32;
-	for (int l = 0; l < nlev; l++) lmax = std::max(lmax, H.lstart[l + 1] - H.lstart[l]);
-	int skew = std::min(sweep_skew(), 4);
-	while (skew > 1 && SW_RING - skew * lmax < 2 * lmax) skew--;
-	if (SW_RING - skew * lmax < 2 * lmax) return FEMGPU_E_MESH;
-	// a dependency read back from global memory must be two levels back: a
-	// lowered reach (FEMGPU_SWEEP_NEAR) stops at two of the widest levels
-	const int near_lim = std::max(std::min(sweep_near_limit(), SW_RING - skew * lmax), 2 * lmax);
+	const long long IBy = rec_ib(rw), RB = IBy + rec_vb_cs(rw, UPPER, (int)tsize);
+	// int q and value v of a chunk's slot j, from the chunk's start
+	auto iat = [](int q, int j) { return (long long)DF_HDR + q / 4 * 512 + 16 * j + q % 4 * 4; };
+	auto vat = [&](int v, int j) {
+		const int per = 16 / (int)tsize;
+		return DF_HDR + 32 * IBy + v / per * 512 + 16 * j + v % per * tsize;
+	};
 	struct Sub { int l, j0, c; };
 	std::vector<Sub> subs;
 	for (int l = 0; l < nlev; l++) {
 		const int c = H.lstart[l + 1] - H.lstart[l];
-		for (int j0 = 0; j0 < c; j0 += SW_SUB) subs.push_back({ l, j0, std::min(SW_SUB, c - j0) });
+		for (int j0 = 0; j0 < c; j0 += 32) subs.push_back({ l, j0, 32 });
 	}
 	const int nsb = (int)subs.size();
-	int cmax = 32;
-	for (const Sub &S : subs) cmax = std::max(cmax, S.c);
-	const long long fixed = (al16((SW_RING + 1) * tsize) + SW_BAR_BYTES + 127) & ~127LL;
-	const long long stage = DF_HDR + (long long)cmax * RB + al16((long long)cmax * tsize);
-	if (fixed + 2 * ((stage + 127) & ~127LL) > SW_SMEM_CAP) return FEMGPU_E_MESH;
-	std::vector<int> lev_of(H.nslot);
-	for (int l = 0; l < nlev; l++)
-		for (int q = H.lstart[l]; q < H.lstart[l + 1]; q++) lev_of[q] = l;
+	const int cmax = 32;
+	DfFit fit;
+	if (!df_fit(df_warps(true, rw), DF_HDR + cmax * RB + cmax * tsize, tsize, fit)) return FEMGPU_E_MESH;
+	std::vector<int> cfirst(nsb);                        // chunks before each chunk in its matrix block
+	for (size_t i = 0, bk = 0, first = 0; i < (size_t)nsb; i++) {
+		while (bk + 1 < H.clev.size() && subs[i].l >= H.clev[bk + 1]) { bk++; first = i; }
+		cfirst[i] = (int)(i - first);
+	}
 	std::vector<long long> off(nsb + 1, 0);
 	std::vector<int> sb_in(nsb), sb_inb(nsb);
 	long long bvo = 0, maxin = 0;
@@ -1537,8 +1617,7 @@ static int build_prog_chain(const int *IA, const int *JA, int n, const ChainLeve
 	val_src.reserve((size_t)H.nslot * (rw + 1));
 	for (int i = 0; i < nsb; i++) {
 		const Sub &S = subs[i];
-		const int l = S.l, c = S.c, start = H.lstart[l] + S.j0, end = H.lstart[l + 1];
-		const int nsub = (end - H.lstart[l] + SW_SUB - 1) / SW_SUB;
+		const int l = S.l, c = S.c, start = H.lstart[l] + S.j0;
 		unsigned char *b = prog.data() + off[i];
 		int hasfar = 0;
 		for (int j = 0; j < c; j++) {
@@ -1547,51 +1626,39 @@ static int build_prog_chain(const int *IA, const int *JA, int n, const ChainLeve
 			for (int q = IA[r]; q < IA[r + 1]; q++) {
 				const int col = JA[q];
 				if ((lower ? col < r : col > r) && B.same(r, col) && q != H.slot_pred[start + j] &&
-				    end - H.slot[col] > near_lim) hasfar = 1;
+				    i - H.slot[col] / 32 > fit.reach) hasfar = std::max(hasfar, cfirst[H.slot[col] / 32] + 1);
 			}
 		}
-		const int hh[4] = { c, nsub, start, hasfar };
+		const int hh[4] = { c, 0, 0, hasfar };
 		memcpy(b, hh, sizeof hh);
-		unsigned char *need = b + 16;
-		memset(need, 255, (size_t)SW2_CW * NEED_STRIDE);
 		for (int j = 0; j < c; j++) {
 			const int r = H.slot_row[start + j];
-			int *ri = (int *)(b + DF_HDR + (size_t)j * RB), k = 0;
-			const long long vo = off[i] + DF_HDR + (long long)j * RB + IBy;
-			for (int q = 0; q < rw; q++) ri[q] = (int)(SW_NEAR | SW_RING);     // the zero slot
-			if (r < 0) {                                                       // padding
-				ri[rw] = -1;
-				for (int q = 0; q < rw + (UPPER ? 1 : 0); q++) { val_off.push_back(vo + q * tsize); val_src.push_back(-1); }
+			int k = 0;
+			auto ri = [&](int q) -> int & { return *(int *)(b + iat(q, j)); };
+			cs_voff[start + j] = off[i] + vat(0, j);
+			for (int q = 0; q < rw; q++) ri(q) = fit.ring * (int)tsize;        // the zero slot
+			if (r < 0) {                                                       // padding (multipliers zero)
+				ri(rw) = -1;
+				for (int q = 0; q < rw + (UPPER ? 1 : 0); q++) { val_off.push_back(off[i] + vat(q, j)); val_src.push_back(-1); }
 				continue;
 			}
-			ri[rw] = lower ? target->slot[r] : r;
+			ri(rw) = lower ? target->slot[r] : r;
 			for (int q = IA[r]; q < IA[r + 1]; q++) {
 				const int col = JA[q];
 				if ((lower ? !(col < r) : !(col > r)) || !B.same(r, col) || q == H.slot_pred[start + j]) continue;
-				const int p = H.slot[col], lp = lev_of[p];
-				int dl = l - lp;
-				const bool nearp = end - p <= near_lim;
-				ri[k] = (int)(nearp ? (SW_NEAR | (unsigned)(p & (SW_RING - 1))) : (unsigned)(lower ? target->slot[col] : col));
-				if (!nearp) dl--;                     // read back from global memory: the next level's release
-				if (dl <= skew + 1) {
-					const int pw = ((p - H.lstart[lp]) % SW_SUB) / 32;
-					unsigned char &e = need[(j / 32) * NEED_STRIDE + pw];
-					if (dl < (int)e) e = (unsigned char)dl;
-				}
-				val_off.push_back(vo + k * tsize);
+				const int p = H.slot[col];
+				ri(k) = (int)(i - p / 32 <= fit.reach
+				                  ? (unsigned)((32 * cfirst[p / 32] + p % 32) & (fit.ring - 1)) * (unsigned)tsize
+				                  : SW_NEAR | (unsigned)(lower ? target->slot[col] : col));
+				val_off.push_back(off[i] + vat(k, j));
 				val_src.push_back(q);
 				k++;
 			}
-			for (; k < rw; k++) { val_off.push_back(vo + k * tsize); val_src.push_back(-1); }
-			if (!lower) { val_off.push_back(vo + rw * tsize); val_src.push_back(-2 - r); }
-			cs_voff[start + j] = vo + (rw + (UPPER ? 1 : 0)) * tsize;
+			for (; k < rw; k++) { val_off.push_back(off[i] + vat(k, j)); val_src.push_back(-1); }
+			if (!lower) { val_off.push_back(off[i] + vat(rw, j)); val_src.push_back(-2 - r); }
 			cs_src[start + j] = H.slot_pred[start + j];
 			cs_row[start + j] = r;
 		}
-		// padding slots: multipliers zero (the refresh writes them too)
-		for (int j = 0; j < c; j++)
-			if (H.slot_row[start + j] < 0) cs_voff[start + j] = off[i] + DF_HDR + (long long)j * RB + IBy +
-			                                                    (rw + (UPPER ? 1 : 0)) * tsize;
 	}
 	// every index the kernel will follow stays inside its array: dependency
 	// codes (ring slots or output positions), output positions, input slices
@@ -1600,19 +1667,19 @@ static int build_prog_chain(const int *IA, const int *JA, int n, const ChainLeve
 		for (int i = 0; i < nsb; i++) {
 			const unsigned char *b = prog.data() + off[i];
 			const int c = subs[i].c;
-			if (sb_in[i] < 0 || (long long)sb_in[i] + c > H.nslot) return FEMGPU_E_MESH;
+			if (sb_in[i] != 32 * i || c != 32 || (long long)sb_in[i] + c > H.nslot) return FEMGPU_E_MESH;
 			for (int j = 0; j < c; j++) {
-				const int *ri = (const int *)(b + DF_HDR + (size_t)j * RB);
+				auto ri = [&](int q) { return *(const int *)(b + iat(q, j)); };
 				for (int q = 0; q < rw; q++) {
-					const unsigned code = (unsigned)ri[q];
-					if (code & SW_NEAR) { if ((code & ~SW_NEAR) > SW_RING) return FEMGPU_E_MESH; }
-					else if ((long long)code >= nout) return FEMGPU_E_MESH;
+					const unsigned code = (unsigned)ri(q);
+					if (code & SW_NEAR) { if ((long long)(code & ~SW_NEAR) >= nout) return FEMGPU_E_MESH; }
+					else if (code > (unsigned)(fit.ring * tsize)) return FEMGPU_E_MESH;
 				}
-				if (ri[rw] < -1 || ri[rw] >= nout) return FEMGPU_E_MESH;
+				if (ri(rw) < -1 || ri(rw) >= nout) return FEMGPU_E_MESH;
 			}
 		}
 		for (size_t q = 0; q < cs_voff.size(); q++)
-			if (cs_voff[q] < 0 || cs_voff[q] + 5 * tsize > off[nsb]) return FEMGPU_E_MESH;
+			if (cs_voff[q] < 0 || cs_voff[q] - vat(0, 0) + vat(rw + (UPPER ? 1 : 0) + 4, 0) + tsize > off[nsb]) return FEMGPU_E_MESH;
 		for (size_t q = 0; q < val_off.size(); q++)
 			if (val_off[q] < 0 || val_off[q] + tsize > off[nsb]) return FEMGPU_E_MESH;
 	}
@@ -1632,7 +1699,9 @@ static int build_prog_chain(const int *IA, const int *JA, int n, const ChainLeve
 	sw.rw = rw;
 	sw.df = 1;
 	sw.cs = 1;
-	sw.skew = skew;
+	sw.ring = fit.ring;
+	sw.look = fit.look;
+	sw.warps = fit.warps;
 	sw.bvo = (int)bvo;
 	sw.cmax = cmax;
 	sw.nlev = nlev;
@@ -1732,27 +1801,18 @@ static int build_factor_prog(const int *IA, const int *JA, int n, const HostLeve
 	SW_SET(float, false, CW, false); SW_SET(float, true, CW, false)
 #define SR_SET(T, U, F, W) FG_TRY(cudaFuncSetAttribute(k_sweep_rec<T, U, F, W>, \
 	cudaFuncAttributeMaxDynamicSharedMemorySize, SW_SMEM_CAP))
-#define SD_SET(T, U, F, W) FG_TRY(cudaFuncSetAttribute(k_sweep_df<T, U, F, W>, \
+#define SD_SET(T, U, F, C, W) FG_TRY(cudaFuncSetAttribute(k_sweep_df<T, U, F, C, W>, \
 	cudaFuncAttributeMaxDynamicSharedMemorySize, SW_SMEM_CAP))
-#define SC_SET(T, U, W) FG_TRY(cudaFuncSetAttribute(k_sweep_cs<T, U, W>, \
+#define SF_SET(T, F, C, W) FG_TRY(cudaFuncSetAttribute(k_sweep_fb<T, F, C, W>, \
 	cudaFuncAttributeMaxDynamicSharedMemorySize, SW_SMEM_CAP))
-#define SR_SET_W(W) SC_SET(double, false, W); SC_SET(double, true, W); SC_SET(float, false, W); \
-	SC_SET(float, true, W); SC_SET(dsf, false, W); SC_SET(dsf, true, W); \
+#define SD_BOTH(T, F, C, W) SD_SET(T, false, F, C, W); SD_SET(T, true, F, C, W); SF_SET(T, F, C, W)
+#define SR_SET_W(W) SD_BOTH(double, true, true, W); SD_BOTH(float, true, true, W); SD_BOTH(dsf, true, true, W); \
+	SD_BOTH(double, false, false, W); SD_BOTH(double, true, false, W); SD_BOTH(float, false, false, W); \
 	SR_SET(double, false, false, W); SR_SET(double, true, false, W); \
 	SR_SET(double, false, true, W); SR_SET(double, true, true, W); \
-	SR_SET(float, false, false, W); SR_SET(float, true, false, W); \
-	SD_SET(double, false, false, W); SD_SET(double, true, false, W); \
-	SD_SET(double, false, true, W); SD_SET(double, true, true, W); \
-	SD_SET(float, false, false, W); SD_SET(float, true, false, W)
-#define SF_SET(W) FG_TRY(cudaFuncSetAttribute(k_sweep_cs_fb<dsf, W, W>, \
-	cudaFuncAttributeMaxDynamicSharedMemorySize, SW_SMEM_CAP))
+	SR_SET(float, false, false, W); SR_SET(float, true, false, W)
 static int sweep_attrs(void)
 {
-	SF_SET(2);
-	SF_SET(3);
-	SF_SET(4);
-	SF_SET(6);
-	SF_SET(8);
 	SW_SET_CW(4);
 	SW_SET_CW(8);
 	SW_SET_CW(16);
@@ -1780,51 +1840,22 @@ static int sweep_cw(void)
 
 // fma: fused multiply-subtract in the FP64 sweeps (the FGMRES solves); the
 // separately rounded form reproduces the reference bit for bit.
-template <typename T, bool UPPER, bool FMA>
-static void launch_df(const SweepArgs &a, int rw, int grid, int bytes, cudaStream_t s, const T *in, T *out)
+#define DF_CASES(RUN) switch (rw) { case 2: RUN(2); break; case 3: RUN(3); break; case 4: RUN(4); break; \
+	case 6: RUN(6); break; case 8: RUN(8); break; case 12: RUN(12); break; default: RUN(16); break; }
+template <typename T, bool UPPER, bool FMA, bool CS>
+static void launch_df(const SweepArgs &a, int rw, int grid, int warps, int bytes, cudaStream_t s, const T *in, T *out)
 {
-	const int nt = (SW2_CW + 1) * 32;
-	switch (rw) {
-	case 2: k_sweep_df<T, UPPER, FMA, 2><<<grid, nt, bytes, s>>>(a, in, out); break;
-	case 3: k_sweep_df<T, UPPER, FMA, 3><<<grid, nt, bytes, s>>>(a, in, out); break;
-	case 4: k_sweep_df<T, UPPER, FMA, 4><<<grid, nt, bytes, s>>>(a, in, out); break;
-	case 6: k_sweep_df<T, UPPER, FMA, 6><<<grid, nt, bytes, s>>>(a, in, out); break;
-	case 8: k_sweep_df<T, UPPER, FMA, 8><<<grid, nt, bytes, s>>>(a, in, out); break;
-	case 12: k_sweep_df<T, UPPER, FMA, 12><<<grid, nt, bytes, s>>>(a, in, out); break;
-	default: k_sweep_df<T, UPPER, FMA, 16><<<grid, nt, bytes, s>>>(a, in, out); break;
-	}
+#define RUN(W) k_sweep_df<T, UPPER, FMA, CS, W><<<grid, 32 * warps, bytes, s>>>(a, in, out)
+	DF_CASES(RUN)
+#undef RUN
 }
-
-template <typename T, bool UPPER>
-static void launch_cs(const SweepArgs &a, int rw, int grid, int bytes, cudaStream_t s, const T *in, T *out)
+template <typename T, bool FMA, bool CS>
+static void launch_fb(const SweepArgs &al, const SweepArgs &au, int rw, int grid, int warps, int bytes, cudaStream_t s,
+                      const T *in, T *y, T *out)
 {
-	const int nt = (SW2_CW + 1) * 32;
-	switch (rw) {
-	case 2: k_sweep_cs<T, UPPER, 2><<<grid, nt, bytes, s>>>(a, in, out); break;
-	case 3: k_sweep_cs<T, UPPER, 3><<<grid, nt, bytes, s>>>(a, in, out); break;
-	case 4: k_sweep_cs<T, UPPER, 4><<<grid, nt, bytes, s>>>(a, in, out); break;
-	case 6: k_sweep_cs<T, UPPER, 6><<<grid, nt, bytes, s>>>(a, in, out); break;
-	case 8: k_sweep_cs<T, UPPER, 8><<<grid, nt, bytes, s>>>(a, in, out); break;
-	case 12: k_sweep_cs<T, UPPER, 12><<<grid, nt, bytes, s>>>(a, in, out); break;
-	default: k_sweep_cs<T, UPPER, 16><<<grid, nt, bytes, s>>>(a, in, out); break;
-	}
-}
-
-// Both double-single sweeps in one launch (k_sweep_cs_fb) when the two
-// programs have the same record width (one of 2, 3, 4, 6, 8) and blocks;
-// false: the caller launches them one by one.
-static bool launch_cs_fb(const SweepArgs &al, const SweepArgs &au, int rw, int grid, int bytes, cudaStream_t s,
-                         const dsf *in, dsf *y, dsf *out)
-{
-	const int nt = (SW2_CW + 1) * 32;
-	switch (rw) {
-	case 2: k_sweep_cs_fb<dsf, 2, 2><<<grid, nt, bytes, s>>>(al, au, in, y, out); return true;
-	case 3: k_sweep_cs_fb<dsf, 3, 3><<<grid, nt, bytes, s>>>(al, au, in, y, out); return true;
-	case 4: k_sweep_cs_fb<dsf, 4, 4><<<grid, nt, bytes, s>>>(al, au, in, y, out); return true;
-	case 6: k_sweep_cs_fb<dsf, 6, 6><<<grid, nt, bytes, s>>>(al, au, in, y, out); return true;
-	case 8: k_sweep_cs_fb<dsf, 8, 8><<<grid, nt, bytes, s>>>(al, au, in, y, out); return true;
-	default: return false;
-	}
+#define RUN(W) k_sweep_fb<T, FMA, CS, W><<<grid, 32 * warps, bytes, s>>>(al, au, in, y, out)
+	DF_CASES(RUN)
+#undef RUN
 }
 
 template <typename T, bool UPPER, bool FMA>
@@ -1843,18 +1874,8 @@ static void launch_rec(const SweepArgs &a, int rw, int grid, int bytes, cudaStre
 }
 
 template <typename T, bool UPPER>
-static void launch_sweep(const SweepArgs &a, int rw, int df, int grid, int bytes, cudaStream_t s, const T *in,
-                         T *out, bool fma, int cs = 0)
+static void launch_sweep(const SweepArgs &a, int rw, int grid, int bytes, cudaStream_t s, const T *in, T *out, bool fma)
 {
-	if (cs) {
-		launch_cs<T, UPPER>(a, rw, grid, bytes, s, in, out);
-		return;
-	}
-	if (rw && df) {
-		if (fma && sizeof(T) == 8) launch_df<T, UPPER, true>(a, rw, grid, bytes, s, in, out);
-		else launch_df<T, UPPER, false>(a, rw, grid, bytes, s, in, out);
-		return;
-	}
 	if (rw) {
 		if (fma && sizeof(T) == 8) launch_rec<T, UPPER, true>(a, rw, grid, bytes, s, in, out);
 		else launch_rec<T, UPPER, false>(a, rw, grid, bytes, s, in, out);
@@ -1872,8 +1893,14 @@ static void launch_sweep(const SweepArgs &a, int rw, int df, int grid, int bytes
 	}
 }
 
-static int sweep_smem(const fg_sweep &sw, size_t tsize, int *D, int *stage_bytes)
+static int sweep_smem(const fg_sweep &sw, size_t tsize, int *D, int *stage_bytes, int warps = 0)
 {
+	if (sw.df) {
+		const int w = warps ? warps : sw.warps;
+		*stage_bytes = (int)al16(sw.maxblk);
+		if (!df_stages(sw.ring, sw.maxblk, (long long)tsize, w, D)) return FEMGPU_E_MESH;
+		return (int)((al16((sw.ring + 1LL) * (long long)tsize) + 2 * DF_BARS * 8 + 127) & ~127LL) + w * *D * *stage_bytes;
+	}
 	size_t fixed = ((al16((SW_RING + 1) * tsize) + SW_BAR_BYTES + 127) & ~(size_t)127);
 	size_t sb = (size_t)((sw.maxblk + 127) & ~127LL);
 	if (fixed + 2 * sb > SW_SMEM_CAP) return FEMGPU_E_MESH;   // a sub-block too wide to stage
@@ -2055,10 +2082,10 @@ extern "C" int fg_ilu0_factor(femgpu_transport *t)
 		k_refresh<dsf><<<fg_grid(U.nval), FG_TPB, 0, s>>>(S.prog_up_ds, U.val_off, U.val_src, U.nval, t->ilu.LU,
 		                                                  t->ilu.Dinv);
 		k_chain_mult<dsf, false><<<fg_grid((long long)L.nslot), FG_TPB, 0, s>>>(S.prog_lo_ds, L.cs_voff, L.cs_src,
-		                                                                      L.cs_row, L.nslot, t->ilu.LU,
+		                                                                      L.cs_row, L.nslot, L.rw, t->ilu.LU,
 		                                                                      t->ilu.Dinv);
 		k_chain_mult<dsf, true><<<fg_grid((long long)U.nslot), FG_TPB, 0, s>>>(S.prog_up_ds, U.cs_voff, U.cs_src,
-		                                                                     U.cs_row, U.nslot, t->ilu.LU,
+		                                                                     U.cs_row, U.nslot, U.rw + 1, t->ilu.LU,
 		                                                                     t->ilu.Dinv);
 	}
 	return (int)cudaGetLastError();
@@ -2083,13 +2110,13 @@ static int refresh_pair(femgpu_transport *t, int i0)
 		if (i >= 4) {
 			const int gc = fg_grid((long long)c.nslot);
 			if (f64 && up) k_chain_mult<double, true><<<gc, FG_TPB, 0, s>>>(c.prog, c.cs_voff, c.cs_src, c.cs_row,
-			                                                               c.nslot, t->ilu.LU, t->ilu.Dinv);
+			                                                               c.nslot, c.rw + (up ? 1 : 0), t->ilu.LU, t->ilu.Dinv);
 			else if (f64) k_chain_mult<double, false><<<gc, FG_TPB, 0, s>>>(c.prog, c.cs_voff, c.cs_src, c.cs_row,
-			                                                               c.nslot, t->ilu.LU, t->ilu.Dinv);
+			                                                               c.nslot, c.rw + (up ? 1 : 0), t->ilu.LU, t->ilu.Dinv);
 			else if (up) k_chain_mult<float, true><<<gc, FG_TPB, 0, s>>>(c.prog, c.cs_voff, c.cs_src, c.cs_row,
-			                                                            c.nslot, t->ilu.LU, t->ilu.Dinv);
+			                                                            c.nslot, c.rw + (up ? 1 : 0), t->ilu.LU, t->ilu.Dinv);
 			else k_chain_mult<float, false><<<gc, FG_TPB, 0, s>>>(c.prog, c.cs_voff, c.cs_src, c.cs_row,
-			                                                     c.nslot, t->ilu.LU, t->ilu.Dinv);
+			                                                     c.nslot, c.rw + (up ? 1 : 0), t->ilu.LU, t->ilu.Dinv);
 		}
 		S.stale &= ~(1 << i);
 	}
@@ -2104,29 +2131,66 @@ static int sweep_wait(const femgpu_transport *t)
 	return t->sweep_wait1 > 0 ? t->sweep_wait1 - 1 : SW_WAIT_LIMIT;
 }
 
+static int sweep_args(const femgpu_transport *t, const fg_sweep &sw, const unsigned char *prog, size_t tsize,
+                      const int *active, int warps, SweepArgs &a)
+{
+	a.err = &t->st->err;
+	a.active = active;
+	a.wait = sweep_wait(t);
+	a.prog = prog; a.blk_off = sw.blk_off; a.sb_in = sw.sb_in; a.sb_inb = sw.sb_inb;
+	a.nlev = sw.nlev; a.nsb = sw.nsb;
+	a.chunk_sb = sw.chunk_sb; a.chunk_lev = sw.chunk_lev; a.bvo = sw.bvo; a.cmax = sw.cmax;
+	a.ring = sw.ring; a.look = sw.look;
+	return sweep_smem(sw, tsize, &a.D, &a.stage_bytes, warps);
+}
+
+// Both sweeps of a dataflow program pair, in one launch when the two have the
+// same record width and blocks (FEMGPU_SWEEP_FB=0: always two).
+template <typename T, bool FMA, bool CS>
+static int run_df(femgpu_transport *t, const fg_sweep &lo, const fg_sweep &up, const unsigned char *plo,
+                  const unsigned char *pup, const int *active, const T *in, T *y, T *out)
+{
+	SweepArgs a, b;
+	const char *e = getenv("FEMGPU_SWEEP_FB");
+	const bool fb = !(e && e[0] == '0') && lo.rw == up.rw && lo.nchunk == up.nchunk;
+	const int w = std::min(lo.warps, up.warps);
+	const int bl = sweep_args(t, lo, plo, sizeof(T), active, fb ? w : lo.warps, a);
+	if (bl < 0) return bl;
+	const int bu = sweep_args(t, up, pup, sizeof(T), active, fb ? w : up.warps, b);
+	if (bu < 0) return bu;
+	if (fb) launch_fb<T, FMA, CS>(a, b, lo.rw, lo.nchunk, w, std::max(bl, bu), t->stream, in, y, out);
+	else {
+		launch_df<T, false, FMA, CS>(a, lo.rw, lo.nchunk, lo.warps, bl, t->stream, in, y);
+		launch_df<T, true, FMA, CS>(b, up.rw, up.nchunk, up.warps, bu, t->stream, y, out);
+	}
+	return (int)cudaGetLastError();
+}
+
 template <typename T, typename TI, typename TO>
 static int apply_t(femgpu_transport *t, const fg_sweep &lo, const fg_sweep &up, T *bl, T *y,
                    const TI *p, TO *z, const int *active, bool fma)
 {
 	cudaStream_t s = t->stream;
-	int n = t->neq, D, sb, bytes;
+	const int n = t->neq;
 	k_perm_in<T, TI><<<fg_grid(n), FG_TPB, 0, s>>>(p, lo.rows, lo.ppos, n, bl);
+	if (lo.cs) return run_df<T, true, true>(t, lo, up, lo.prog, up.prog, active, bl, y, (T *)z);
+	fma = fma && sizeof(T) == 8;
+	if (lo.df && up.df)
+		return fma ? run_df<T, sizeof(T) == 8, false>(t, lo, up, lo.prog, up.prog, active, bl, y, (T *)z)
+		           : run_df<T, false, false>(t, lo, up, lo.prog, up.prog, active, bl, y, (T *)z);
 	SweepArgs a;
-	a.err = &t->st->err;
-	a.active = active;
-	a.wait = sweep_wait(t);
-	bytes = sweep_smem(lo, sizeof(T), &D, &sb);
+	int bytes = sweep_args(t, lo, lo.prog, sizeof(T), active, 0, a);
 	if (bytes < 0) return bytes;
-	a.prog = lo.prog; a.blk_off = lo.blk_off; a.sb_in = lo.sb_in; a.sb_inb = lo.sb_inb;
-	a.nlev = lo.nlev; a.nsb = lo.nsb; a.D = D; a.stage_bytes = sb;
-	a.chunk_sb = lo.chunk_sb; a.chunk_lev = lo.chunk_lev; a.bvo = lo.bvo; a.cmax = lo.cmax; a.skew = lo.skew;
-	launch_sweep<T, false>(a, lo.rw, lo.df, lo.nchunk, bytes, s, bl, y, fma, lo.cs);
-	bytes = sweep_smem(up, sizeof(T), &D, &sb);
+	if (lo.df) {
+		if (fma) launch_df<T, false, sizeof(T) == 8, false>(a, lo.rw, lo.nchunk, lo.warps, bytes, s, bl, y);
+		else launch_df<T, false, false, false>(a, lo.rw, lo.nchunk, lo.warps, bytes, s, bl, y);
+	} else launch_sweep<T, false>(a, lo.rw, lo.nchunk, bytes, s, bl, y, fma);
+	bytes = sweep_args(t, up, up.prog, sizeof(T), active, 0, a);
 	if (bytes < 0) return bytes;
-	a.prog = up.prog; a.blk_off = up.blk_off; a.sb_in = up.sb_in; a.sb_inb = up.sb_inb;
-	a.nlev = up.nlev; a.nsb = up.nsb; a.D = D; a.stage_bytes = sb;
-	a.chunk_sb = up.chunk_sb; a.chunk_lev = up.chunk_lev; a.bvo = up.bvo; a.cmax = up.cmax; a.skew = up.skew;
-	launch_sweep<T, true>(a, up.rw, up.df, up.nchunk, bytes, s, y, (T *)z, fma, up.cs);
+	if (up.df) {
+		if (fma) launch_df<T, true, sizeof(T) == 8, false>(a, up.rw, up.nchunk, up.warps, bytes, s, y, (T *)z);
+		else launch_df<T, true, false, false>(a, up.rw, up.nchunk, up.warps, bytes, s, y, (T *)z);
+	} else launch_sweep<T, true>(a, up.rw, up.nchunk, bytes, s, y, (T *)z, fma);
 	return (int)cudaGetLastError();
 }
 
@@ -2159,34 +2223,8 @@ static int apply_ds(femgpu_transport *t, const double *p, const dsf *p_ds, doubl
 static int sweeps_ds(femgpu_transport *t, const int *active)
 {
 	fg_ilu_sweeps &S = t->sweeps;
-	const fg_sweep &lo = S.lo64c, &up = S.up64c;
-	cudaStream_t s = t->stream;
-	int D, sb, bytes;
-	dsf *bl = (dsf *)S.bl64, *y = (dsf *)S.y64, *o = (dsf *)S.o64;
-	SweepArgs a;
-	a.err = &t->st->err;
-	a.active = active;
-	a.wait = sweep_wait(t);
-	bytes = sweep_smem(lo, sizeof(dsf), &D, &sb);
-	if (bytes < 0) return bytes;
-	a.prog = S.prog_lo_ds; a.blk_off = lo.blk_off; a.sb_in = lo.sb_in; a.sb_inb = lo.sb_inb;
-	a.nlev = lo.nlev; a.nsb = lo.nsb; a.D = D; a.stage_bytes = sb;
-	a.chunk_sb = lo.chunk_sb; a.chunk_lev = lo.chunk_lev; a.bvo = lo.bvo; a.cmax = lo.cmax; a.skew = lo.skew;
-	SweepArgs b = a;
-	const int bytes_lo = bytes;
-	bytes = sweep_smem(up, sizeof(dsf), &D, &sb);
-	if (bytes < 0) return bytes;
-	b.prog = S.prog_up_ds; b.blk_off = up.blk_off; b.sb_in = up.sb_in; b.sb_inb = up.sb_inb;
-	b.nlev = up.nlev; b.nsb = up.nsb; b.D = D; b.stage_bytes = sb;
-	b.chunk_sb = up.chunk_sb; b.chunk_lev = up.chunk_lev; b.bvo = up.bvo; b.cmax = up.cmax; b.skew = up.skew;
-	// one launch for both sweeps unless FEMGPU_SWEEP_FB=0
-	const char *e = getenv("FEMGPU_SWEEP_FB");
-	if (!(e && e[0] == '0') && lo.rw == up.rw && lo.nchunk == up.nchunk &&
-	    launch_cs_fb(a, b, lo.rw, lo.nchunk, bytes_lo > bytes ? bytes_lo : bytes, s, bl, y, o))
-		return (int)cudaGetLastError();
-	launch_cs<dsf, false>(a, lo.rw, lo.nchunk, bytes_lo, s, bl, y);
-	launch_cs<dsf, true>(b, up.rw, up.nchunk, bytes, s, y, o);
-	return (int)cudaGetLastError();
+	return run_df<dsf, true, true>(t, S.lo64c, S.up64c, S.prog_lo_ds, S.prog_up_ds, active, (const dsf *)S.bl64,
+	                               (dsf *)S.y64, (dsf *)S.o64);
 }
 
 extern "C" int fg_ilu0_sweeps_gathered(femgpu_transport *t, const int *active)
