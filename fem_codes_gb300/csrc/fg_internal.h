@@ -147,10 +147,10 @@ typedef struct fg_krylov {
 	double *orth;                   /* device-wide sums of the one-launch steps
 	                                 * and scratch (fg_kry_orth_bytes)        */
 	/* FGMRES look-ahead (la_s != NULL): the preconditioner of the next step
-	 * runs on la_s, on the raw operator output la_w, while the Gram-Schmidt
-	 * of this step runs on stream; la_t [ldv] the combination of the stored
+	 * runs on the raw operator output la_w while the Gram-Schmidt of this
+	 * step runs on la_s; la_t [ldv] the combination of the stored
 	 * directions, la_eta the subdiagonal entry, la_flag [kmax+1] per-step
-	 * snapshots of the convergence flag for the la_s work */
+	 * snapshots of the convergence flag for the preconditioner */
 	cudaStream_t la_s;
 	cudaEvent_t la_ev_w, la_ev_y;
 	double *la_w, *la_t, *la_eta;

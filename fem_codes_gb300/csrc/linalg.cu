@@ -818,8 +818,8 @@ __global__ void k_la_fin_ds(double *z, const dsf *y, const double *t, int n, con
 	}
 }
 
-// The convergence flag as the step starts, for the work on the look-ahead
-// stream: a copy that no later kernel changes, so every thread of a sweep
+// The convergence flag as the step starts, for the sweeps beside the
+// Gram-Schmidt: a copy that no later kernel changes, so every thread of a sweep
 // reads the same value while the Givens kernel of the step may clear the
 // flag itself concurrently.
 __global__ void k_la_snap(const fg_status *st, int *flag) { *flag = st->active; }
@@ -834,11 +834,15 @@ __global__ void k_la_snap(const fg_status *st, int *flag) { *flag = st->active; 
 
 // Look-ahead flexible GMRES cycle.  With w = A z_i and v_(i+1) =
 // (w - V h) / eta, linearity of M^-1 gives M^-1 v_(i+1) = (y - Z h) / eta
-// for y = M^-1 w and Z = [M^-1 v_0 .. M^-1 v_i].  So y is computed on la_s
-// from the raw operator output while the step's Gram-Schmidt runs on the main
-// stream (block ILU(0)'s sweeps hold one SM per matrix block, the multi-dot
-// and the update the others), t = Z h follows the coefficients, and the step
-// then waits only for y and forms z_(i+1) = (y - t) / eta.  The z_i equal
+// for y = M^-1 w and Z = [M^-1 v_0 .. M^-1 v_i].  So y is computed from the raw
+// operator output while the step's Gram-Schmidt runs on la_s (block ILU(0)'s
+// sweeps hold one SM per matrix block, the multi-dot and the update the
+// others), t = Z h follows the coefficients, and the step then waits only for
+// both and forms z_(i+1) = (y - t) / eta.  The sweeps stay on the main stream,
+// where they start as soon as the product ends; behind an event on la_s they
+// came after the multi-dot had taken every SM, 60 us late with a few basis
+// vectors and 170 with fifty (2048x1024 cells, 32 blocks; a Picard step of 97
+// iterations 85.9 ms, 82.2 this way).  The z_i equal
 // M^-1 v_i up to rounding; the Arnoldi relation A Z = V H holds for the
 // stored z_i whatever their rounding, and, as every FGMRES solve here, the
 // solve is accepted on the true residual.
@@ -871,23 +875,25 @@ static int fgmres_cycle_la(const fg_krylov *k, const fg_linop *op, const double 
 			k_la_snap<<<1, 1, 0, s>>>(k->st, k->la_flag + i);
 			FG_TRY(cudaEventRecord(k->la_ev_w, s));
 			FG_TRY(cudaStreamWaitEvent(s2, k->la_ev_w, 0));
-			if (fused) rc = op->precond_g(op->ctx, k->la_flag + i, s2);
-			else rc = op->precond_s(op->ctx, k->la_w, znext, k->la_flag + i, s2);
+			if (fused) rc = op->precond_g(op->ctx, k->la_flag + i, s);
+			else rc = op->precond_s(op->ctx, k->la_w, znext, k->la_flag + i, s);
 			if (rc) return rc;
-			FG_TRY(cudaEventRecord(k->la_ev_y, s2));
 		}
+		fg_krylov o = *k;                                  // the orthogonalisation's stream
+		o.stream = more ? s2 : s;
 		for (int pass = 0; pass < gs; pass++) {
 			const int last = pass == gs - 1;
 			const double *win = pass == 0 ? k->la_w : w;
-			k_mdot<<<dim3(G, (m + MD_J - 1) / MD_J), RED_TPB, LA_SMEM, s>>>(V, ldv, n, m, win, k->partials, k->st);
-			k_mdot_fin<<<m, 32, 0, s>>>(k->partials, G, m, h, k->H + i, ldh, pass, k->st);
-			k_cgs_update<<<cgs_grid, RED_TPB, hs, s>>>(V, ldv, n, m, win, w, h, last, k->H + (i + 1) * ldh + i,
-			                                           k->partials, k->st);
+			k_mdot<<<dim3(G, (m + MD_J - 1) / MD_J), RED_TPB, LA_SMEM, o.stream>>>(V, ldv, n, m, win, k->partials, k->st);
+			k_mdot_fin<<<m, 32, 0, o.stream>>>(k->partials, G, m, h, k->H + i, ldh, pass, k->st);
+			k_cgs_update<<<cgs_grid, RED_TPB, hs, o.stream>>>(V, ldv, n, m, win, w, h, last, k->H + (i + 1) * ldh + i,
+			                                                  k->partials, k->st);
 		}
-		if (more) k_zcombo<<<cgs_grid, RED_TPB, hs, s>>>(Z, ldv, n, m, k->H + i, ldh, k->la_t, k->la_eta, k->st);
-		k_scale<<<fg_grid(n), FG_TPB, 0, s>>>(w, n, k->H + (i + 1) * ldh + i, k->st);
-		if ((rc = fg_kry_givens(k, i))) return rc;
+		if (more) k_zcombo<<<cgs_grid, RED_TPB, hs, s2>>>(Z, ldv, n, m, k->H + i, ldh, k->la_t, k->la_eta, k->st);
+		k_scale<<<fg_grid(n), FG_TPB, 0, o.stream>>>(w, n, k->H + (i + 1) * ldh + i, k->st);
+		if ((rc = fg_kry_givens(&o, i))) return rc;
 		if (more) {
+			FG_TRY(cudaEventRecord(k->la_ev_y, s2));
 			FG_TRY(cudaStreamWaitEvent(s, k->la_ev_y, 0));
 			if (fused)
 				k_la_fin_ds<<<fg_grid(n), FG_TPB, 0, s>>>(znext, (const dsf *)op->precond_g_out(op->ctx), k->la_t, n,
@@ -1079,7 +1085,7 @@ static int krylov_ds(const femgpu_transport *t)
 	return env && t->o.solver == FEMGPU_FGMRES && t->o.precision == FEMGPU_FP64 &&
 	       t->o.precond == FEMGPU_PREC_ILU0 && fg_ilu0_ds_ready(t);
 }
-// The preconditioner on another stream (the look-ahead step): the ILU(0)
+// The preconditioner on a given stream (the look-ahead step): the ILU(0)
 // apply launches everything on the context's stream, which is swapped for
 // the call.
 static int tr_precond_s(void *c, const double *p, double *z, const int *a, cudaStream_t s)
@@ -1108,10 +1114,10 @@ static int tr_precond_g(void *c, const int *a, cudaStream_t s)
 static const void *tr_precond_g_out(void *c) { return ((femgpu_transport *)c)->sweeps.o64; }
 
 // FGMRES with the look-ahead step (fgmres_cycle_la): FP64 block or global
-// ILU(p) contexts, unless FEMGPU_LOOKAHEAD=0 (read at every cycle).  Its stream (the highest
-// priority, so the sweep CTAs are placed before the Gram-Schmidt blocks
-// that become ready with them), events and vectors are made on first use;
-// without them the plain cycle runs.
+// ILU(p) contexts, unless FEMGPU_LOOKAHEAD=0 (read at every cycle).  Its stream (the lowest
+// priority, so the Gram-Schmidt blocks never go before the sweep CTAs that
+// become ready with them), events and vectors are made on first use; without
+// them the plain cycle runs.
 static int lookahead_on(femgpu_transport *t)
 {
 	const char *e = getenv("FEMGPU_LOOKAHEAD");
@@ -1122,7 +1128,7 @@ static int lookahead_on(femgpu_transport *t)
 		int lo = 0, hi = 0;
 		cudaStream_t st = nullptr;
 		if (cudaDeviceGetStreamPriorityRange(&lo, &hi) != cudaSuccess ||
-		    cudaStreamCreateWithPriority(&st, cudaStreamNonBlocking, hi) != cudaSuccess) {
+		    cudaStreamCreateWithPriority(&st, cudaStreamNonBlocking, lo) != cudaSuccess) {
 			cudaGetLastError();
 			return 0;
 		}
