@@ -177,10 +177,16 @@ __device__ __forceinline__ bool poll_words(unsigned long long (&x)[NQ], const do
 	}
 }
 
-// Eight warps' sums as linalg.cu's block_sum adds them (its shuffle tree).
-__device__ __forceinline__ double tree8(const double *s)
+// Eight warps' sums as linalg.cu's block_sum adds them (its shuffle tree), lane
+// 8 g + w holding warp w's sum of group g.  Three FP64 operations of one warp:
+// every thread adding the eight up for itself is seven of eight warps, 900
+// clocks of the four FP64 pipes for each of MGS's sums (64x64 transport, ten
+// sums a step on average: 19.5 us a step that way, 14.3 now).
+__device__ __forceinline__ double tree8_lanes(double s)
 {
-	return ((s[0] + s[4]) + (s[2] + s[6])) + ((s[1] + s[5]) + (s[3] + s[7]));
+	s += __shfl_xor_sync(0xffffffffu, s, 4);
+	s += __shfl_xor_sync(0xffffffffu, s, 2);
+	return s + __shfl_xor_sync(0xffffffffu, s, 1);
 }
 
 // The total of nb published parts as last_block_total adds them: thread t takes
@@ -189,18 +195,25 @@ template <int NQ>
 __device__ __forceinline__ bool block_total(const double *slot, int nb, const OrthArgs &a, double *sw, int *fail,
                                             double *tot)
 {
-	unsigned long long x[NQ];
-	const bool ok = poll_words<NQ>(x, slot, threadIdx.x, OR_TPB, nb, a.tk, &a.st->err);
+	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 	double v = 0.0;
+	if (32 * warp < nb) {                                 // (uniform; the others' sums are zeros)
+		unsigned long long x[NQ];
+		const bool ok = poll_words<NQ>(x, slot, threadIdx.x, OR_TPB, nb, a.tk, &a.st->err);
 #pragma unroll
-	for (int q = 0; q < NQ; q++) if (q == 0 || q * OR_TPB < nb) v += __longlong_as_double((long long)x[q]);
-	v = fg_warp_sum(v);
-	if ((threadIdx.x & 31) == 0) {
-		sw[threadIdx.x >> 5] = v;
-		if (!ok) *fail = 1;
+		for (int q = 0; q < NQ; q++) if (q == 0 || q * OR_TPB < nb) v += __longlong_as_double((long long)x[q]);
+		v = fg_warp_sum(v);
+		if (lane == 0 && !ok) *fail = 1;
 	}
+	if (nb <= 32) {                                       // the first warp's sum is the total
+		if (threadIdx.x == 0) sw[0] = v;
+		__syncthreads();
+		*tot = sw[0];
+		return *fail == 0;
+	}
+	if (lane == 0) sw[warp] = v;
 	__syncthreads();
-	*tot = tree8(sw);
+	*tot = tree8_lanes(sw[lane & 7]);
 	return *fail == 0;
 }
 
@@ -262,7 +275,11 @@ __global__ void __launch_bounds__(OR_TPB) k_orth_mgs(OrthArgs a)
 			if (lane == 0) sw[q][warp] = part;
 		}
 		__syncthreads();
-		if (tid < NV && (int)blockIdx.x + tid * a.G < a.nvb) fg_st_value(&slot[blockIdx.x + tid * a.G], tree8(sw[tid]));
+		if (warp == 0) {
+			const int g = lane >> 3;
+			const double t = tree8_lanes(g < NV ? sw[g][lane & 7] : 0.0);
+			if (g < NV && !(lane & 7) && (int)blockIdx.x + g * a.G < a.nvb) fg_st_value(&slot[blockIdx.x + g * a.G], t);
+		}
 		if (!block_total<2>(slot, a.nvb, a, sv[j & 1], &fail, &h)) return;
 	}
 	const double sc = 1.0 / sqrt(h);
@@ -400,9 +417,11 @@ __global__ void __launch_bounds__(OR_TPB) k_orth_cgs(OrthArgs a)
 			if (lane == 0) sw[q * S + s][warp] = t;
 		}
 	__syncthreads();
-	if (tid < NV * S) {
-		const int q = tid / S, s = tid - q * S, b = blockIdx.x + q * a.G + s * OR_VB;
-		if ((int)blockIdx.x + q * a.G < nvb && b < nb) fg_st_value(&norm[b], tree8(sw[tid]));
+	if (warp == 0) {
+		static_assert(NV * S <= 4, "a group of eight lanes each");
+		const int g = lane >> 3, q = g / S, s = g - q * S, b = blockIdx.x + q * a.G + s * OR_VB;
+		const double t = tree8_lanes(g < NV * S ? sw[g][lane & 7] : 0.0);
+		if (g < NV * S && !(lane & 7) && (int)blockIdx.x + q * a.G < nvb && b < nb) fg_st_value(&norm[b], t);
 	}
 	double tot;
 	if (!block_total<3>(norm, nb, a, sv, &fail, &tot)) return;
@@ -443,8 +462,8 @@ static double *orth_tail(const fg_krylov *k) { return k->orth + 2 * orth_words(k
 // unknowns at most); beyond, the separate kernels are bound by the FP64 pipes
 // and the launches between them no longer count.  Measured, whole solves with
 // the launches of converged steps gone too: 64x64 transport, GMRES(30), a Picard
-// iteration 6.2 -> 3.4 ms (a step's orthogonalisation 19 us, of 10 dot products
-// on average, each a launch of 2.3 us and a gap before); Euler 256x64, FGMRES(50),
+// iteration 6.2 -> 3.4 ms (a step's orthogonalisation 19 us, now 14, of 10 dot
+// products on average, each a launch of 2.3 us and a gap before); Euler 256x64, FGMRES(50),
 // a time step 19.7 -> 10.8 ms (35 us a step, half of them two passes; multi-dot
 // 13, finish 2, update 7, scaling 2 and Givens 8 us before, gaps apart).
 extern "C" int fg_kry_orth_fits(const fg_krylov *k)
