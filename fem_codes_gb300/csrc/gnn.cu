@@ -649,56 +649,87 @@ __global__ void k_gnn_decode(int n, const TA *h, const float *__restrict__ th, c
 // Loss gradients dL/dz: supervised (ILU target) 2 (z - t) / sum t^2, and
 // residual 2 A^T (A z - v) / sum v^2 with A = diag(d) (I + W) from the graph
 // (a_ij = d_i wA_ij; (A^T y)_j = d_j y_j + sum_q wT[q] d_col y_col).
-__global__ void k_gnn_gz_sup(int n, const double *z, const double *t, const double *sums, double *gz, int add)
+__global__ void k_gnn_gz_sup(int n, const double *z, const double *t, const double *sums, double *gz)
 {
 	const double T2 = sums[0];
-	for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-		double g = 2.0 * (z[i] - t[i]) / T2;
-		gz[i] = add ? gz[i] + g : g;
-	}
+	for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+		gz[i] = 2.0 * (z[i] - t[i]) / T2;
 }
 
-__global__ void k_gnn_resid(int n, const int *__restrict__ gptr, const int *__restrict__ gcol,
+// res = A z - v and the loss sums out[0] = sum v_i^2, out[1] = sum res_i^2: each
+// thread sums what it computes, in k_gnn_psums's order, and the last block to
+// finish adds the partial sums up as k_gnn_fsums does.  65k nodes: 9.7 us; six
+// launches (the residual, two sums of two kernels, a copy) took 21 and ten of
+// gaps, the residual part of dL/dz in a kernel before k_gnn_decode_bwd six more.
+__global__ void __launch_bounds__(RTPB) k_gnn_resid(int n, const int *__restrict__ gptr, const int *__restrict__ gcol,
                             const float *__restrict__ wA, const double *d, const double *z, const double *v,
-                            double *res)
+                            double *res, double *part, unsigned *ticket, double *out)
 {
+	__shared__ double sh[32];
+	__shared__ bool last;
+	double s0 = 0.0, s1 = 0.0;
 	for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+		const double vi = v[i];
 		double s = z[i];
 		for (int p = gptr[i]; p < gptr[i + 1]; p++) s += (double)wA[p] * z[gcol[p]];
-		res[i] = d[i] * s - v[i];
+		const double e = d[i] * s - vi;
+		res[i] = e;
+		s0 += vi * vi;
+		s1 += e * e;
 	}
+	s0 = blk_sum(s0, sh);
+	s1 = blk_sum(s1, sh);
+	if (threadIdx.x == 0) {
+		part[2 * blockIdx.x] = s0;
+		part[2 * blockIdx.x + 1] = s1;
+		__threadfence();
+		last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+	}
+	__syncthreads();
+	if (!last) return;
+	double t0 = 0.0, t1 = 0.0;
+	for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x) {
+		t0 += __ldcg(&part[2 * b]);
+		t1 += __ldcg(&part[2 * b + 1]);
+	}
+	t0 = blk_sum(t0, sh);
+	t1 = blk_sum(t1, sh);
+	if (threadIdx.x == 0) { out[0] = t0; out[1] = t1; *ticket = 0u; }
 }
 
-__global__ void k_gnn_gz_res(int n, const int *__restrict__ gptr, const int *__restrict__ gcol,
-                             const float *__restrict__ wT, const double *d, const double *res, const double *sums,
-                             double scale, double *gz, int add)
-{
-	const double c = scale * 2.0 / sums[0];
-	for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
-		double s = d[j] * res[j];
-		for (int q = gptr[j]; q < gptr[j + 1]; q++) {
-			int i = gcol[q];
-			s += (double)wT[q] * d[i] * res[i];
-		}
-		gz[j] = add ? gz[j] + c * s : c * s;
-	}
-}
+// The residual loss's part of dL/dz (see k_gnn_gz_sup): its graph and A z - v.
+struct ResGrad { const int *gptr, *gcol; const float *wT; const double *res, *sums; };
 
 // gh = gy Wd with gy = gz s dbar / d; partials of gWd (32), gbd (1).  A warp
 // takes 32 nodes, lane q forming node q's gy (FP64) and lane f then feature f of
 // every node, so each row is one coalesced access and a lane keeps one sum.
-template <typename TA>
-__global__ void __launch_bounds__(RTPB) k_gnn_decode_bwd(int n, const double *gzv, const double *stats,
+// SUP: gz has the supervised part; RES: the residual part is formed here.
+template <typename TA, bool SUP, bool RES>
+__global__ void __launch_bounds__(RTPB) k_gnn_decode_bwd(int n, const double *gzv, ResGrad rg, const double *stats,
 		const double *d, const TA *h, const float *__restrict__ th, float *gh, float *part)
 {
 	__shared__ float sacc[RTPB / 32][W], sbd[RTPB / 32];
 	const double s = stats[0], dbar = stats[1];
 	const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, warps = (gridDim.x * blockDim.x) >> 5;
 	const float wd = th[GNN_OFF_WD + lane];
+	const double c = RES ? 2.0 / rg.sums[0] : 0.0;
 	float acc = 0.0f, accb = 0.0f;
 	for (int g0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32; g0 < n; g0 += warps * 32) {
 		const int i = g0 + lane, cnt = min(32, n - g0);
-		const float mine = i < n ? (float)(gzv[i] * s * dbar / d[i]) : 0.0f;
+		float mine = 0.0f;
+		if (i < n) {
+			double gz = SUP ? gzv[i] : 0.0;
+			const double di = d[i];
+			if (RES) {
+				double r = di * rg.res[i];
+				for (int q = __ldg(&rg.gptr[i]); q < __ldg(&rg.gptr[i + 1]); q++) {
+					const int k = __ldg(&rg.gcol[q]);
+					r += (double)__ldg(&rg.wT[q]) * d[k] * rg.res[k];
+				}
+				gz = SUP ? gz + c * r : c * r;
+			}
+			mine = (float)(gz * s * dbar / di);
+		}
 		accb += mine;
 		#pragma unroll 8
 		for (int q = 0; q < cnt; q++) {
@@ -1013,7 +1044,6 @@ __global__ void k_gnn_adam(int P, float *th, const float *g, float *m, float *v,
 }
 
 // ls[0..1] = (sum v^2, -), ls[2..3] = (sum res^2, -) -> ls[1] = sum res^2.
-__global__ void k_gnn_fix_sums(double *ls) { ls[1] = ls[2]; }
 
 __global__ void k_gnn_dbar(const double *sums, int n, double *stats) { stats[1] = sums[0] / n; }
 
@@ -1124,18 +1154,15 @@ static int backward_t(fg_gnn *g, const double *r, const double *z, const double 
 	const int PL = 3 * W * W + W;
 	int gn = nb(n, 256, 16 * FG_SMS);
 	// loss sums in g->lsums: [0] = normaliser, [1] = squared error (loss = [1]/[0])
+	ResGrad rg = { nullptr, nullptr, nullptr, nullptr, nullptr };
 	if (g->loss_kind != GNN_LOSS_RESIDUAL) {
 		sums(g, n, t, z, 0, g->lsums);            // sum t^2, sum (z - t)^2
-		k_gnn_gz_sup<<<gn, 256, 0, s>>>(n, z, t, g->lsums, g->gz, 0);
+		k_gnn_gz_sup<<<gn, 256, 0, s>>>(n, z, t, g->lsums, g->gz);
 	}
 	if (g->loss_kind != GNN_LOSS_SUPERVISED) {
 		double *ls = g->loss_kind == GNN_LOSS_RESIDUAL ? g->lsums : g->lsums2;
-		k_gnn_resid<<<gn, 256, 0, s>>>(n, g->gptr, g->gcol, g->wA, g->d, z, r, g->res);
-		sums(g, n, r, nullptr, 0, ls);            // sum r^2 (the input residual)
-		sums(g, n, g->res, nullptr, 0, ls + 2);   // sum (A z - v)^2
-		k_gnn_fix_sums<<<1, 1, 0, s>>>(ls);
-		k_gnn_gz_res<<<gn, 256, 0, s>>>(n, g->gptr, g->gcol, g->wT, g->d, g->res, ls, 1.0, g->gz,
-		                                g->loss_kind == GNN_LOSS_BOTH);
+		k_gnn_resid<<<GNN_RED_BLOCKS, RTPB, 0, s>>>(n, g->gptr, g->gcol, g->wA, g->d, z, r, g->res, g->rpart, g->ticket, ls);
+		rg = ResGrad{g->gptr, g->gcol, g->wT, g->res, ls};
 	}
 	// partial sums of the stages, one after another in g->part
 	RedArgs red;
@@ -1148,8 +1175,13 @@ static int backward_t(fg_gnn *g, const double *r, const double *z, const double 
 		return red.st[k].part;
 	};
 	int gd = nb(n, RTPB, GNN_BWD_BLOCKS);
-	k_gnn_decode_bwd<TA><<<gd, RTPB, 0, s>>>(n, g->gz, g->stats, g->d, H[GNN_LAYERS], g->theta, g->gh[0],
-	                                         (float *)stage(0, gd, W + 1, GNN_OFF_WD));
+	float *pd = (float *)stage(0, gd, W + 1, GNN_OFF_WD);
+#define DECODE_BWD(S, R) k_gnn_decode_bwd<TA, S, R><<<gd, RTPB, 0, s>>>(n, g->gz, rg, g->stats, g->d, H[GNN_LAYERS], \
+	g->theta, g->gh[0], pd)
+	if (g->loss_kind == GNN_LOSS_RESIDUAL) DECODE_BWD(false, true);
+	else if (g->loss_kind == GNN_LOSS_SUPERVISED) DECODE_BWD(true, false);
+	else DECODE_BWD(true, true);
+#undef DECODE_BWD
 	int cur = 0;
 	int gu = nb(n, TILE, GNN_BWD_BLOCKS);
 	for (int l = GNN_LAYERS - 1; l >= 0; l--) {
