@@ -73,6 +73,7 @@ typedef struct fg_ilu_sweeps {
 	/* ds: dpos [n] the slot of natural row r in the sweeps' gathered input
 	 * (the inverse of the gather of the double-single apply) */
 	int *dpos;
+	int *dpos64;                    /* the same for lo64's input               */
 	double *bl64, *y64;
 	double *o64;                    /* ds: the double-single sweeps' output
 	                                   (natural order), apart from their input */
@@ -182,6 +183,9 @@ typedef struct fg_linop {
 	int (*matvec_g)(void *ctx, const double *p, double *q, const int *active);
 	int (*precond_g)(void *ctx, const int *active, cudaStream_t s);
 	const void *(*precond_g_out)(void *ctx);
+	/* left-preconditioned GMRES: z = M^-1 A p with the product written as the
+	 * preconditioner's gathered input only (NULL: the two one by one) */
+	int (*matvec_precond)(void *ctx, const double *p, double *z, const int *active);
 } fg_linop;
 
 struct femgpu_transport {

@@ -2035,6 +2035,9 @@ extern "C" int fg_ilu_prepare(femgpu_transport *t, const int *hIA, const int *hJ
 	}
 	FG_TRY(cudaMemset(S.bl32, 0, sizeof(float) * nb));
 	FG_TRY(cudaMemset(S.y32, 0, sizeof(float) * nb));
+	FG_TRY(cudaMalloc((void **)&S.dpos64, sizeof(int) * (size_t)std::max(n, 1)));
+	k_inv_gather<<<fg_grid(n), FG_TPB, 0, t->stream>>>(S.lo64.rows, S.lo64.ppos, n, S.dpos64);
+	FG_TRY(cudaGetLastError());
 	const fg_sweep *all[4] = { &S.lo64, &S.up64, &S.lo32, &S.up32 };
 	for (int i = 0; i < 4; i++) {
 		rc = sweep_smem(*all[i], i < 2 ? sizeof(double) : sizeof(float), &D, &sb);
@@ -2172,7 +2175,7 @@ static int apply_t(femgpu_transport *t, const fg_sweep &lo, const fg_sweep &up, 
 {
 	cudaStream_t s = t->stream;
 	const int n = t->neq;
-	k_perm_in<T, TI><<<fg_grid(n), FG_TPB, 0, s>>>(p, lo.rows, lo.ppos, n, bl);
+	if (p) k_perm_in<T, TI><<<fg_grid(n), FG_TPB, 0, s>>>(p, lo.rows, lo.ppos, n, bl);
 	if (lo.cs) return run_df<T, true, true>(t, lo, up, lo.prog, up.prog, active, bl, y, (T *)z);
 	fma = fma && sizeof(T) == 8;
 	if (lo.df && up.df)
@@ -2245,6 +2248,16 @@ extern "C" int fg_ilu0_apply64(femgpu_transport *t, const double *p, double *z, 
 	return apply_t<double, double, double>(t, S.lo64, S.up64, S.bl64, S.y64, p, z, active, fma);
 }
 
+// z = M^-1 p by the separately rounded sweeps, p already in bl64 as lo64 takes it
+// (at dpos64[row]).
+extern "C" int fg_ilu0_apply64_gathered(femgpu_transport *t, double *z, const int *active)
+{
+	fg_ilu_sweeps &S = t->sweeps;
+	const int rc = refresh_pair(t, 0);
+	if (rc) return rc;
+	return apply_t<double, double, double>(t, S.lo64, S.up64, S.bl64, S.y64, nullptr, z, active, false);
+}
+
 // The double-single sweeps with a double-single input (the Krylov basis of
 // the double-single Arnoldi); available when fg_ilu0_ds_ready says so.
 extern "C" int fg_ilu0_ds_ready(const femgpu_transport *t)
@@ -2288,7 +2301,8 @@ extern "C" void fg_ilu_free(femgpu_transport *t)
 	S.fA = nullptr;
 	S.fill = 0;
 	if (S.dpos) cudaFree(S.dpos);
-	S.dpos = nullptr;
+	if (S.dpos64) cudaFree(S.dpos64);
+	S.dpos = S.dpos64 = nullptr;
 	if (S.prog_lo_ds) cudaFree(S.prog_lo_ds);
 	if (S.prog_up_ds) cudaFree(S.prog_up_ds);
 	S.prog_lo_ds = S.prog_up_ds = nullptr;
