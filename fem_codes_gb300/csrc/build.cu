@@ -13,14 +13,14 @@
 // This translation unit is compiled with --fmad=false: every product and sum
 // is rounded separately, as in the reference compiled without contraction.
 #include "fg_common.cuh"
-#include "fg_div.cuh"
 
 struct BuildArgs {
 	const double *x, *y, *u, *upresc, *beta, *fsrc;
 	const int *vert, *node_id;
 	double k, gamma, cbx, cby;
 	int nel, shock, hshock, beta_const, fsrc_zero;
-	double bnorm, rbnorm;         // constant velocity: its norm and the inverse
+	const double2 *geo;           // steady build: an element's 1 / area and length h
+	const double *tau;            // ... and its SUPG parameter
 	double *ke, *fe;              // fe: NULL without a source (steady build)
 	// transient builds only
 	const double *du;             // the time derivative a (neq+1)
@@ -91,12 +91,13 @@ __device__ __forceinline__ double shock_capture(int kind, double kx, double ky, 
 // and are left out, as is Fe without a source).
 //
 // Bound by the FP64 pipes: 64 clocks a warp's instruction on this part, about
-// 360 instructions an element with the terms that vanish, 270 without them, the
-// constant velocity's norm formed once, h_shock = h for 2sqrtArea (2 Area is
-// TwoA exactly) and one quotient where shock_capture had one a branch.  The
+// 360 instructions an element with the terms that vanish, 270 without them, with
+// h_shock = h for 2sqrtArea (2 Area is TwoA exactly) and one quotient where
+// shock_capture had one a branch, 24 fewer with the reciprocal, the root and the
+// quotient that depend on mesh and velocity only from fg_element_geometry.  The
 // element matrices leave through shared memory in whole lines (nine 8-byte
 // stores 72 bytes apart touch every sector four times).  At 2.16M elements, constant velocity, no
-// source or reaction: 1270 us before, 919 with both.
+// source or reaction: 1270 us before, 839 now.
 template <bool SRC, bool REACT>
 __global__ void __launch_bounds__(128) k_build_supg(BuildArgs a)
 {
@@ -110,17 +111,11 @@ __global__ void __launch_bounds__(128) k_build_supg(BuildArgs a)
 		double Y0 = __ldg(&a.y[J1]), Y1 = __ldg(&a.y[J2]), Y2 = __ldg(&a.y[J3]);
 		double y23 = Y1 - Y2, y31 = Y2 - Y0, y12 = Y0 - Y1;
 		double x32 = X2 - X1, x13 = X0 - X2, x21 = X1 - X0;
-		double TwoA = x21*y31 - x13*y12, Area = 0.5*TwoA, invArea = 1.0/Area;
-		double h = sqrt(fabs(TwoA));
-		double bx, by, tau = 0.0;
-		if (a.beta_const) {
-			bx = a.cbx; by = a.cby;
-			if (a.bnorm > 0) tau = fg_div(0.5*h, a.bnorm, a.rbnorm);
-		} else {
-			bx = __ldg(&a.beta[2*E]); by = __ldg(&a.beta[2*E+1]);
-			double norm = sqrt(bx*bx + by*by);
-			if (norm > 0) tau = 0.5*h/norm;
-		}
+		double TwoA = x21*y31 - x13*y12, Area = 0.5*TwoA;      // (Area: REACT, SRC and other lengths only)
+		const double2 geo = __ldg(&a.geo[E]);
+		const double invArea = geo.x, h = geo.y, tau = __ldg(&a.tau[E]);
+		double bx = a.cbx, by = a.cby;
+		if (!a.beta_const) { bx = __ldg(&a.beta[2*E]); by = __ldg(&a.beta[2*E+1]); }
 		double fe1 = 0.0, fe2 = 0.0, fe3 = 0.0;
 		if (SRC) { fe1 = __ldg(&a.fsrc[3*E]); fe2 = __ldg(&a.fsrc[3*E+1]); fe3 = __ldg(&a.fsrc[3*E+2]); }
 		double feb = SRC ? third*(fe1+fe2+fe3) : 0.0;
@@ -191,6 +186,31 @@ __global__ void __launch_bounds__(128) k_build_supg(BuildArgs a)
 	}
 }
 
+// What a steady element build takes from the mesh and the velocity alone, formed
+// once for the context.
+__global__ void k_element_geometry(BuildArgs a, double2 *geo, double *tau)
+{
+	for (int E = blockIdx.x * blockDim.x + threadIdx.x; E < a.nel; E += gridDim.x * blockDim.x) {
+		const int J1 = a.vert[3*E], J2 = a.vert[3*E+1], J3 = a.vert[3*E+2];
+		const double y31 = a.y[J3] - a.y[J1], y12 = a.y[J1] - a.y[J2];
+		const double x13 = a.x[J1] - a.x[J3], x21 = a.x[J2] - a.x[J1];
+		const double TwoA = x21*y31 - x13*y12, Area = 0.5*TwoA, h = sqrt(fabs(TwoA));
+		const double bx = a.beta_const ? a.cbx : a.beta[2*E], by = a.beta_const ? a.cby : a.beta[2*E+1];
+		const double norm = sqrt(bx*bx + by*by);
+		geo[E] = make_double2(1.0/Area, h);
+		tau[E] = norm > 0 ? 0.5*h/norm : 0.0;
+	}
+}
+
+extern "C" int fg_element_geometry(femgpu_transport *t)
+{
+	BuildArgs a;
+	a.x = t->x; a.y = t->y; a.beta = t->beta; a.vert = t->vert;
+	a.cbx = t->cbx; a.cby = t->cby; a.nel = t->nel; a.beta_const = t->beta_const;
+	k_element_geometry<<<fg_grid(t->nel), FG_TPB, 0, t->stream>>>(a, (double2 *)t->geo, t->geo_tau);
+	return (int)cudaGetLastError();
+}
+
 extern "C" int fg_build_elements(femgpu_transport *t)
 {
 	BuildArgs a;
@@ -199,8 +219,7 @@ extern "C" int fg_build_elements(femgpu_transport *t)
 	a.k = t->k; a.gamma = t->gamma; a.cbx = t->cbx; a.cby = t->cby;
 	a.nel = t->nel; a.shock = t->o.shock; a.hshock = t->o.hshock;
 	a.beta_const = t->beta_const; a.fsrc_zero = t->fsrc_zero;
-	a.bnorm = sqrt(a.cbx*a.cbx + a.cby*a.cby);
-	a.rbnorm = 1.0/a.bnorm;
+	a.geo = (const double2 *)t->geo; a.tau = t->geo_tau;
 	a.ke = (t->o.scheme == FEMGPU_EBE) ? t->A : t->ke;
 	a.fe = t->fe;
 	const int g = fg_grid(t->nel, 128, 32);

@@ -196,6 +196,7 @@ struct femgpu_transport {
 
 	/* mesh / problem */
 	double *x, *y, *upresc, *beta, *fsrc;
+	double *geo, *geo_tau;          /* steady build: [nel][2] 1 / area and h, [nel] tau */
 	int *node_type, *node_id, *vert, *lm;
 	double k, gamma, cbx, cby;
 	int beta_const, fsrc_zero;
@@ -275,6 +276,7 @@ int fg_build_ede(femgpu_transport *t);                       /* lm2, sbe, ... */
 int fg_compute_lm(femgpu_transport *t);                      /* lm from ids   */
 
 /* build.cu */
+int fg_element_geometry(femgpu_transport *t);
 int fg_build_elements(femgpu_transport *t);                  /* ke / A, fe    */
 int fg_assemble(femgpu_transport *t);                        /* A (CSR/EDE), F */
 int fg_build_transient(femgpu_transport *t, int dd, double adt);   /* Ae, re   */

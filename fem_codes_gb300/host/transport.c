@@ -250,6 +250,9 @@ int femgpu_transport_create(femgpu_transport **out, const femgpu_transport_opts 
 	DM(t->A, sizeof(double) * nA);
 	CK(cudaMemsetAsync(t->A, 0, sizeof(double) * nA, t->stream));
 	DM(t->fe, sizeof(double) * 3 * (size_t)nel);
+	DM(t->geo, sizeof(double) * 2 * (size_t)nel);
+	DM(t->geo_tau, sizeof(double) * (size_t)nel);
+	KR(fg_element_geometry(t));
 	DM(t->u, sizeof(double) * ((size_t)neq + 1));
 	DM(t->F, sizeof(double) * ((size_t)neq + 1));
 	DM(t->F0, sizeof(double) * ((size_t)neq + 1));
@@ -342,7 +345,7 @@ void femgpu_transport_destroy(femgpu_transport *t)
 	if (t->amg) femgpu_amg_set_stream(t->amg, NULL);
 	void *ptrs[] = { t->x, t->y, t->upresc, t->beta, t->fsrc, t->node_type, t->node_id, t->vert,
 		t->lm, t->ri_ptr, t->ri, t->IA, t->JA, t->sbe, t->diag, t->lm2, t->order, t->ec_ptr,
-		t->ec, t->e2_ptr, t->e2, t->A, t->ke, t->fe, t->A32, t->u, t->F, t->F0, t->invDiag,
+		t->ec, t->e2_ptr, t->e2, t->A, t->ke, t->fe, t->geo, t->geo_tau, t->A32, t->u, t->F, t->F0, t->invDiag,
 		t->invDiag32, t->ilu.LU, t->ilu.Dinv, t->V, t->H, t->cs, t->sn, t->ge, t->gy, t->w2,
 		t->Z, t->Z32, t->xr, t->dr, t->partials, t->orth, t->st, t->du, t->uold, t->Da, t->re, t->dold,
 		t->u1, t->u2, t->uB, t->aB, t->bub, t->uB1, t->uB2, t->la_buf, t->la_flag, t->sell_base, t->sell_w, t->sell_JA, t->sell_A };
