@@ -17,13 +17,13 @@ residual (right-preconditioned flexible GMRES(80); the reference's
 left-preconditioned stopping rule is not used because it accepts residuals of
 0.5 on this mesh).  Default preconditioner: block ILU(0) over 32 contiguous
 row blocks of the SYMRCM numbering cut at equal spans of the factor's
-dependency levels, each factorised by its own thread-block cluster and swept
-by its own thread block (--ilu-blocks 0: ILU(0) of the whole matrix).  The
+dependency levels, factorised as one dataflow of rows over the device, each
+block swept by its own thread block (--ilu-blocks 0: ILU(0) of the whole matrix).  The
 sweeps solve rows chained along the SYMRCM fronts 32 at a time by a warp scan
 in double-single arithmetic (48-bit significands on the FP32 pipes, the
 residual and Arnoldi in FP64), forward and backward in one launch.  Each
-FGMRES step starts the next direction's sweeps on a second stream as soon as
-the operator product is done and runs the Gram-Schmidt on the other SMs
+FGMRES step starts the next direction's sweeps as soon as the operator
+product is done and runs the Gram-Schmidt on a second stream and the other SMs
 meanwhile (the look-ahead step; FEMGPU_LOOKAHEAD=0 for the plain step).
 Steps continue the Picard sequence from the warm-up steps.
 
@@ -376,8 +376,8 @@ def run_ours(a):
         if chain:
             ds = a.precision == "FP64" and os.environ.get("FEMGPU_SWEEP_DS", "1") != "0"
             fb = ds and os.environ.get("FEMGPU_SWEEP_FB", "1") != "0"
-            name = (("k_sweep_cs_fb (ILU(0) forward and backward sweeps in one launch" if fb else
-                     "k_sweep_cs (ILU(0) forward+backward")
+            name = (("k_sweep_fb (ILU(0) forward and backward sweeps in one launch" if fb else
+                     "k_sweep_df (ILU(0) forward+backward")
                     + ", chain-scan: rows chained along the SYMRCM fronts solved "
                     "32 at a time by a warp scan" + (" in double-single arithmetic" if ds else "")
                     + ", row records, dataflow between warps")
@@ -386,7 +386,7 @@ def run_ours(a):
         elif os.environ.get("FEMGPU_SWEEP_SYNC") == "barrier":
             name = "k_sweep_rec (ILU(0) forward+backward, row records, a barrier per level"
         else:
-            name = "k_sweep_df (ILU(0) forward+backward, row records, dataflow between warps"
+            name = "k_sweep_fb (ILU(0) forward and backward sweeps in one launch, row records, dataflow between warps"
         name += f", TMA-staged, one CTA per matrix block, {max(a.ilu_blocks, 1)} blocks)"
     else:
         alg = nnz * 12 + (neq + 1) * 4 + 2 * neq * 8
@@ -655,9 +655,9 @@ def read_traffic(kind):
 
 
 def launches_estimate(a, iters):
-    """Kernel launches of the timed steps (a FGMRES cycle enqueues all kmax
-    steps; those past convergence are predicated off but launched): build 2
-    (element build, CSR assembly with the RHS) + factor 5 (cluster elimination,
+    """Kernel launches of the timed steps (a FGMRES cycle enqueues its steps six
+    ahead of the device; those past convergence find nothing to do): build 2
+    (element build, CSR assembly with the RHS) + factor 6 (marking, elimination,
     double-single program refresh and scan multipliers of both sweeps) + per
     cycle 5 (product, residual start, scaling; back-substitution and update)
     and in the look-ahead step 3 more for the first direction's preconditioner
@@ -674,11 +674,12 @@ def launches_estimate(a, iters):
         cyc = max(1, (int(it) + kmax - 1) // kmax)
         for c in range(cyc):
             gs = 3 * (1 if c == 0 else 2)
+            steps = min(kmax, int(it) - c * kmax + 6)
             if la:
-                tot += 8 + (kmax - 1) * (7 + gs) + (3 + gs)
+                tot += 8 + steps * (7 + gs) - (4 if steps == kmax else 0)
             else:
-                tot += 5 + kmax * (3 + 1 + gs + 2)
-        tot += 2 + 5 + 2
+                tot += 5 + steps * (3 + 1 + gs + 2)
+        tot += 2 + 6 + 2
     return tot
 
 

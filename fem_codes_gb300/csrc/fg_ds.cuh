@@ -37,6 +37,15 @@ __device__ __forceinline__ dsf ds_fma(dsf a, dsf b, dsf c)
 	return ds_fast_two_sum(s.hi, s.lo);
 }
 
+// a * b: ds_fma with c = 0 without the sums that add nothing
+__device__ __forceinline__ dsf ds_mul(dsf a, dsf b)
+{
+	const float p = a.hi * b.hi;
+	float e = fmaf(a.hi, b.hi, -p);
+	e = fmaf(a.hi, b.lo, fmaf(a.lo, b.hi, e));
+	return ds_fast_two_sum(p, e);
+}
+
 __host__ __device__ __forceinline__ dsf ds_neg(dsf a) { return dsf{ -a.hi, -a.lo }; }
 
 __device__ __forceinline__ dsf ds_from(double v)

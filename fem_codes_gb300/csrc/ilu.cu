@@ -49,7 +49,7 @@
 #define SW_MAXW 8                     // dependencies per row on the unrolled path
 #define SW_RPT 4                      // rows per consumer thread per pass
 #define SW_RING 4096                  // ring slots (power of two)
-#define SW_RING_WIDE 8192             // ... of dataflow programs with wide levels
+#define SW_RING_WIDE 8192             // ... of dataflow programs whose stages leave room
 #define SW_NEAR 0x80000000u           // dependency code: ring slot (dataflow programs: global position)
 #define SW_WAIT_LIMIT (1 << 24)
 #define SW_MAXD 12                    // max stages
@@ -165,7 +165,7 @@ template <typename T, bool FMA> __device__ __forceinline__ T fmsub(T x, T a, T b
 #include "fg_ds.cuh"
 
 template <> __device__ __forceinline__ dsf fmsub<dsf, true>(dsf x, dsf a, dsf b) { return ds_fma(ds_neg(a), b, x); }
-template <> __device__ __forceinline__ dsf mul(dsf a, dsf b) { return ds_fma(a, b, dsf{ 0.0f, 0.0f }); }
+template <> __device__ __forceinline__ dsf mul(dsf a, dsf b) { return ds_mul(a, b); }
 
 // zero, FP64 -> T, and the cache-global load / warp shuffle of a T
 template <typename T> __device__ __forceinline__ T zero_t() { return T(0); }
@@ -217,7 +217,7 @@ struct SweepArgs {
 	int wait;                     // spins of a warp waiting for the rows it depends on
 };
 
-// The producer warp of every sweep kernel: streams this thread block's
+// The producer warp of the barrier sweeps: streams this thread block's
 // sub-blocks [sb0, sb1) and their input slices into the D-stage ring with
 // cp.async.bulk (completion on full[s]), reusing a stage once the consumers
 // have released it (empty[s]); stops when a consumer has failed.  The input
@@ -508,7 +508,7 @@ k_sweep_rec(SweepArgs a, const T *__restrict__ in, T *out)
 // level always on the first warps) and now: 64x64 cells, 2 x 127 levels, FP64:
 // 117 us, 67; 400x300 cells, 2 x 1098 levels, FP64: 1.50 ms, 0.80; 2048x1024
 // cells in 32 blocks, double-single chains, the largest block 9106 chunks:
-// 0.70 ms, 0.46.  FP64: a level is a poll (about 100 clocks) and the newest
+// 0.70 ms, 0.45.  FP64: a level is a poll (about 100 clocks) and the newest
 // values' multiplications and subtractions, 64 clocks each on a warp; four
 // chunks a level and more keep the four FP64 pipes (6 or 7 such operations a
 // chunk) half busy.  Double-single: issue slots, about 130 FP32 operations a
@@ -521,7 +521,8 @@ k_sweep_rec(SweepArgs a, const T *__restrict__ in, T *out)
 // Warps: rows in FP64 wait for their level (20 or 24 warps gain nothing over
 // 16); a chain chunk is a long run of dependent FP32 operations, so the narrow
 // ones, whose registers allow it, take 24 (2048x1024, 32 blocks: 667 us an
-// application with 16, 586 with 20, 554 with 24).
+// application with 16, 586 with 20, 554 with 24 before their chunks lay side by
+// side, 448 now).
 __host__ __device__ constexpr int df_warps(bool cs, int w) { return cs && w <= 4 ? 24 : 16; }
 
 // Ring values: polled loads, stores, the mark.
@@ -639,7 +640,7 @@ __device__ __forceinline__ bool sweep_run(const SweepArgs &a, const T *__restric
                                           unsigned long long *full, int *failed, int *prog)
 {
 	typedef SweepRec<T, UPPER, CS, W> Rec;
-	const unsigned mask = (unsigned)a.ring - 1, rb = smem_u32(sm), zero = rb + (unsigned)a.ring * (unsigned)sizeof(T);
+	const unsigned rb = smem_u32(sm), zero = rb + (unsigned)a.ring * (unsigned)sizeof(T);
 	const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, D = a.D, nw = blockDim.x >> 5;
 	const int sb0 = a.chunk_sb[blockIdx.x], cnt = a.chunk_sb[blockIdx.x + 1] - sb0;
 	unsigned char *stages = sm + (((unsigned)al16((a.ring + 1) * sizeof(T)) + 2 * DF_BARS * 8 + 127) & ~127u) +
@@ -672,27 +673,27 @@ __device__ __forceinline__ bool sweep_run(const SweepArgs &a, const T *__restric
 	};
 	int tb = 0;
 	if (!CS) { m = meta(lane); mn = meta(32 + lane); }
+	// chain programs: whole chunks, one after the other
+	const unsigned char *gp = a.prog + (long long)(sb0 + warp) * a.bvo;
+	const T *ip = in + 32LL * (sb0 + warp);
 	auto issue = [&](int turn, int s) {                   // turn's chunk into stage s (turns in order)
-		long long off;
-		int len, p0, vb;
-		if (CS) {                                         // whole chunks, one after the other
-			const int i = sb0 + warp + turn * nw;
-			len = a.bvo; off = (long long)i * len; p0 = 32 * i; vb = 32 * (int)sizeof(T);
-		} else {
+		int len = a.bvo, vb = 32 * (int)sizeof(T);
+		if (!CS) {
 			if (turn == tb + 32) { tb += 32; m = mn; mn = meta(tb + 32 + lane); }
 			const int k = turn - tb;
-			off = __shfl_sync(0xffffffffu, m.off, k);
+			gp = a.prog + __shfl_sync(0xffffffffu, m.off, k);
+			ip = in + __shfl_sync(0xffffffffu, m.p0, k);
 			len = __shfl_sync(0xffffffffu, m.len, k);
-			p0 = __shfl_sync(0xffffffffu, m.p0, k);
 			vb = __shfl_sync(0xffffffffu, m.vb, k);
 		}
 		if (lane == 0) {
 			unsigned char *dst = stages + (unsigned)s * (unsigned)a.stage_bytes;
 			fence_proxy_async();
 			mbar_expect_tx(&full[s], (unsigned)(len + vb));
-			bulk_g2s(dst, a.prog + off, (unsigned)len, &full[s]);
-			bulk_g2s(dst + (unsigned)a.bvo, in + p0, (unsigned)vb, &full[s]);
+			bulk_g2s(dst, gp, (unsigned)len, &full[s]);
+			bulk_g2s(dst + (unsigned)a.bvo, ip, (unsigned)vb, &full[s]);
 		}
+		if (CS) { gp += (long long)nw * a.bvo; ip += 32 * nw; }
 	};
 	const int turns = warp < cnt ? (cnt - warp + nw - 1) / nw : 0;
 	int issued = 0, waited = 0;
@@ -703,6 +704,10 @@ __device__ __forceinline__ bool sweep_run(const SweepArgs &a, const T *__restric
 	int s = 0, known = -DF_DONE;
 	unsigned ph = 0;
 	bool fail = false;
+	// byte offsets of the chunk's slot and of the one it marks
+	const unsigned bytes = (unsigned)a.ring * (unsigned)sizeof(T) - 1, step = 32u * (unsigned)nw * (unsigned)sizeof(T);
+	unsigned pos = (32u * (unsigned)warp + (unsigned)lane) * (unsigned)sizeof(T) & bytes,
+	         next = (pos + 32u * (unsigned)(a.look + 1) * (unsigned)sizeof(T)) & bytes;
 	for (int t = 0; t < turns && !fail; t++) {
 		const int c = warp + t * nw;
 		if (!mbar_wait_or_fail(&full[s], ph, vfailed)) { fail = true; break; }
@@ -772,9 +777,10 @@ __device__ __forceinline__ bool sweep_run(const SweepArgs &a, const T *__restric
 			}
 		}
 		if (on) y = ring_value(y);
-		const unsigned pos = (unsigned)(32 * c + lane), next = pos + 32u * (unsigned)(a.look + 1);
-		if (on) ring_st(rb + (pos & mask) * (unsigned)sizeof(T), y);
-		ring_st(rb + (next & mask) * (unsigned)sizeof(T), ring_mark<T>());
+		if (on) ring_st(rb + pos, y);
+		ring_st(rb + next, ring_mark<T>());
+		pos = (pos + step) & bytes;
+		next = (next + step) & bytes;
 		__syncwarp();
 		if (lane == 0) st_release_cta(&prog[warp], c + nw);
 		if (on && cur.i[W] >= 0) out[cur.i[W]] = y;
