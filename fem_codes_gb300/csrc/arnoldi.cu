@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(32) k_givens(double *H, int ldh, double *cs, d
 {
 	if (!st->active) return;
 	extern __shared__ double sh[];
-	double *hc = work ? work : sh, *pre = sh + kmax + 1, *neg = pre + kmax + 1, *run = neg + kmax + 1;
+	double *hc = work ? work : sh, *pre = hc + kmax + 1, *neg = pre + kmax + 1, *run = neg + kmax + 1;
 	for (int j = threadIdx.x; j <= i; j += 32) hc[j] = H[j * ldh + i];
 	__syncwarp();
 	const double hii = rotate_column(hc, pre, neg, run, cs, sn, H, ldh, i);
