@@ -209,6 +209,7 @@ def load(build_if_needed: bool = True) -> ctypes.CDLL:
         "femgpu_euler_solve": [_vp, _vp, _vp, _ip],
         "femgpu_euler_csr": [_vp, _vp, _vp, _vp, _vp, _vp],
         "femgpu_euler_set_amg": [_vp, _vp],
+        "femgpu_euler_set_wait": [_vp, ctypes.c_int],
         "femgpu_euler_solve_dev": [_vp, _ip],
         "femgpu_euler_predictor": [_vp, _vp, ctypes.c_int, _vp, _vp],
         "femgpu_euler_predictor_dev": [_vp, ctypes.c_int, _vp],
@@ -233,6 +234,7 @@ def load(build_if_needed: bool = True) -> ctypes.CDLL:
         "femgpu_ns_solve": [_vp, _vp, _vp, _ip],
         "femgpu_ns_set_tol": [_vp, ctypes.c_double],
         "femgpu_ns_set_amg": [_vp, _vp],
+        "femgpu_ns_set_wait": [_vp, ctypes.c_int],
         "femgpu_ns_newton": [_vp, ctypes.c_int, _vp, _vp, _vp, _vp, _vp],
         "femgpu_ns_csr": [_vp, _vp, _vp, _vp, _vp],
     }.items():
@@ -265,6 +267,7 @@ def load(build_if_needed: bool = True) -> ctypes.CDLL:
         "femgpu_transport_set_learned": [_vp, _vp],
         "femgpu_amg_create": [ctypes.POINTER(_vp), ctypes.c_int, ctypes.c_double, ctypes.c_double, ctypes.c_int],
         "femgpu_amg_set_stream": [_vp, _vp],
+        "femgpu_amg_set_wait": [_vp, ctypes.c_int],
         "femgpu_amg_setup": [_vp, ctypes.c_int, _vp, _vp, _vp],
         "femgpu_amg_levels": [_vp],
         "femgpu_amg_level": [_vp, ctypes.c_int, _vp, _vp, _vp, _vp, _vp],
@@ -702,7 +705,7 @@ class SSTransport:
         return dict(u=uh[:S * n], t=th[:n], ncorr=nc[:S * n], iters=it[:S * n])
 
     def set_sweep_wait(self, spins=-1):
-        """Bound on a sweep warp's wait for its dependencies (-1: default);
+        """Bound on the waits inside the context's kernels (-1: the defaults);
         also clears the context's device error word."""
         self._check(self._L.femgpu_transport_set_sweep_wait(self._h, int(spins)), "set_sweep_wait")
 
@@ -775,6 +778,10 @@ class AMG:
     def _check(self, rc, where):
         if rc:
             raise FemGpuError(rc, where)
+
+    def set_wait(self, polls=-1):
+        """Bound on the SOR sweeps' waits (-1: the default)."""
+        self._check(self._L.femgpu_amg_set_wait(self._h, int(polls)), "amg_set_wait")
 
     def setup(self, IA, JA, AA):
         IA, JA, AA = _i32(IA), _i32(JA), _f64(AA)
@@ -914,6 +921,11 @@ class Euler:
         of a CSR context (hierarchy rebuilt at every precond_setup)."""
         self._amg = amg
         self._check(self._L.femgpu_euler_set_amg(self._h, amg.handle), "set_amg")
+
+    def set_wait(self, spins=-1):
+        """Bound on the waits inside the context's kernels (-1: the defaults);
+        also clears the context's device error words."""
+        self._check(self._L.femgpu_euler_set_wait(self._h, int(spins)), "set_wait")
 
     def scaling(self, want_matrix=False):
         """FemFunctions->scaling = Block_scaling_EBE after a Build: returns
@@ -1084,12 +1096,17 @@ class NavierStokes:
         self._check(self._L.femgpu_ns_precond_setup(self._h, _ptr(F)), "precond_setup")
         return F
 
-
     def set_amg(self, amg):
         """Use an :class:`AMG` context as the FEMGPU_PREC_AMG preconditioner
         of a CSR context (hierarchy rebuilt at every precond_setup)."""
         self._amg = amg
         self._check(self._L.femgpu_ns_set_amg(self._h, amg.handle), "set_amg")
+
+    def set_wait(self, spins=-1):
+        """Bound on the waits inside the context's kernels (-1: the defaults);
+        also clears the context's device error words."""
+        self._check(self._L.femgpu_ns_set_wait(self._h, int(spins)), "set_wait")
+
     def solver(self, B=None):
         BB = None if B is None else _f64(B)
         X = np.zeros(self.neq + 1)

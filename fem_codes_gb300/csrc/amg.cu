@@ -55,6 +55,7 @@ struct SorArgs {
 	fg_ticket *tk;
 	int *err;
 	const int *active;
+	int poll0;                    // BOUND: fg_poll0
 };
 
 // SOR_relax / SOR_relax_rev, L lanes per row update (the row's entries side by
@@ -62,7 +63,9 @@ struct SorArgs {
 // not there yet polls it again whenever any entry of the warp is waited for, so
 // a row whose last values come together pays one trip through L2, not one for
 // each.  The row's sum runs over the lanes in CSR order as far as the values go.
-template <int L>
+// BOUND: the waits' bound is the context's own (as an argument of every launch
+// it costs 0.6 % of a cycle).
+template <int L, bool BOUND>
 __global__ void __launch_bounds__(kSorThreads) k_sor(SorArgs a)
 {
 	if (skip(a.active)) return;
@@ -95,7 +98,7 @@ __global__ void __launch_bounds__(kSorThreads) k_sor(SorArgs a)
 			for (int k = 0; k < L; k++) {
 				if (base + k >= most) break;                      // uniform
 				if (!__all_sync(0xffffffffu, there >> k & 1u)) {
-					for (int it = 0;; it++) {
+					for (int it = BOUND ? a.poll0 : 0;; it++) {
 						if (!fg_keep_polling(it, a.tk, a.err)) return;
 						if (x == FG_UNSET) x = fg_ld_poll(&src[c]);
 						there = __ballot_sync(0xffffffffu, x != FG_UNSET) >> l0;
@@ -108,7 +111,7 @@ __global__ void __launch_bounds__(kSorThreads) k_sor(SorArgs a)
 				if (used >> k & 1u) sum = s;
 			}
 		}
-		for (int it = 0;; it++) {
+		for (int it = BOUND ? a.poll0 : 0;; it++) {
 			const bool w = own == FG_UNSET;
 			if (!__any_sync(0xffffffffu, w)) break;
 			if (!fg_keep_polling(it, a.tk, a.err)) return;
@@ -204,12 +207,16 @@ int sor(const femgpu_amg *g, const fg_amg_level *L, const double *in, double *z,
 		const fg_amg_sched *S = reverse ? &L->bw[two] : &L->fw[two];
 		const int lanes = L->longest <= 8 ? 8 : (L->longest <= 16 ? 16 : 32), rows = 32 / lanes;
 		SorArgs a = { L->ptr, L->col, L->val, L->diag, L->rdiag, L->f, cur, two ? mid : end, end, S->item,
-		              (unsigned)(S->nitem / rows), reverse, g->omega != 1.0, g->omega, q, g->err, active };
+		              (unsigned)(S->nitem / rows), reverse, g->omega != 1.0, g->omega, q, g->err, active,
+		              fg_poll0(g->wait1) };
 		const int per = kSorThreads / 32 * rows, want = (int)(((long long)kSorAhead * S->wide + per - 1) / per);
 		const int grid = want < 1 ? 1 : (want > 4 * FG_SMS ? 4 * FG_SMS : want);
-		if (lanes == 8) k_sor<8><<<grid, kSorThreads, 0, g->stream>>>(a);
-		else if (lanes == 16) k_sor<16><<<grid, kSorThreads, 0, g->stream>>>(a);
-		else k_sor<32><<<grid, kSorThreads, 0, g->stream>>>(a);
+#define SOR(L) do { if (g->wait1) k_sor<L, true><<<grid, kSorThreads, 0, g->stream>>>(a); \
+	else k_sor<L, false><<<grid, kSorThreads, 0, g->stream>>>(a); } while (0)
+		if (lanes == 8) SOR(8);
+		else if (lanes == 16) SOR(16);
+		else SOR(32);
+#undef SOR
 		cur = end;
 	}
 	*out = (double *)cur;

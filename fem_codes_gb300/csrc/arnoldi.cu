@@ -149,6 +149,7 @@ struct OrthArgs {
 	fg_ticket *tk;                        // abort word
 	fg_status *st;
 	int *step;
+	int poll0;                            // fg_poll0
 };
 
 __device__ __forceinline__ void reset_next(const OrthArgs &a)
@@ -161,19 +162,19 @@ __device__ __forceinline__ void reset_next(const OrthArgs &a)
 // all there on return (a warp); false when the wait gave up.
 template <int NQ>
 __device__ __forceinline__ bool poll_words(unsigned long long (&x)[NQ], const double *slot, int first, int stride, int end,
-                                           fg_ticket *tk, int *err)
+                                           const OrthArgs &a)
 {
 #pragma unroll
 	for (int q = 0; q < NQ; q++) x[q] = first + q * stride < end ? fg_ld_poll(&slot[first + q * stride]) : 0ull;
-	for (int it = 0;; it++) {
+	for (int it = a.poll0;; it++) {
 		bool w = false;
 #pragma unroll
 		for (int q = 0; q < NQ; q++) w |= x[q] == FG_UNSET;
 		if (!__any_sync(0xffffffffu, w)) return true;
-		if (!fg_keep_polling(it, tk, err)) return false;
 #pragma unroll
 		for (int q = 0; q < NQ; q++)
 			if (x[q] == FG_UNSET) x[q] = fg_ld_poll(&slot[first + q * stride]);
+		if (!fg_keep_polling(it, a.tk, &a.st->err)) return false;
 	}
 }
 
@@ -199,7 +200,7 @@ __device__ __forceinline__ bool block_total(const double *slot, int nb, const Or
 	double v = 0.0;
 	if (32 * warp < nb) {                                 // (uniform; the others' sums are zeros)
 		unsigned long long x[NQ];
-		const bool ok = poll_words<NQ>(x, slot, threadIdx.x, OR_TPB, nb, a.tk, &a.st->err);
+		const bool ok = poll_words<NQ>(x, slot, threadIdx.x, OR_TPB, nb, a);
 #pragma unroll
 		for (int q = 0; q < NQ; q++) if (q == 0 || q * OR_TPB < nb) v += __longlong_as_double((long long)x[q]);
 		v = fg_warp_sum(v);
@@ -314,7 +315,7 @@ __global__ void __launch_bounds__(OR_TPB) k_orth_cgs(OrthArgs a)
 				const double *res = a.slot + p * plen + (size_t)m * nvb;
 				for (int j0 = 0; j0 < m; j0 += 32) {
 					unsigned long long x[1];
-					if (!poll_words<1>(x, res, j0 + lane, 32, m, a.tk, &a.st->err)) break;
+					if (!poll_words<1>(x, res, j0 + lane, 32, m, a)) { fail = 1; break; }
 					const double t = __longlong_as_double((long long)x[0]);
 					if (j0 + lane < m) hc[j0 + lane] = p ? hc[j0 + lane] + t : t;
 				}
@@ -375,7 +376,7 @@ __global__ void __launch_bounds__(OR_TPB) k_orth_cgs(OrthArgs a)
 		// product j is added up by block j (mod G), a warp each, as k_mdot_fin does
 		for (int j = blockIdx.x + warp * a.G; j < m; j += 8 * a.G) {
 			unsigned long long x[10];
-			if (!poll_words<10>(x, part + (size_t)j * nvb, lane, 32, nvb, a.tk, &a.st->err)) fail = 1;
+			if (!poll_words<10>(x, part + (size_t)j * nvb, lane, 32, nvb, a)) fail = 1;
 			double t = 0.0;
 #pragma unroll
 			for (int y = 0; y < 10; y++) if (32 * y < nvb) t += __longlong_as_double((long long)x[y]);
@@ -384,7 +385,7 @@ __global__ void __launch_bounds__(OR_TPB) k_orth_cgs(OrthArgs a)
 		}
 		for (int j0 = 32 * warp; j0 < m; j0 += OR_TPB) {
 			unsigned long long x[1];
-			if (!poll_words<1>(x, res, j0 + lane, 32, m, a.tk, &a.st->err)) fail = 1;
+			if (!poll_words<1>(x, res, j0 + lane, 32, m, a)) fail = 1;
 			if (j0 + lane < m) hs[j0 + lane] = __longlong_as_double((long long)x[0]);
 		}
 		__syncthreads();
@@ -490,6 +491,7 @@ extern "C" int fg_kry_orth(const fg_krylov *k, int i, int passes)
 	a.next = k->orth + ((i + 1) & 1) * half;
 	a.nnext = (long long)orth_words(i + 2, a.nvb, passes == 0);
 	a.tk = (fg_ticket *)orth_tail(k);
+	a.poll0 = fg_poll0(k->wait1);
 	const int nv = a.nvb > a.G ? 2 : 1, f = nv - 1 + (k->n > OR_VB * OR_TPB ? 1 : 0);
 	static void *const mgs[3] = { (void *)k_orth_mgs<1, 1>, (void *)k_orth_mgs<2, 1>, (void *)k_orth_mgs<2, 2> };
 	static void *const cgs[3] = { (void *)k_orth_cgs<1, 1>, (void *)k_orth_cgs<2, 1>, (void *)k_orth_cgs<2, 2> };

@@ -50,6 +50,7 @@ struct femgpu_amg {
 	void *ticket;                /* [nticket] fg_ticket, one per SOR launch of a cycle */
 	int nticket;
 	int *err;                    /* FEMGPU_E_TIMEOUT after a wait that ran out */
+	int wait1;                   /* 1 + bound of a wait, in polls; 0: default  */
 	cudaStream_t stream, own_stream;
 };
 

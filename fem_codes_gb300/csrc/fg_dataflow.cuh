@@ -18,7 +18,11 @@
 #include "fg_common.cuh"
 
 #define FG_UNSET 0xffffffffffffffffull
-#define FG_POLL_LIMIT (1 << 22)       // polls of one wait (about 1.5 s)
+#define FG_POLL_LIMIT (1 << 22)       // polls of one wait (about 1.5 s) unless the context says otherwise
+
+// A context's bound on a wait (wait1 = bound + 1, 0 the default) as the count a
+// wait starts at, so that the loops compare with a constant.
+static inline int fg_poll0(int wait1) { return wait1 > 0 ? FG_POLL_LIMIT - (wait1 - 1) : 0; }
 
 // Control words of one launch, zeroed before it: next ticket, abort.
 struct fg_ticket { unsigned next, abort; };
@@ -49,8 +53,8 @@ __device__ __forceinline__ unsigned fg_take(fg_ticket *tk, unsigned end)
 	return __shfl_sync(0xffffffffu, t, 0);
 }
 
-// One more poll of a wait (the same count in every lane): false when the
-// bound is reached or another warp gave up.
+// One more poll of a wait (the same count in every lane, from fg_poll0 on):
+// false when the bound is reached or another warp gave up.
 __device__ __forceinline__ bool fg_keep_polling(int it, fg_ticket *tk, int *err)
 {
 	if (it >= FG_POLL_LIMIT) {

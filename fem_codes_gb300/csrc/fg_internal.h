@@ -147,6 +147,7 @@ typedef struct fg_krylov {
 	int dsv;                        /* FGMRES: Arnoldi basis in double-single */
 	double *orth;                   /* device-wide sums of the one-launch steps
 	                                 * and scratch (fg_kry_orth_bytes)        */
+	int wait1;                      /* 1 + bound of those steps' waits; 0: default */
 	/* FGMRES look-ahead (la_s != NULL): the preconditioner of the next step
 	 * runs on the raw operator output la_w while the Gram-Schmidt of this
 	 * step runs on la_s; la_t [ldv] the combination of the stored
@@ -216,7 +217,7 @@ struct femgpu_transport {
 	float *invDiag32;
 	fg_ilu ilu;
 	fg_ilu_sweeps sweeps;
-	int sweep_wait1;                /* 1 + dependency-wait bound; 0: default */
+	int sweep_wait1;                /* 1 + bound of the kernels' waits; 0: default */
 	/* the CSR matrix in 32-row slices (SELL-32) for the products: entry j of
 	 * row r at sell_base[r/32] + 32 j + r%32; the assembly writes the values */
 	long long *sell_base;

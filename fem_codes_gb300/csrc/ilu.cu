@@ -958,7 +958,7 @@ __device__ __forceinline__ unsigned fac_code(uint2 c, int k) { return ((k < 4 ? 
 template <int L>
 __global__ void __launch_bounds__(FAC_TPB)
 k_ilu0_factor_df(const double *__restrict__ AA, const int4 *__restrict__ head, const int2 *__restrict__ grp,
-                 const uint2 *__restrict__ pos, int nslot, double *LU, double *Dinv, fg_ticket *tk, int *err)
+                 const uint2 *__restrict__ pos, int nslot, double *LU, double *Dinv, fg_ticket *tk, int *err, int poll0)
 {
 	constexpr int R = 32 / L, NB = L / 8;
 	const int lane = threadIdx.x & 31, q = lane & (L - 1), l0 = lane & ~(L - 1);
@@ -995,13 +995,13 @@ k_ilu0_factor_df(const double *__restrict__ AA, const int4 *__restrict__ head, c
 					const int from = own ? l0 + __ffs(own) - 1 : lane;
 					// everything still missing is polled again together: operands
 					// that come at the same time cost one trip, not one each
-					for (int it = 0;; it++) {
+					for (int it = poll0;; it++) {
 						if (!__any_sync(0xffffffffu, u[k] == FG_UNSET || (q == gi && piv == FG_UNSET))) break;
-						if (!fg_keep_polling(it, tk, err)) return;
 						if (piv == FG_UNSET) piv = fg_ld_poll(&Dinv[g.x]);
 #pragma unroll
 						for (int m = k; m < 8; m++)
 							if (u[m] == FG_UNSET) u[m] = fg_ld_poll(at[m]);
+						if (!fg_keep_polling(it, tk, err)) return;
 					}
 					const double lq = __dmul_rn(__shfl_sync(0xffffffffu, v, from),
 					                            __shfl_sync(0xffffffffu, __longlong_as_double((long long)piv), l0 + gi));
@@ -2076,7 +2076,7 @@ extern "C" int fg_ilu0_factor(femgpu_transport *t)
 	fg_ticket *tk = (fg_ticket *)S.fac_ticket;
 	k_ilu0_factor_init<<<fg_grid(t->ilu.nnz), FG_TPB, 0, s>>>(t->ilu.LU, t->ilu.nnz, t->ilu.Dinv, t->neq, tk);
 #define FAC_RUN(L) k_ilu0_factor_df<L><<<grid, FAC_TPB, 0, s>>>(A, (const int4 *)S.fac_head, (const int2 *)S.fac_grp, \
-	(const uint2 *)S.fac_pos, S.fac_nslot, t->ilu.LU, t->ilu.Dinv, tk, &t->st->err)
+	(const uint2 *)S.fac_pos, S.fac_nslot, t->ilu.LU, t->ilu.Dinv, tk, &t->st->err, fg_poll0(t->sweep_wait1))
 	if (S.fac_lanes == 8) FAC_RUN(8);
 	else if (S.fac_lanes == 16) FAC_RUN(16);
 	else FAC_RUN(32);

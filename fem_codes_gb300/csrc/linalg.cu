@@ -1199,6 +1199,7 @@ extern "C" void fg_transport_krylov(femgpu_transport *t, fg_krylov *k, fg_linop 
 	k->n = t->neq; k->kmax = t->kmax; k->nblk = red_grid(t); k->ldv = t->ldv; k->stream = t->stream;
 	k->V = t->V; k->H = t->H; k->cs = t->cs; k->sn = t->sn; k->ge = t->ge; k->gy = t->gy;
 	k->Z = t->Z; k->Z32 = t->Z32; k->partials = t->partials; k->orth = t->orth; k->st = t->st; k->st_host = t->st_host;
+	k->wait1 = t->sweep_wait1;
 	op->ctx = t;
 	op->matvec = tr_matvec;
 	op->precond = tr_precond;

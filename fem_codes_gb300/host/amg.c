@@ -593,6 +593,14 @@ int femgpu_amg_set_stream(femgpu_amg *g, void *stream)
 	return 0;
 }
 
+int femgpu_amg_set_wait(femgpu_amg *g, int polls)
+{
+	if (!g) return FEMGPU_E_ARG;
+	CK(cudaStreamSynchronize(g->stream));
+	g->wait1 = fgh_wait1(polls);
+	return 0;
+}
+
 /* Device copy of a smoothed level: CSR, diagonal and its inverse, SOR
  * schedules; f except on level 0 (the caller's vector). */
 static int upload_level(femgpu_amg *g, int l, fg_amg_level *D, const hmat *A)

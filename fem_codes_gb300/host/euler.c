@@ -251,6 +251,11 @@ int femgpu_euler_set_slip(femgpu_euler *c, const int *slip, const double *cs, co
 	return rc;
 }
 
+int femgpu_euler_set_wait(femgpu_euler *c, int spins)
+{
+	return c ? fgh_set_wait(&c->kry, &c->csr, spins) : FEMGPU_E_ARG;
+}
+
 int femgpu_euler_set_amg(femgpu_euler *c, femgpu_amg *g)
 {
 	if (!c || !g || c->o.precond != FEMGPU_PREC_AMG) return FEMGPU_E_ARG;

@@ -50,6 +50,12 @@ int fgh_kry_cycles(const struct fg_krylov *k, const struct fg_linop *op, const d
 int fgh_kry_begin(const struct fg_krylov *k, double eps);
 int fgh_kry_cycle(const struct fg_krylov *k, const struct fg_linop *op, const double *B, double *X, int kind,
                   int cycle);
+/* The encoding of a wait bound (fg_krylov.wait1), and a context's set_wait:
+ * the bound of the solver's and the CSR system's kernels (b may be NULL), their
+ * error words cleared. */
+struct fg_blockcsr;
+int fgh_wait1(int spins);
+int fgh_set_wait(struct fg_krylov *k, struct fg_blockcsr *b, int spins);
 /* ||B||^2 on the device, returned to the host (synchronises the stream). */
 int fgh_kry_dot_host(const struct fg_krylov *k, const double *a, const double *b, int n, double *out);
 
@@ -63,7 +69,6 @@ int fgh_iluk_pattern(int n, const int *IA, const int *JA, int p, int **fIA, int 
  * context's lm and incidence lists and, when ilu0, the ILU(0) structure of
  * a transport context (solver: the Krylov solver its sweeps serve,
  * ilu_blocks as femgpu_transport_opts.ilu_blocks). */
-struct fg_blockcsr;
 struct femgpu_ebe;
 int fgh_blockcsr_create(struct fg_blockcsr *b, int M, const struct femgpu_ebe *ebe, int nel, int neq,
                         cudaStream_t s, int ilu0, int solver, int ilu_blocks);

@@ -53,6 +53,25 @@ void fgh_kry_free(fg_krylov *k)
 	memset(k, 0, sizeof *k);
 }
 
+int fgh_wait1(int spins)
+{
+	return spins < 0 ? 0 : (spins == 0x7fffffff ? spins : spins + 1);
+}
+
+int fgh_set_wait(fg_krylov *k, fg_blockcsr *b, int spins)
+{
+	CK(cudaStreamSynchronize(k->stream));
+	k->wait1 = fgh_wait1(spins);
+	CK(cudaMemsetAsync(&k->st->err, 0, sizeof(int), k->stream));
+	k->st_host->err = 0;
+	if (b && b->ilu) {
+		b->ilu->sweep_wait1 = k->wait1;
+		CK(cudaMemsetAsync(&b->ilu->st->err, 0, sizeof(int), k->stream));
+	}
+	CK(cudaStreamSynchronize(k->stream));
+	return 0;
+}
+
 static int sync_status(const fg_krylov *k)
 {
 	CK(cudaMemcpyAsync(k->st_host, k->st, sizeof(fg_status), cudaMemcpyDeviceToHost, k->stream));

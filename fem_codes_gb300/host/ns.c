@@ -272,6 +272,11 @@ static int solve(femgpu_ns *c, const double *B, double *X, int *iters)
 	return rc;
 }
 
+int femgpu_ns_set_wait(femgpu_ns *c, int spins)
+{
+	return c ? fgh_set_wait(&c->kry, &c->csr, spins) : FEMGPU_E_ARG;
+}
+
 int femgpu_ns_set_amg(femgpu_ns *c, femgpu_amg *g)
 {
 	if (!c || !g || c->o.precond != FEMGPU_PREC_AMG) return FEMGPU_E_ARG;

@@ -410,7 +410,7 @@ int femgpu_transport_set_sweep_wait(femgpu_transport *t, int spins)
 {
 	if (!t) return FEMGPU_E_ARG;
 	CK(cudaStreamSynchronize(t->stream));
-	t->sweep_wait1 = spins < 0 ? 0 : (spins == 0x7fffffff ? spins : spins + 1);
+	t->sweep_wait1 = fgh_wait1(spins);
 	CK(cudaMemsetAsync(&t->st->err, 0, sizeof(int), t->stream));
 	t->st_host->err = 0;
 	CK(cudaStreamSynchronize(t->stream));

@@ -142,13 +142,16 @@ int femgpu_transport_ilu_blocks(const femgpu_transport *ctx, int *first, int cap
  * FEMGPU_E_NOT_BUILT before the ILU(0) structure exists. */
 int femgpu_transport_ilu_chain(const femgpu_transport *ctx, int *levels);
 
-/* Bound, in spins, on a sweep warp's wait for the rows its own rows depend
- * on (spins < 0: the default, 2^24); a warp that gives up records
- * FEMGPU_E_TIMEOUT, the other warps of its block stop, the block waits for
- * the copies it has in flight (that wait keeps the default bound) and
- * returns, and the call reports the error.  0 makes every sweep time out at
- * its first dependent row, the way a test reaches the error path.  Also
- * clears the context's device error word, so the context is usable again. */
+/* Bound, in spins, on the waits inside the context's kernels: a sweep warp's
+ * for the rows its own rows depend on, a factorisation warp's for the rows its
+ * row reads, a one-launch Arnoldi step's for the sums of the other blocks
+ * (spins < 0: the defaults, 2^24, 2^22 and 2^22).  A warp that gives up records
+ * FEMGPU_E_TIMEOUT, the other warps of its block (of its launch, outside the
+ * sweeps) stop, a sweep's block waits for the copies it has in flight (that
+ * wait keeps the default bound) and returns, and the call reports the error.
+ * 0 makes every kernel time out at its first wait, the way a test reaches the
+ * error path.  Also clears the context's device error word, so the context is
+ * usable again. */
 int femgpu_transport_set_sweep_wait(femgpu_transport *ctx, int spins);
 
 /* The same cut for a CSR pattern on the host, no device needed: returns the
@@ -636,6 +639,12 @@ int femgpu_transport_set_amg(femgpu_transport *t, femgpu_amg *ctx);
  * its own stream when the context is destroyed, so ctx must outlive it. */
 int femgpu_ns_set_amg(femgpu_ns *ns, femgpu_amg *ctx);
 int femgpu_euler_set_amg(femgpu_euler *eu, femgpu_amg *ctx);
+/* femgpu_transport_set_sweep_wait for the other contexts; an AMG context's
+ * bound (its SOR sweeps' polls for the rows they read, default 2^22) is its
+ * own, whoever uses it. */
+int femgpu_ns_set_wait(femgpu_ns *ns, int spins);
+int femgpu_euler_set_wait(femgpu_euler *eu, int spins);
+int femgpu_amg_set_wait(femgpu_amg *ctx, int polls);
 /* Slip walls of the Euler SUPG build (Build_M_K_F_SUPG.c:1044-1056 with
  * rotation.c:3-43): slip [nnodes] != 0 marks the nodes the reference gives
  * v1Type = -1; their rows and columns of each element matrix and their
