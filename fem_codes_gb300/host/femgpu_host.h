@@ -50,6 +50,10 @@ int fgh_kry_cycles(const struct fg_krylov *k, const struct fg_linop *op, const d
 int fgh_kry_begin(const struct fg_krylov *k, double eps);
 int fgh_kry_cycle(const struct fg_krylov *k, const struct fg_linop *op, const double *B, double *X, int kind,
                   int cycle);
+/* Status block st to its host mirror (synchronises): the first device-side
+ * error since the last report, which clears it. */
+struct fg_status;
+int fgh_status(struct fg_status *st, struct fg_status *host, cudaStream_t s);
 /* The encoding of a wait bound (fg_krylov.wait1), and a context's set_wait:
  * the bound of the solver's and the CSR system's kernels (b may be NULL), their
  * error words cleared. */

@@ -72,15 +72,21 @@ int fgh_set_wait(fg_krylov *k, fg_blockcsr *b, int spins)
 	return 0;
 }
 
-static int sync_status(const fg_krylov *k)
+int fgh_status(fg_status *st, fg_status *host, cudaStream_t s)
 {
-	CK(cudaMemcpyAsync(k->st_host, k->st, sizeof(fg_status), cudaMemcpyDeviceToHost, k->stream));
-	CK(cudaStreamSynchronize(k->stream));
-	if (k->st_host->err) {
-		fgh_set_error("device reported error %d", k->st_host->err);
-		return k->st_host->err;
+	CK(cudaMemcpyAsync(host, st, sizeof(fg_status), cudaMemcpyDeviceToHost, s));
+	CK(cudaStreamSynchronize(s));
+	if (host->err) {
+		fgh_set_error("device reported error %d", host->err);
+		CK(cudaMemsetAsync(&st->err, 0, sizeof(int), s));
+		return host->err;
 	}
 	return 0;
+}
+
+static int sync_status(const fg_krylov *k)
+{
+	return fgh_status(k->st, k->st_host, k->stream);
 }
 
 int fgh_kry_begin(const fg_krylov *k, double eps)

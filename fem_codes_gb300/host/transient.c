@@ -120,13 +120,7 @@ int femgpu_transport_build_transient(femgpu_transport *t, const double *u_host, 
 		          : t->o.scheme == FEMGPU_EDE ? 4 * ((size_t)t->nedge + 1) : 9 * (size_t)t->nel;
 		CK(cudaMemcpyAsync(A_host, t->A, sizeof(double) * nA, cudaMemcpyDeviceToHost, t->stream));
 	}
-	CK(cudaStreamSynchronize(t->stream));
-	CK(cudaMemcpy(t->st_host, t->st, sizeof(fg_status), cudaMemcpyDeviceToHost));
-	if (t->st_host->err) {
-		fgh_set_error("device reported error %d", t->st_host->err);
-		return t->st_host->err;
-	}
-	return 0;
+	return fgh_status(t->st, t->st_host, t->stream);
 }
 
 /* Criteria.c:22-38 */

@@ -72,13 +72,7 @@ static int upload(void **dst, const void *src, size_t bytes)
 
 static int sync_err(femgpu_transport *t)
 {
-	CK(cudaMemcpyAsync(t->st_host, t->st, sizeof(fg_status), cudaMemcpyDeviceToHost, t->stream));
-	CK(cudaStreamSynchronize(t->stream));
-	if (t->st_host->err) {
-		fgh_set_error("device reported error %d", t->st_host->err);
-		return t->st_host->err;
-	}
-	return 0;
+	return fgh_status(t->st, t->st_host, t->stream);
 }
 
 /* The SELL-32 layout of the CSR pattern (rows in slices of 32, each slice
