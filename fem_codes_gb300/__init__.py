@@ -268,6 +268,7 @@ def load(build_if_needed: bool = True) -> ctypes.CDLL:
         "femgpu_amg_create": [ctypes.POINTER(_vp), ctypes.c_int, ctypes.c_double, ctypes.c_double, ctypes.c_int],
         "femgpu_amg_set_stream": [_vp, _vp],
         "femgpu_amg_set_wait": [_vp, ctypes.c_int],
+        "femgpu_amg_status": [_vp],
         "femgpu_amg_setup": [_vp, ctypes.c_int, _vp, _vp, _vp],
         "femgpu_amg_levels": [_vp],
         "femgpu_amg_level": [_vp, ctypes.c_int, _vp, _vp, _vp, _vp, _vp],
@@ -810,6 +811,11 @@ class AMG:
 
     def apply_dev(self, q_ptr, z_ptr):
         self._check(self._L.femgpu_amg_apply_dev(self._h, _vp(q_ptr), _vp(z_ptr)), "amg_apply_dev")
+
+    def status(self):
+        """Wait for the device calls so far; the first error among them since
+        the last call (0: none)."""
+        return self._L.femgpu_amg_status(self._h)
 
     def close(self):
         if getattr(self, "_h", None):

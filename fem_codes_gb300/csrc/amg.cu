@@ -185,9 +185,9 @@ inline unsigned blocks(int n) { return (unsigned)((n + kThreads - 1) / kThreads)
 
 // nr SOR sweeps on level L from the iterate `in' (NULL: zero), two to a launch;
 // *out: the last iterate (z when given).  With nr <= 2 the iterates were
-// marked unset when the cycle began.
+// marked unset when the cycle began.  err: where a wait that runs out is told.
 int sor(const femgpu_amg *g, const fg_amg_level *L, const double *in, double *z, int reverse, fg_ticket **tk,
-        const int *active, double **out)
+        const int *active, int *err, double **out)
 {
 	const double *cur = in;
 	for (int left = g->nr; left > 0;) {
@@ -207,7 +207,7 @@ int sor(const femgpu_amg *g, const fg_amg_level *L, const double *in, double *z,
 		const fg_amg_sched *S = reverse ? &L->bw[two] : &L->fw[two];
 		const int lanes = L->longest <= 8 ? 8 : (L->longest <= 16 ? 16 : 32), rows = 32 / lanes;
 		SorArgs a = { L->ptr, L->col, L->val, L->diag, L->rdiag, L->f, cur, two ? mid : end, end, S->item,
-		              (unsigned)(S->nitem / rows), reverse, g->omega != 1.0, g->omega, q, g->err, active,
+		              (unsigned)(S->nitem / rows), reverse, g->omega != 1.0, g->omega, q, err, active,
 		              fg_poll0(g->wait1) };
 		const int per = kSorThreads / 32 * rows, want = (int)(((long long)kSorAhead * S->wide + per - 1) / per);
 		const int grid = want < 1 ? 1 : (want > 4 * FG_SMS ? 4 * FG_SMS : want);
@@ -225,7 +225,7 @@ int sor(const femgpu_amg *g, const fg_amg_level *L, const double *in, double *z,
 
 }  // namespace
 
-extern "C" int fg_amg_vcycle(femgpu_amg *g, const double *q, double *z, const int *active)
+extern "C" int fg_amg_vcycle(femgpu_amg *g, const double *q, double *z, const int *active, int *err)
 {
 	int top = g->nlevels - 1, l, rc;
 	fg_amg_level *lv = g->lv;
@@ -240,16 +240,16 @@ extern "C" int fg_amg_vcycle(femgpu_amg *g, const double *q, double *z, const in
 		k_unset<<<fg_grid(g->narena), kThreads, 0, g->stream>>>(g->arena, g->narena, z, n0, tk, g->nticket, active);
 	for (l = 0; l < top; l += 2) {
 		fg_amg_level *L = &lv[l], *C = &lv[l + 2];
-		if ((rc = sor(g, L, nullptr, nullptr, 0, &tk, active, &L->u))) return rc;
+		if ((rc = sor(g, L, nullptr, nullptr, 0, &tk, active, err, &L->u))) return rc;
 		k_restrict2<<<blocks(L->nc2), kThreads, 0, g->stream>>>(L->ptr, L->col, L->val, L->f, L->u, L->quad,
 		                                                          L->nc2, C->f, active);
 	}
-	if ((rc = sor(g, &lv[top], nullptr, nullptr, 0, &tk, active, &lv[top].u))) return rc;
-	if ((rc = sor(g, &lv[top], lv[top].u, nullptr, 1, &tk, active, &lv[top].u))) return rc;
+	if ((rc = sor(g, &lv[top], nullptr, nullptr, 0, &tk, active, err, &lv[top].u))) return rc;
+	if ((rc = sor(g, &lv[top], lv[top].u, nullptr, 1, &tk, active, err, &lv[top].u))) return rc;
 	for (l = top; l > 0; l -= 2) {
 		fg_amg_level *F = &lv[l - 2];
 		k_prolong2<<<blocks(F->n), kThreads, 0, g->stream>>>(F->agg2, lv[l].u, F->u, F->n, active);
-		if ((rc = sor(g, F, F->u, l == 2 ? z : nullptr, 1, &tk, active, &F->u))) return rc;
+		if ((rc = sor(g, F, F->u, l == 2 ? z : nullptr, 1, &tk, active, err, &F->u))) return rc;
 	}
 	lv[0].f = nullptr;
 	lv[0].u = nullptr;

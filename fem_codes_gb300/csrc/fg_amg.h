@@ -49,14 +49,15 @@ struct femgpu_amg {
 	long long narena;
 	void *ticket;                /* [nticket] fg_ticket, one per SOR launch of a cycle */
 	int nticket;
-	int *err;                    /* FEMGPU_E_TIMEOUT after a wait that ran out */
+	int *err;                    /* [2] errors of the device calls and of the
+	                              * host ones (a solver passes its own word) */
 	int wait1;                   /* 1 + bound of a wait, in polls; 0: default  */
 	cudaStream_t stream, own_stream;
 };
 
 /* z = M^-1 q: one V-cycle (dpa_Vcycle_precond, amg_dpa.c:485-506).  Every
  * kernel is skipped while *active == 0 (active may be NULL). */
-int fg_amg_vcycle(femgpu_amg *g, const double *q, double *z, const int *active);
+int fg_amg_vcycle(femgpu_amg *g, const double *q, double *z, const int *active, int *err);
 
 #ifdef __cplusplus
 }

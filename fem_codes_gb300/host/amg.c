@@ -643,8 +643,8 @@ static int alloc_cycle(femgpu_amg *g)
 		for (int k = 0; k < FG_AMG_NW; k++, at += (g->lv[l].n + 1) & ~1) g->lv[l].w[k] = g->arena + at;
 	g->nticket = (g->nlevels + 1) * ((g->nr + 1) / 2);
 	DM(g->ticket, 8 * (size_t)g->nticket);
-	DM(g->err, sizeof(int));
-	CK(cudaMemsetAsync(g->err, 0, sizeof(int), g->stream));
+	DM(g->err, 2 * sizeof(int));
+	CK(cudaMemsetAsync(g->err, 0, 2 * sizeof(int), g->stream));
 	return 0;
 }
 
@@ -756,8 +756,22 @@ int femgpu_amg_apply_dev(femgpu_amg *g, const double *q, double *z)
 {
 	if (!g || !q || !z) return FEMGPU_E_ARG;
 	if (!g->nlevels) { fgh_set_error("AMG apply before setup"); return FEMGPU_E_NOT_BUILT; }
-	KR(fg_amg_vcycle(g, q, z, NULL));
+	KR(fg_amg_vcycle(g, q, z, NULL, g->err));
 	return 0;
+}
+
+int femgpu_amg_status(femgpu_amg *g)
+{
+	int err = 0;
+	if (!g) return FEMGPU_E_ARG;
+	if (!g->err) return 0;
+	CK(cudaMemcpyAsync(&err, g->err, sizeof(int), cudaMemcpyDeviceToHost, g->stream));
+	CK(cudaStreamSynchronize(g->stream));
+	if (err) {
+		fgh_set_error("device reported error %d", err);
+		CK(cudaMemsetAsync(g->err, 0, sizeof(int), g->stream));
+	}
+	return err;
 }
 
 int femgpu_amg_apply(femgpu_amg *g, const double *q_host, double *z_host)
@@ -770,9 +784,11 @@ int femgpu_amg_apply(femgpu_amg *g, const double *q_host, double *z_host)
 	    (rc = fgh_dmalloc((void **)&z, sizeof(double) * (size_t)n)))
 		return rc;
 	CK(cudaMemcpyAsync(q, q_host, sizeof(double) * (size_t)n, cudaMemcpyHostToDevice, g->stream));
-	rc = femgpu_amg_apply_dev(g, q, z);
+	CK(cudaMemsetAsync(g->err + 1, 0, sizeof(int), g->stream));
+	rc = fg_amg_vcycle(g, q, z, NULL, g->err + 1);
+	if (rc > 0) { fgh_set_error("V-cycle: %s", cudaGetErrorString((cudaError_t)rc)); rc = FEMGPU_E_CUDA; }
 	if (!rc) CK(cudaMemcpyAsync(z_host, z, sizeof(double) * (size_t)n, cudaMemcpyDeviceToHost, g->stream));
-	if (!rc) CK(cudaMemcpyAsync(&err, g->err, sizeof(int), cudaMemcpyDeviceToHost, g->stream));
+	if (!rc) CK(cudaMemcpyAsync(&err, g->err + 1, sizeof(int), cudaMemcpyDeviceToHost, g->stream));
 	CK(cudaStreamSynchronize(g->stream));
 	cudaFree(q);
 	cudaFree(z);

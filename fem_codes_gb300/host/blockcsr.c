@@ -20,7 +20,7 @@
 #define DM(ptr, bytes) do { int r_ = fgh_dmalloc((void **)&(ptr), (bytes)); if (r_) return r_; } while (0)
 
 int fgh_blockcsr_create(fg_blockcsr *b, int M, const femgpu_ebe *ebe, int nel, int neq, cudaStream_t s, int ilu0,
-                        int solver, int ilu_blocks)
+                        int solver, int ilu_blocks, fg_status *st)
 {
 	femgpu_transport *t;
 	int *hIA = NULL, *hJA = NULL, *err = NULL, rc;
@@ -42,8 +42,7 @@ int fgh_blockcsr_create(fg_blockcsr *b, int M, const femgpu_ebe *ebe, int nel, i
 	t->neq = neq; t->nnz = b->nnz;
 	t->IA = b->IA; t->JA = b->JA; t->A = b->AA;
 	t->stream = s;
-	DM(t->st, sizeof(fg_status));
-	CK(cudaMemset(t->st, 0, sizeof(fg_status)));
+	t->st = st;
 	t->ilu.n = neq; t->ilu.nnz = b->nnz;
 	DM(t->ilu.LU, sizeof(double) * ((size_t)b->nnz + 1));
 	DM(t->ilu.Dinv, sizeof(double) * n1);
@@ -67,7 +66,6 @@ void fgh_blockcsr_destroy(fg_blockcsr *b)
 	if (b->amg) femgpu_amg_set_stream(b->amg, NULL);
 	if (t) {
 		if (b->have_ilu) fg_ilu_free(t);
-		if (t->st) cudaFree(t->st);
 		if (t->ilu.LU) cudaFree(t->ilu.LU);
 		if (t->ilu.Dinv) cudaFree(t->ilu.Dinv);
 		free(t);
@@ -92,7 +90,11 @@ int fgh_blockcsr_factor(fg_blockcsr *b, cudaStream_t s)
 	KR(fg_ilu0_factor(b->ilu));
 	CK(cudaMemcpyAsync(&err, &b->ilu->st->err, sizeof(int), cudaMemcpyDeviceToHost, s));
 	CK(cudaStreamSynchronize(s));
-	if (err) { fgh_set_error("ILU(0) factorisation: %d", err); return err; }
+	if (err) {
+		fgh_set_error("ILU(0) factorisation: %d", err);
+		CK(cudaMemsetAsync(&b->ilu->st->err, 0, sizeof(int), s));
+		return err;
+	}
 	return 0;
 }
 

@@ -78,7 +78,8 @@ static int op_precond_ilu(void *ctx, const double *p, double *z, const int *acti
 
 static int op_precond_amg(void *ctx, const double *p, double *z, const int *active)
 {
-	return fg_amg_vcycle(((femgpu_euler *)ctx)->csr.amg, p, z, active);
+	femgpu_euler *c = (femgpu_euler *)ctx;
+	return fg_amg_vcycle(c->csr.amg, p, z, active, &c->kry.st->err);
 }
 
 static void linop(femgpu_euler *c, fg_linop *op)
@@ -141,7 +142,7 @@ static int create(femgpu_euler *c, const femgpu_euler_opts *o, int nnodes, const
 	if (rc) return rc;
 	if (o->scheme == FEMGPU_CSR &&
 	    (rc = fgh_blockcsr_create(&c->csr, 12, c->ebe, nel, neq, c->stream, o->precond == FEMGPU_PREC_ILU0,
-	                              o->solver, o->ilu_blocks))) return rc;
+	                              o->solver, o->ilu_blocks, c->kry.st))) return rc;
 	for (i = 0; i < 4; i++) CK(cudaEventCreate(&c->ev[i]));
 	CK(cudaStreamSynchronize(c->stream));
 	return 0;
@@ -362,7 +363,7 @@ int femgpu_euler_precond_setup_dev(femgpu_euler *c)
 		/* AMG_precond_setup (amg_precond.c:26-100) on the CSR matrix, R := M^-1 R */
 		KR(fgh_blockcsr_amg_setup(&c->csr, c->neq, c->stream));
 		c->have_bd = 1;
-		if (c->o.solver == FEMGPU_PGMRES) KR(fg_amg_vcycle(c->csr.amg, c->R, c->R, NULL));
+		if (c->o.solver == FEMGPU_PGMRES) KR(fg_amg_vcycle(c->csr.amg, c->R, c->R, NULL, &c->kry.st->err));
 		return 0;
 	}
 	if (c->o.precond != FEMGPU_PREC_BLOCKDIAG) return 0;     /* NO_precond_setup */
@@ -380,8 +381,7 @@ int femgpu_euler_precond_setup(femgpu_euler *c, double *R_host)
 	if (R_host)
 		CK(cudaMemcpyAsync(R_host, c->R, sizeof(double) * ((size_t)c->neq + 1), cudaMemcpyDeviceToHost,
 		                   c->stream));
-	CK(cudaStreamSynchronize(c->stream));
-	return 0;
+	return fgh_status(c->kry.st, c->kry.st_host, c->stream);
 }
 
 static int solve(femgpu_euler *c, const double *B, double *X, int *iters)

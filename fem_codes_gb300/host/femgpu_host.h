@@ -72,10 +72,11 @@ int fgh_iluk_pattern(int n, const int *IA, const int *JA, int p, int **fIA, int 
  * element (host/blockcsr.c): the pattern built on the device from the EBE
  * context's lm and incidence lists and, when ilu0, the ILU(0) structure of
  * a transport context (solver: the Krylov solver its sweeps serve,
- * ilu_blocks as femgpu_transport_opts.ilu_blocks). */
+ * ilu_blocks as femgpu_transport_opts.ilu_blocks).  st: the status block of the
+ * solver that the system belongs to, where its kernels put their errors. */
 struct femgpu_ebe;
 int fgh_blockcsr_create(struct fg_blockcsr *b, int M, const struct femgpu_ebe *ebe, int nel, int neq,
-                        cudaStream_t s, int ilu0, int solver, int ilu_blocks);
+                        cudaStream_t s, int ilu0, int solver, int ilu_blocks, struct fg_status *st);
 void fgh_blockcsr_destroy(struct fg_blockcsr *b);
 /* csr_assembly.c per row from the element matrices ebe->A. */
 int fgh_blockcsr_assemble(struct fg_blockcsr *b, int M, const struct femgpu_ebe *ebe, int neq, cudaStream_t s);

@@ -64,10 +64,7 @@ int fgh_set_wait(fg_krylov *k, fg_blockcsr *b, int spins)
 	k->wait1 = fgh_wait1(spins);
 	CK(cudaMemsetAsync(&k->st->err, 0, sizeof(int), k->stream));
 	k->st_host->err = 0;
-	if (b && b->ilu) {
-		b->ilu->sweep_wait1 = k->wait1;
-		CK(cudaMemsetAsync(&b->ilu->st->err, 0, sizeof(int), k->stream));
-	}
+	if (b && b->ilu) b->ilu->sweep_wait1 = k->wait1;
 	CK(cudaStreamSynchronize(k->stream));
 	return 0;
 }

@@ -59,7 +59,8 @@ static int op_precond_ilu(void *ctx, const double *p, double *z, const int *acti
 /* CSR storage: AMG_precond, one V-cycle */
 static int op_precond_amg(void *ctx, const double *p, double *z, const int *active)
 {
-	return fg_amg_vcycle(((femgpu_ns *)ctx)->csr.amg, p, z, active);
+	femgpu_ns *c = (femgpu_ns *)ctx;
+	return fg_amg_vcycle(c->csr.amg, p, z, active, &c->kry.st->err);
 }
 
 static int up(double **dst, const double *src, size_t n)
@@ -95,7 +96,7 @@ static int create(femgpu_ns *c, const femgpu_ns_opts *o, int nnodes, const doubl
 	if (rc) return rc;
 	if (o->scheme == FEMGPU_CSR &&
 	    (rc = fgh_blockcsr_create(&c->csr, 9, c->ebe, c->nel, c->neq, c->stream, o->precond == FEMGPU_PREC_ILU0,
-	                              o->solver, o->ilu_blocks))) return rc;
+	                              o->solver, o->ilu_blocks, c->kry.st))) return rc;
 	CK(cudaStreamSynchronize(c->stream));
 	return 0;
 }
@@ -225,7 +226,7 @@ static int setup_dev(femgpu_ns *c)
 		 * current CSR matrix on the host, then F := M^-1 F */
 		KR(fgh_blockcsr_amg_setup(&c->csr, c->neq, c->stream));
 		c->have_bd = 1;
-		if (c->o.solver == FEMGPU_PGMRES) KR(fg_amg_vcycle(c->csr.amg, c->F, c->F, NULL));
+		if (c->o.solver == FEMGPU_PGMRES) KR(fg_amg_vcycle(c->csr.amg, c->F, c->F, NULL, &c->kry.st->err));
 		return 0;
 	}
 	if (c->o.precond != FEMGPU_PREC_BLOCKDIAG) return 0;
@@ -243,8 +244,7 @@ int femgpu_ns_precond_setup(femgpu_ns *c, double *F_host)
 	if (F_host)
 		CK(cudaMemcpyAsync(F_host, c->F, sizeof(double) * ((size_t)c->neq + 1), cudaMemcpyDeviceToHost,
 		                   c->stream));
-	CK(cudaStreamSynchronize(c->stream));
-	return 0;
+	return fgh_status(c->kry.st, c->kry.st_host, c->stream);
 }
 
 static int solve(femgpu_ns *c, const double *B, double *X, int *iters)

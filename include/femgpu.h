@@ -626,6 +626,11 @@ int femgpu_amg_level(const femgpu_amg *ctx, int l, int *n_nnz, int *IA, int *JA,
 /* z = M^-1 q, one V-cycle (q == z allowed). */
 int femgpu_amg_apply(femgpu_amg *ctx, const double *q_host, double *z_host);
 int femgpu_amg_apply_dev(femgpu_amg *ctx, const double *q, double *z);
+/* Waits for the device calls so far and returns the first error among them
+ * (FEMGPU_E_TIMEOUT: a wait of the SOR sweeps ran out) since the last call, 0
+ * when there was none.  femgpu_amg_apply returns its own cycle's error, a solve
+ * that uses the context the solve's. */
+int femgpu_amg_status(femgpu_amg *ctx);
 /* Use ctx as the FEMGPU_PREC_AMG preconditioner of a CSR transport context
  * (precond_setup rebuilds the hierarchy from the current matrix), or as the
  * fallback of a FEMGPU_PREC_LEARNED context (built when a solve stalls). */
