@@ -112,6 +112,18 @@ __device__ __forceinline__ bool mbar_wait_or_fail(unsigned long long *bar, unsig
 	return false;
 }
 
+// The same for a whole warp, the answer the same in every lane: lanes that saw
+// the failure while others saw the phase end would leave the others at the next
+// warp barrier.
+__device__ __forceinline__ bool mbar_wait_warp(unsigned long long *bar, unsigned parity, volatile int *failed)
+{
+	for (int i = 0; i < SW_WAIT_LIMIT; i++) {
+		if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+		if (__any_sync(0xffffffffu, *failed != 0)) return false;
+	}
+	return false;
+}
+
 __device__ __forceinline__ void fence_proxy_async()
 {
 	asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -319,7 +331,7 @@ k_sweep(SweepArgs a, const T *__restrict__ in, T *out)
 	for (int l = l0; l < l1; l++) {
 		int nsub = 1, j = 0, s0 = s;
 		for (; j < nsub; j++) {
-			bool ok = mbar_wait_or_fail(&full[s], ph, vfailed);
+			bool ok = mbar_wait_warp(&full[s], ph, vfailed);
 			if (!ok) { *vfailed = 1; break; }
 			const unsigned char *st = stages + (unsigned)s * sbytes;
 			const LevHdr h = *(const LevHdr *)st;
@@ -431,7 +443,7 @@ k_sweep_rec(SweepArgs a, const T *__restrict__ in, T *out)
 	for (int l = l0; l < l1; l++) {
 		int nsub = 1, j = 0, s0 = s;
 		for (; j < nsub; j++) {
-			bool ok = mbar_wait_or_fail(&full[s], ph, vfailed);
+			bool ok = mbar_wait_warp(&full[s], ph, vfailed);
 			if (!ok) { *vfailed = 1; break; }
 			const unsigned char *st = stages + (unsigned)s * sbytes;
 			union { int4 q[IB / 16]; int i[IB / 4]; } ci;
@@ -710,7 +722,7 @@ __device__ __forceinline__ bool sweep_run(const SweepArgs &a, const T *__restric
 	         next = (pos + 32u * (unsigned)(a.look + 1) * (unsigned)sizeof(T)) & bytes;
 	for (int t = 0; t < turns && !fail; t++) {
 		const int c = warp + t * nw;
-		if (!mbar_wait_or_fail(&full[s], ph, vfailed)) { fail = true; break; }
+		if (!mbar_wait_warp(&full[s], ph, vfailed)) { fail = true; break; }
 		waited++;
 		Rec cur;
 		cur.load(stages + (unsigned)s * (unsigned)a.stage_bytes, roff, boff);
