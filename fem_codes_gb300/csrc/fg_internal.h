@@ -32,15 +32,16 @@ typedef struct fg_sweep {
 	long long bytes, maxblk, nval;
 	int npad;                  /* padded length of the level-ordered vector  */
 	unsigned char *prog;       /* sub-blocks                                 */
+	/* (chain programs' chunks and slices are alike and need neither)       */
 	long long *blk_off;        /* [nsb+1] byte offsets of the sub-blocks     */
 	int *sb_in, *sb_inb;       /* [nsb] input slice start (padded), bytes    */
-	int *lev_start;            /* [nlev+1] first level-order position        */
 	int *rows;                 /* [n] row at each level-order position       */
 	int *ppos;                 /* [n] padded position of each position       */
 	long long *val_off;        /* [nval] byte offset of each value slot      */
 	int *val_src;              /* [nval] CSR position (-1 zero, -2-r pivot)  */
 	int nchunk;                /* matrix blocks (block ILU(0); 1: global)    */
-	int *chunk_sb, *chunk_lev; /* [nchunk+1] first sub-block / level of each */
+	int *chunk_sb, *chunk_lev; /* [nchunk+1] first sub-block / level of each
+	                            * (levels: row programs only)               */
 	int rw;                    /* record layout width (0: ELL sub-blocks)    */
 	int df;                    /* record layout swept without level barriers */
 	int ring, look, warps;     /* ... ring slots, chunks a warp may run

@@ -1043,8 +1043,6 @@ __global__ void k_gnn_adam(int P, float *th, const float *g, float *m, float *v,
 	}
 }
 
-// ls[0..1] = (sum v^2, -), ls[2..3] = (sum res^2, -) -> ls[1] = sum res^2.
-
 __global__ void k_gnn_dbar(const double *sums, int n, double *stats) { stats[1] = sums[0] / n; }
 
 // ---------------------------------------------------------------- launchers

@@ -940,6 +940,12 @@ __global__ void k_refresh(unsigned char *prog, const long long *val_off, const i
 // of ILUp_precond_setup.c:119-139.  What each lane reads is precompiled, so a
 // row needs no pattern searches.
 //
+// The program takes 16 + 8 L + L L bytes a row, 144, 400 or 1296 for rows of up
+// to 8, 16 and 32 entries (the longest row's L for all), on the device and, while
+// it is built, on the host: transport 144, ILU(1) and ILU(2) of it 400,
+// Navier-Stokes (21 entries) and Euler (28) 1296.  Programs of operand lists took
+// 212, 312, 297, 724 and 1291.
+//
 // What bounds it is the chain of levels: per level one trip of a value
 // through L2 (0.36 us), two dependent rows' groups (three FP64 operations of 31
 // ns each; a warp's FP64 instruction holds this part's FP64 pipe for 64
@@ -948,8 +954,8 @@ __global__ void k_refresh(unsigned char *prog, const long long *val_off, const i
 // cluster barrier after each (4.6 us a level), or, for rows of more than 64
 // program words, walked by one CTA (17 us a level).  Measured, before and now:
 // 400x300 transport, one block (1098 levels) 4.80 -> 1.42 ms; 2048x1024 in 32
-// blocks 5.81 -> 2.2 ms; Navier-Stokes 96x96 (27k rows of up to 21 entries)
-// 17.0 -> 1.00 ms.  (Polling one operand at a time, each missing one costs a
+// blocks 5.81 -> 1.96 ms; Navier-Stokes 96x96 (27k rows of up to 21 entries)
+// 17.0 -> 0.96 ms.  (Polling one operand at a time, each missing one costs a
 // trip of its own: 1.65 and 1.11 ms.)
 #define FAC_CAP 32                    // entries of a row
 #define FAC_TPB 128                   // four warps: one per FP64 pipe
@@ -1465,7 +1471,6 @@ static int build_prog(const int *IA, const int *JA, int n, const HostLevels &H, 
 	if ((rc = up_vec(&sw.blk_off, off))) return rc;
 	if ((rc = up_vec(&sw.sb_in, sb_in))) return rc;
 	if ((rc = up_vec(&sw.sb_inb, sb_inb))) return rc;
-	if ((rc = up_vec(&sw.lev_start, H.start))) return rc;
 	if ((rc = up_vec(&sw.rows, H.rows))) return rc;
 	std::vector<int> ppos_by_pos(n);
 	for (int p = 0; p < n; p++) ppos_by_pos[p] = H.ppos[H.rows[p]];
@@ -1618,15 +1623,12 @@ static int build_prog_chain(const int *IA, const int *JA, int n, const ChainLeve
 		cfirst[i] = (int)(i - first);
 	}
 	std::vector<long long> off(nsb + 1, 0);
-	std::vector<int> sb_in(nsb), sb_inb(nsb);
-	long long bvo = 0, maxin = 0;
+	long long bvo = 0;
+	const long long inb = al16(cmax * tsize);            // bytes of a chunk's input slice
 	for (int i = 0; i < nsb; i++) {
 		const long long bb = DF_HDR + (long long)subs[i].c * RB;
 		off[i + 1] = off[i] + bb;
-		sb_in[i] = H.lstart[subs[i].l] + subs[i].j0;
-		sb_inb[i] = (int)al16((long long)subs[i].c * tsize);
 		bvo = std::max(bvo, bb);
-		maxin = std::max(maxin, (long long)sb_inb[i]);
 	}
 	std::vector<unsigned char> prog((size_t)off[nsb] + 16, 0);
 	std::vector<long long> val_off, cs_voff(H.nslot, -1);
@@ -1685,7 +1687,8 @@ static int build_prog_chain(const int *IA, const int *JA, int n, const ChainLeve
 		for (int i = 0; i < nsb; i++) {
 			const unsigned char *b = prog.data() + off[i];
 			const int c = subs[i].c;
-			if (sb_in[i] != 32 * i || c != 32 || (long long)sb_in[i] + c > H.nslot) return FEMGPU_E_MESH;
+			const int at = H.lstart[subs[i].l] + subs[i].j0;          // its input slice
+			if (at != 32 * i || c != 32 || (long long)at + c > H.nslot) return FEMGPU_E_MESH;
 			for (int j = 0; j < c; j++) {
 				auto ri = [&](int q) { return *(const int *)(b + iat(q, j)); };
 				for (int q = 0; q < rw; q++) {
@@ -1712,7 +1715,6 @@ static int build_prog_chain(const int *IA, const int *JA, int n, const ChainLeve
 	ppos.reserve(n);
 	for (int q = 0; q < H.nslot; q++)
 		if (H.slot_row[q] >= 0) { rows.push_back(H.slot_row[q]); ppos.push_back(q); }
-	std::vector<int> lev_start(H.lstart);
 	sw.nchunk = (int)H.clev.size() - 1;
 	sw.rw = rw;
 	sw.df = 1;
@@ -1725,23 +1727,18 @@ static int build_prog_chain(const int *IA, const int *JA, int n, const ChainLeve
 	sw.nlev = nlev;
 	sw.nsb = nsb;
 	sw.bytes = off[nsb];
-	sw.maxblk = bvo + maxin;
+	sw.maxblk = bvo + inb;
 	sw.nval = (long long)val_off.size();
 	sw.npad = H.nslot;
 	sw.nslot = H.nslot;
 	int rc;
 	FG_TRY(cudaMalloc((void **)&sw.prog, prog.size()));
 	FG_TRY(cudaMemcpy(sw.prog, prog.data(), prog.size(), cudaMemcpyHostToDevice));
-	if ((rc = up_vec(&sw.blk_off, off))) return rc;
-	if ((rc = up_vec(&sw.sb_in, sb_in))) return rc;
-	if ((rc = up_vec(&sw.sb_inb, sb_inb))) return rc;
-	if ((rc = up_vec(&sw.lev_start, lev_start))) return rc;
 	if ((rc = up_vec(&sw.rows, rows))) return rc;
 	if ((rc = up_vec(&sw.ppos, ppos))) return rc;
 	if ((rc = up_vec(&sw.val_off, val_off))) return rc;
 	if ((rc = up_vec(&sw.val_src, val_src))) return rc;
 	if ((rc = up_vec(&sw.chunk_sb, csb))) return rc;
-	if ((rc = up_vec(&sw.chunk_lev, H.clev))) return rc;
 	if ((rc = up_vec(&sw.cs_voff, cs_voff))) return rc;
 	if ((rc = up_vec(&sw.cs_src, cs_src))) return rc;
 	if ((rc = up_vec(&sw.cs_row, cs_row))) return rc;
@@ -2303,7 +2300,7 @@ extern "C" void fg_ilu_free(femgpu_transport *t)
 	fg_ilu_sweeps &S = t->sweeps;
 	fg_sweep *all[8] = { &S.lo64, &S.up64, &S.lo32, &S.up32, &S.lo64c, &S.up64c, &S.lo32c, &S.up32c };
 	for (int i = 0; i < 8; i++) {
-		void *p[] = { all[i]->prog, all[i]->blk_off, all[i]->sb_in, all[i]->sb_inb, all[i]->lev_start,
+		void *p[] = { all[i]->prog, all[i]->blk_off, all[i]->sb_in, all[i]->sb_inb,
 		              all[i]->rows, all[i]->ppos, all[i]->val_off, all[i]->val_src, all[i]->chunk_sb,
 		              all[i]->chunk_lev, all[i]->cs_voff, all[i]->cs_src, all[i]->cs_row };
 		for (void *q : p) if (q) cudaFree(q);

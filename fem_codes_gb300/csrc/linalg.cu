@@ -739,7 +739,9 @@ static int red_grid(femgpu_transport *t) { return t->nblk_red; }
 // A cycle's steps are enqueued ahead of the device, STEPS_AHEAD at most: far
 // enough that the device never waits for the host, near enough that a cycle
 // that converges early leaves few launches that find nothing to do (up to ten
-// a step, 1.5 to 2 us each).  True when the device has finished the cycle.
+// a step, 1.5 to 2 us each).  The host watches a pinned word meanwhile, so a
+// solving thread keeps its core busy.  True when the device has finished the
+// cycle.
 #define STEPS_AHEAD 6
 static bool cycle_done(const fg_krylov *k, int i)
 {
@@ -1144,10 +1146,12 @@ static int tr_precond_g(void *c, const int *a, cudaStream_t s)
 static const void *tr_precond_g_out(void *c) { return ((femgpu_transport *)c)->sweeps.o64; }
 
 // FGMRES with the look-ahead step (fgmres_cycle_la): FP64 block or global
-// ILU(p) contexts, unless FEMGPU_LOOKAHEAD=0 (read at every cycle).  Its stream (the lowest
-// priority, so the Gram-Schmidt blocks never go before the sweep CTAs that
-// become ready with them), events and vectors are made on first use; without
-// them the plain cycle runs.
+// ILU(p) contexts, unless FEMGPU_LOOKAHEAD=0 (read at every cycle).  Its stream
+// has the least priority, which is the contexts' own streams' too (and a
+// caller's, unless made otherwise): what puts the sweep CTAs first is that they
+// follow the product on the same stream, while the Gram-Schmidt waits for an
+// event on the other.  Stream, events and vectors are made on first use;
+// without them the plain cycle runs.
 static int lookahead_on(femgpu_transport *t)
 {
 	const char *e = getenv("FEMGPU_LOOKAHEAD");
