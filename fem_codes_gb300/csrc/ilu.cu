@@ -534,8 +534,23 @@ k_sweep_rec(SweepArgs a, const T *__restrict__ in, T *out)
 // 16); a chain chunk is a long run of dependent FP32 operations, so the narrow
 // ones, whose registers allow it, take 24 (2048x1024, 32 blocks: 667 us an
 // application with 16, 586 with 20, 554 with 24 before their chunks lay side by
-// side, 448 now).
-__host__ __device__ constexpr int df_warps(bool cs, int w) { return cs && w <= 4 ? 24 : 16; }
+// side, 448 now).  Rows of 16 do not fit the registers of 16 warps.
+__host__ __device__ constexpr int df_warps(bool cs, int w) { return cs && w <= 4 ? 24 : w > 12 ? 12 : 16; }
+
+// How a row waits for values that are late.  Narrow rows, and FP64 ones of any
+// width, go on term by term, each as soon as its value is there.  Wide rows in
+// FP32 or double-single arithmetic wait for all of them and run their terms then
+// without a vote between: a term costs less than its vote.  Looking at every
+// value still missing while one is late takes code that grows with the square
+// of the width, which for 12 and 16 was no longer unrolled (values in local
+// memory): a look at the next three is enough.  An application at 400x300 with
+// ILU(4) (12 wide) and ILU(6) (16), squares / next three / all:
+// FP64 rows 19.6 / 8.11 / 8.52 and 42.5 / 13.8 / 14.3 ms, double-single chains
+// 13.1 / 4.22 / 3.56 and 17.8 / 6.24 / 4.70, FP32 chains 3.91 / 2.66 / 1.50 and
+// 16.9 / 4.15 / 2.03; Navier-Stokes 256x256 (12 wide), an FGMRES iteration 6.04
+// / 2.17 / 1.95 ms.
+template <typename T> __host__ __device__ constexpr bool sweep_all(int w) { return w > 8; }
+template <> __host__ __device__ constexpr bool sweep_all<double>(int) { return false; }
 
 // Ring values: polled loads, stores, the mark.
 template <typename T> __device__ __forceinline__ bool ring_unset(T v)
@@ -652,6 +667,7 @@ __device__ __forceinline__ bool sweep_run(const SweepArgs &a, const T *__restric
                                           unsigned long long *full, int *failed, int *prog)
 {
 	typedef SweepRec<T, UPPER, CS, W> Rec;
+	constexpr bool ALL = sweep_all<T>(W);
 	const unsigned rb = smem_u32(sm), zero = rb + (unsigned)a.ring * (unsigned)sizeof(T);
 	const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, D = a.D, nw = blockDim.x >> 5;
 	const int sb0 = a.chunk_sb[blockIdx.x], cnt = a.chunk_sb[blockIdx.x + 1] - sb0;
@@ -757,7 +773,23 @@ __device__ __forceinline__ bool sweep_run(const SweepArgs &a, const T *__restric
 		}
 #pragma unroll
 		for (int k = 0; k < W; k++) miss = miss || ring_unset(d[k]);
-		if (!__any_sync(0xffffffffu, miss)) {
+		bool late = __any_sync(0xffffffffu, miss);
+		if (ALL && late) {
+			int it = 0;
+			do {
+				if (it >= a.wait || ((it & 63) == 63 && __any_sync(0xffffffffu, *vfailed != 0))) { fail = true; break; }
+				it++;
+				miss = false;
+#pragma unroll
+				for (int k = 0; k < W; k++) {
+					if (ring_unset(d[k])) d[k] = ring_ld<T>(src[k]);
+					miss = miss || ring_unset(d[k]);
+				}
+			} while (__any_sync(0xffffffffu, miss));
+			if (fail) break;
+			late = false;
+		}
+		if (!late) {
 #pragma unroll
 			for (int k = 0; k < W; k++) y = fmsub<T, FMA>(y, d[k], cur.v[k]);
 		} else {
@@ -772,7 +804,7 @@ __device__ __forceinline__ bool sweep_run(const SweepArgs &a, const T *__restric
 					} while (__any_sync(0xffffffffu, ring_unset(d[k])));
 					if (fail) break;
 #pragma unroll
-					for (int q = k + 1; q < W; q++)       // the others may have come meanwhile
+					for (int q = k + 1; q < W && (W <= 8 || q < k + 4); q++)   // the others may have come meanwhile
 						if (ring_unset(d[q])) d[q] = ring_ld<T>(src[q]);
 				}
 				y = fmsub<T, FMA>(y, d[k], cur.v[k]);
