@@ -1086,12 +1086,12 @@ struct Blocks {
 };
 
 // Block ILU(0) cuts: P contiguous runs of the numbering; couplings between
-// runs are dropped.  A sweep costs one barrier per level and its P thread
-// blocks run side by side, so the deepest run (levels counted with the
-// couplings dropped) sets its time, while where the cuts fall sets how many
-// FGMRES iterations the weaker preconditioner costs.  After SYMRCM every front
-// is a dependency chain about as long as the front is wide, so equal row
-// counts leave the middle runs deepest.  FEMGPU_ILU_BLOCK_CUT selects:
+// runs are dropped.  The P thread blocks of a sweep run side by side, so the
+// slowest run (its chunks, and its depth in levels counted with the couplings
+// dropped) sets its time, while where the cuts fall sets how many FGMRES
+// iterations the weaker preconditioner costs.  After SYMRCM every front is a
+// dependency chain about as long as the front is wide, so equal row counts
+// leave the middle runs deepest.  FEMGPU_ILU_BLOCK_CUT selects:
 //   levels (default)  run b starts at the first row where the running maximum
 //                     of the full factor's forward level reaches
 //                     ceil(b * levels / P): equal spans of fronts;
@@ -1100,10 +1100,13 @@ struct Blocks {
 //                     most P runs (bisection), the runs with the most rows then
 //                     halved until there are P: the shallowest deepest run;
 //   rows              row r in run floor(r * P / n).
-// Measured at 2048x1024 with FGMRES(80) to 1e-8 (ms per Picard step, ILU
-// application, iterations): rows P=8 148 / 1.90 ms / 56-59; levels P=16
-// 125 / 1.47 ms / 57-59; depth P=16 136 / 1.38 ms / 65-67, P=12 134 / 1.50
-// ms / 60-63.
+// Measured with FGMRES(80) to 1e-8 on the double-single chain sweeps, an
+// application and the iterations of three Picard steps, levels / rows / depth:
+// 2048x1024, P=32: 500 us 47 109 100 / 502 us 53 136 142 / 808 us 58 205 272;
+// 1023x1023, P=32: 318 us 56 110 341 / 337 us 63 150 293 / 711 us 83 409 625;
+// 1023x511, P=16: 271 us 57 57 61 / 328 us 58 62 65 / 396 us 58 64 67.  The
+// row cut's largest run has half as many chunks at 2048x1024 (4996 against
+// 9106) but more levels: no faster, and more iterations.
 static std::vector<int> greedy_runs(const int *IA, const int *JA, int n, int T, std::vector<int> &lev)
 {
 	std::vector<int> first(1, 0);

@@ -203,7 +203,9 @@ int femgpu_transport_matvec(femgpu_transport *ctx, const double *P_host, double 
 
 /* solver (pgmres.c:4-211, 4-argument steady-transport form): B = the device
  * F (already preconditioned by precond_setup), X = the device u.  X_host
- * [neq+1] receives u when non-NULL; iters receives the inner iterations. */
+ * [neq+1] receives u when non-NULL; iters receives the inner iterations.  In
+ * every context's solve the calling thread watches the device's progress and
+ * keeps its core busy until the solve is done. */
 int femgpu_transport_solve(femgpu_transport *ctx, double *X_host, int *iters);
 
 /* 6-argument pgmres form (Euler/NS solver pointer, EulerEquations.h:168):
